@@ -82,7 +82,7 @@ extern "C" {
 #define DTWJ_PHASE_PREP 0       /* statistics, envelopes, mask, row terms     */
 #define DTWJ_PHASE_PROFILE 1    /* ED matrix profile                          */
 #define DTWJ_PHASE_SEEDS 2      /* seed selection and seed DTWs               */
-#define DTWJ_PHASE_DIAG 3       /* diagonal bound sweep                       */
+#define DTWJ_PHASE_DIAG 3       /* sweep: group bound, diagonal bound         */
 #define DTWJ_PHASE_PAIRS 4      /* LB_Keogh with cumulative bound + DTW       */
 #define DTWJ_PHASE_VERIFY 5     /* FP64 re-verification                       */
 #define DTWJ_PHASE_RUNS 6       /* run filter: block-mean bound + endpoint bound
@@ -97,7 +97,9 @@ typedef struct {
   double dist_fp32;        /* the FP32 distance the device search found      */
   double seed_bsf;         /* best-so-far after the ED-profile seeds         */
   uint64_t pairs;          /* candidate pairs (non-flat, j - i >= m)         */
-  uint64_t pruned_fast;    /* pruned by the O(1) diagonal ED/LB_Keogh bound  */
+  uint64_t pruned_fast;    /* pruned by the sweep: the block-mean bound of window
+                              groups, or the O(1) diagonal bound in the tiles
+                              where that settles nothing                     */
   uint64_t pruned_kim;     /* pruned by the endpoint bound                   */
   uint64_t pruned_masked;  /* pruned by the masked diagonal bound            */
   uint64_t pruned_keogh;   /* pruned by LB_Keogh (either direction)          */

@@ -181,6 +181,14 @@ struct DevSeries {
   float* cmax2;     // 2 kCopyBlocks(n), largest |value| of each copy block
   float4* wrec;     // s, window record: block offset (FP64 in .x/.y), isg as
                     //    FP32 (.z) and the error scale for pq2 (.w)
+  // Window groups of the group bound (nullptr: not built): grp_d slots of
+  // grp_n records, slot-major; a record holds (smallest and largest block
+  // mean, largest upper and smallest lower envelope mean) of grp_g windows
+  // over one segment of grp_b samples, z-normalised, rounded outward.
+  float4* grp;
+  float4* sup;      // the same for kGrpFan consecutive groups, sup_n records per slot
+  int64_t grp_n, sup_n;
+  int grp_g, grp_b, grp_d;
   int* status;      // device status word (0 ok, else error bits)
 };
 
@@ -205,6 +213,71 @@ struct DevSearch {
   unsigned int* kq_next;
   unsigned int kq_cap;
 };
+
+__device__ __forceinline__ float max3f(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+// ---- group filter (group.cu) ----
+constexpr int kGrpSlots = 32;  // segments per window, at most
+constexpr int kGrpFan = 4;     // groups of a super-group
+// Windows per group.  A group's records widen with the shift between its
+// windows, which matters relative to m: of a random walk's pairs, groups of 8
+// and 4 let through 1.8 % and 1.0 % at m = 512, w = 52 (single pairs: 0.7 %),
+// 0.64 % and 0.11 % at m = 256, w = 13 (0.02 %), 6.6 % and 1.9 % at m = 128.
+__host__ __device__ inline int group_windows(int m) { return m >= 512 ? 8 : 4; }
+// Buffers of the filter over one chunk of tiles.
+struct GroupFilter {
+  unsigned int* sup;     // surviving super-group pairs: group_code
+  unsigned int* nsup;
+  uint2* list;           // of them, those with surviving group pairs: (group_code, mask of the
+                         //   kGrpFan x kGrpFan group pairs)
+  unsigned int* nlist;
+  unsigned int* tcount;  // surviving group pairs per tile (nullptr: no filter, every tile dense)
+  unsigned int* dense;   // tiles the diagonal sweep ran on
+  unsigned int* ndense;
+  int nib, nw;           // first-level work items per tile: blocks of row groups x column words
+};
+// A super-group pair of a tile of the chunk: tile, row group relative to the
+// tile's first (at most 252), column group relative to row group + L0 / G (at
+// most 57).
+__host__ __device__ inline unsigned int group_code(unsigned int tile, int row, int col) {
+  return (tile << 14) | ((unsigned int)row << 6) | (unsigned int)col;
+}
+__host__ __device__ inline unsigned int group_code_tile(unsigned int code) { return code >> 14; }
+struct GroupPair {
+  int I, J;
+};
+__host__ __device__ inline GroupPair group_code_pair(unsigned int code, const Tile& T, int G) {
+  GroupPair p;
+  p.I = T.i0 / G + (int)((code >> 6) & 255u);
+  p.J = p.I + T.L0 / G + (int)(code & 63u);
+  return p;
+}
+// Whether a pair of groups of g windows holds pairs of the tile (for groups
+// that reach past the tile's rows or lags on both sides: may hold).
+__host__ __device__ inline bool group_pair_in_tile(const Tile& T, int g, int I, int J) {
+  const int64_t ia = (int64_t)I * g, ja = (int64_t)J * g, last = (int64_t)T.i0 + T.rows - 1;
+  const int64_t lo = ia > T.i0 ? ia : T.i0, hi = ia + g - 1 < last ? ia + g - 1 : last;
+  return lo <= hi && ja < T.send && ja + g - 1 - lo >= T.L0 && ja - hi < T.L0 + kLbLags;
+}
+// Pairs of a tile: rows [0, rows), lags [0, kLbLags) with the later window
+// below send.
+__host__ __device__ inline int64_t tile_pairs(const Tile& T) {
+  const int64_t room = (int64_t)T.send - T.i0 - T.L0;  // lags of the first row, >= rows
+  int64_t full = room - kLbLags + 1;                   // rows with every lag
+  full = full < 0 ? 0 : (full < T.rows ? full : T.rows);
+  const int64_t part = T.rows - full;
+  return full * kLbLags + part * (room - full) - part * (part - 1) / 2;
+}
+// A tile goes through the diagonal bound when more than 7/8 of its group
+// pairs survive: the group bound says nothing about it (noise, or structure
+// shorter than a segment), where the diagonal bound may still prune.
+__host__ __device__ inline bool group_tile_dense(const Tile& T, int g, unsigned int count) {
+  return (int64_t)count * g * g * 8 > 7 * tile_pairs(T);
+}
 
 // Endpoint bound: minimum cost of any warping path's cells in the first and
 // last three layers (LB_KIM, CPU_version1/lb_kim.cpp:10-73).  q = window i,
@@ -304,12 +377,29 @@ void launch_mp_seed(const DevSeries& S, const Tile* tiles, int ntiles, unsigned 
 __device__ __forceinline__ int series_of(const DevSeries& S, int64_t x) {
   return S.sid ? S.sid[x] : 0;
 }
-// Fast diagonal bound over LB tiles [tile_begin, tile_end); survivors leave
-// as bits, [tile][lag][word].  enumerate_all: no pruning (bounds off).
-// Persistent: CTAs take tiles from the work counter *next (zero at launch).
-void launch_lb(const DevSeries& S, const DevSearch& Q, const Tile* tiles, int tile_begin,
-               int tile_end, unsigned int* bits, bool enumerate_all, unsigned int* next,
-               int num_sms, cudaStream_t st);
+// Group filter (group.cu).  group_shape sets the group sizes of S;
+// launch_group_prep fills S.grp and S.sup (means: 3 n doubles of scratch) and
+// returns the number of kernels it launched; group_items sets F's items per tile
+void group_shape(int m, int64_t s, DevSeries* S);
+int launch_group_prep(const DevSeries& S, double* means, cudaStream_t st);
+// and returns the largest number of super-group pairs of one.
+size_t group_items(int g, GroupFilter* F);
+// F.nsup, F.nlist and F.tcount are zero at launch.  Two kernels.
+void launch_group(const DevSeries& S, const DevSearch& Q, const GroupFilter& F, const Tile* tiles,
+                  int tile_begin, int tile_end, int num_sms, cudaStream_t st);
+// Sets the survivor bits of the sparse tiles (masked cascade).
+void launch_group_bits(const DevSeries& S, const DevSearch& Q, const GroupFilter& F,
+                       const Tile* tiles, int tile_begin, int num_sms, unsigned int* bits,
+                       cudaStream_t st);
+// Fast diagonal bound over LB tiles [tile_begin, tile_end) that the group
+// filter left dense (every tile when F.tcount is nullptr); survivors leave as
+// bits, [tile][word][lag], their tiles are listed in F.dense.  Sparse tiles
+// only count their pairs; with clear_sparse their bits are zeroed.
+// enumerate_all: no pruning (bounds off).  Persistent: CTAs take tiles from
+// the work counter *next (zero at launch).
+void launch_lb(const DevSeries& S, const DevSearch& Q, const GroupFilter& F, const Tile* tiles,
+               int tile_begin, int tile_end, unsigned int* bits, bool enumerate_all,
+               bool clear_sparse, unsigned int* next, int num_sms, cudaStream_t st);
 size_t lb_smem_bytes();
 // Run filter over the survivor bits of LB tiles [tile_begin, tile_end):
 // masked bound, endpoint bound and LB_Keogh for every pair of every run of
@@ -323,10 +413,16 @@ void launch_center(const DevSeries& S, cudaStream_t st);
 // profile: grid kSeedGrid); out[64 * t ...] for tile t.
 void launch_tile_features(const DevSeries& S, const Tile* tiles, int ntiles,
                           const unsigned long long* keys, int grid, float* out, cudaStream_t st);
-// Block-mean lower bound (LB_PAA) over the survivor bits of LB tiles
-// [tile_begin, tile_end), then the endpoint bound; survivors go to Q.kq.
-void launch_paa(const DevSeries& S, const DevSearch& Q, const Tile* tiles, int tile_begin,
-                int tile_end, const unsigned int* bits, int num_sms, cudaStream_t st);
+// Block-mean lower bound (LB_PAA), then the endpoint bound, over the survivor
+// bits of the dense tiles; survivors go to Q.kq.
+void launch_paa(const DevSeries& S, const DevSearch& Q, const GroupFilter& F, const Tile* tiles,
+                int tile_begin, int tile_end, const unsigned int* bits, int num_sms,
+                cudaStream_t st);
+// The same over the pairs of the group filter's surviving groups (sparse
+// tiles; next: a zeroed work counter).
+void launch_paa_groups(const DevSeries& S, const DevSearch& Q, const GroupFilter& F,
+                       const Tile* tiles, int tile_begin, unsigned int* next, int num_sms,
+                       cudaStream_t st);
 // Block length of the block-mean bound for windows of length m.
 int paa_block(int m);
 // Sliding block means (pq, or pq2 and wrec for windows of at most 1024

@@ -8,8 +8,9 @@
 //   prep      statistics, envelopes, mask, row constants        (prep.cu)
 //   profile   ED matrix profile, row minima                      (mp.cu)
 //   seeds     kSeeds smallest profile entries -> exact DTW        (mp.cu, pairs.cu)
-//   sweep     per chunk of tiles: diagonal bound -> survivor
-//             queue -> endpoint / masked / LB_Keogh / DTW         (lb.cu, pairs.cu)
+//   sweep     per chunk of tiles: group bound, diagonal bound on the tiles it
+//             leaves dense -> block-mean / endpoint / LB_Keogh /
+//             DTW                          (group.cu, lb.cu, paa.cu, runs.cu, pairs.cu)
 //   verify    FP64 DTW of every candidate near the final best     (pairs.cu)
 // with a single host synchronisation at the end.
 #include "../../include/dtwj.h"
@@ -145,7 +146,8 @@ enum BufId {
   B_MP, B_MPI, B_CB, B_AF, B_ULF, B_BITS, B_LBTILES, B_KQ, B_SBEG, B_SID, B_SEEDBSF,
   B_BEST_IJ, B_BEST_F32, B_QSER, B_TILEBEST, B_FEAT, B_SCORE, B_PA, B_CMAX, B_RW,
   B_MPX_WANT, B_MPX_WREV, B_MPX_MIN, B_MPX_IDX, B_MPX_CAND, B_MPX_CNT, B_NOTES, B_NOTES2,
-  B_SORT, B_SORT_TEMP, B_LBTILES2, B_CMAX2, B_WREC, B_COUNT_
+  B_SORT, B_SORT_TEMP, B_LBTILES2, B_CMAX2, B_WREC, B_GRP, B_SUP, B_GMEANS, B_GSUP, B_GLIST, B_DENSE,
+  B_COUNT_
 };
 
 int ensure(dtwj_ctx* c, int id, size_t bytes, void** out) {
@@ -273,8 +275,11 @@ void build_lb_tiles(dtwj_ctx* ctx, int64_t n, int m, const int64_t* sbeg, int ns
 
 // Allocates and prepares every per-series array; returns the DevSeries.  A
 // batch (sbeg != nullptr) holds nseries series back to back in x_dev, series
-// r on samples [sbeg[r], sbeg[r + 1]).
-int prepare(dtwj_ctx* ctx, const double* x_dev, int64_t n, int m, int w, bool masked,
+// r on samples [sbeg[r], sbeg[r + 1]).  groups: also the records of the group
+// filter, where the single-pair block-mean bound reads one offset per window
+// (m <= 1024) and they fit the device (S.grp stays nullptr otherwise: every
+// tile then goes through the diagonal bound).
+int prepare(dtwj_ctx* ctx, const double* x_dev, int64_t n, int m, int w, bool masked, bool groups,
             const int64_t* sbeg_host, int nseries, DevSeries* out, Phases* ph = nullptr) {
   const int64_t s = n - m + 1;
   DevSeries S;
@@ -330,6 +335,18 @@ int prepare(dtwj_ctx* ctx, const double* x_dev, int64_t n, int m, int w, bool ma
   ENSURE(B_CMAX, ((n >> kBlkShift) + 4) * 4, S.cmax);
   ENSURE(B_RW, s * 4, S.rw);
   S.paa_b = paa_block(m);
+  double* gmeans = nullptr;
+  if (groups && m <= (1 << kBlkShift)) {
+    group_shape(m, s, &S);
+    void *recs = nullptr, *sups = nullptr, *means = nullptr;
+    if (ensure(ctx, B_GRP, (size_t)S.grp_n * S.grp_d * sizeof(float4), &recs) == DTWJ_OK &&
+        ensure(ctx, B_SUP, (size_t)S.sup_n * S.grp_d * sizeof(float4), &sups) == DTWJ_OK &&
+        ensure(ctx, B_GMEANS, (size_t)n * 24, &means) == DTWJ_OK) {
+      S.grp = static_cast<float4*>(recs);
+      S.sup = static_cast<float4*>(sups);
+      gmeans = static_cast<double*>(means);
+    }
+  }
   ENSURE(B_STATUS, 4, S.status);
   cudaStream_t st = ctx->stream;
   CUDA_OK(cudaMemsetAsync(S.status, 0, 4, st));
@@ -378,7 +395,8 @@ int prepare(dtwj_ctx* ctx, const double* x_dev, int64_t n, int m, int w, bool ma
   }
   launch_rowterms(S, masked, st);
   launch_center(S, st);
-  const int paa_launches = launch_paa_prep(S, st);
+  int paa_launches = launch_paa_prep(S, st);
+  if (S.grp) paa_launches += launch_group_prep(S, gmeans, st);
   if (ph) ph->end(DTWJ_PHASE_PREP, (masked ? 11 : 6) + paa_launches);
   CUDA_OK(cudaGetLastError());
   *out = S;
@@ -427,7 +445,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   CUDA_OK(cudaEventRecord(ctx->ev0, st));
 
   DevSeries S;
-  int rc = prepare(ctx, x_dev, n, m, w, masked, sbeg, nseries, &S, &ph);
+  int rc = prepare(ctx, x_dev, n, m, w, masked, !(flags & DTWJ_F_NO_DIAG), sbeg, nseries, &S, &ph);
   if (rc) return rc;
 
   build_lb_tiles(ctx, n, m, sbeg, nseries);
@@ -464,8 +482,16 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   ENSURE(B_QUEUE, (size_t)qcap * sizeof(int2), Q.queue);
   // LB_Keogh candidates of one chunk: twice the DTW queue (most are pruned)
   ENSURE(B_KQ, (size_t)qcap * 2 * sizeof(int4), Q.kq);
+  const bool enumerate_all = flags & DTWJ_F_NO_DIAG;
+  const double tile_pairs = (double)kLbLags * kLbRows;
+  int chunk = ctx->chunk_tiles > 0 ? ctx->chunk_tiles
+                                   : kLbChunkRounds * kLbCtasPerSm * ctx->num_sms;
+  if (enumerate_all) chunk = (int)((double)qcap / tile_pairs) > 0 ? (int)((double)qcap / tile_pairs) : 1;
+  const int chunk_max = chunk < nlb ? chunk : (nlb > 0 ? nlb : 1);  // tiles of the largest chunk
+  // counters of a chunk, then the group filter's surviving group pairs per tile
+  constexpr int kQcTiles = 16;
   unsigned int* qc;
-  ENSURE(B_QCOUNT, 32, qc);
+  ENSURE(B_QCOUNT, (size_t)(kQcTiles + chunk_max) * 4, qc);
   Q.queue_count = qc;
   Q.queue_next = qc + 1;
   Q.run_count = qc + 2;
@@ -473,6 +499,19 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   Q.kq_count = qc + 4;
   Q.kq_next = qc + 5;
   unsigned int* lb_next = qc + 6;
+  GroupFilter F;
+  memset(&F, 0, sizeof F);
+  F.nsup = qc + 8;
+  F.nlist = qc + 9;
+  F.ndense = qc + 10;
+  unsigned int* paa_next = qc + 11;
+  ENSURE(B_DENSE, (size_t)chunk_max * 4, F.dense);
+  if (S.grp) {
+    const size_t pairs = (size_t)chunk_max * group_items(S.grp_g, &F);
+    ENSURE(B_GSUP, pairs * 4, F.sup);
+    ENSURE(B_GLIST, pairs * sizeof(uint2), F.list);
+    F.tcount = qc + kQcTiles;
+  }
   Q.queue_cap = qcap;
   Q.kq_cap = qcap * 2;
   Q.runs = nullptr;
@@ -577,21 +616,19 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   CUDA_OK(cudaMemcpyAsync(seed_bsf, Q.bsf2, (size_t)nslots * 4, cudaMemcpyDeviceToDevice, st));
 
   // ---- diagonal sweep in chunks of LB tiles ----
-  const bool enumerate_all = flags & DTWJ_F_NO_DIAG;
-  const double tile_pairs = (double)kLbLags * kLbRows;
-  int chunk = ctx->chunk_tiles > 0 ? ctx->chunk_tiles
-                                   : kLbChunkRounds * kLbCtasPerSm * ctx->num_sms;
-  if (enumerate_all) chunk = (int)((double)qcap / tile_pairs) > 0 ? (int)((double)qcap / tile_pairs) : 1;
   unsigned int* bits;
-  ENSURE(B_BITS, (size_t)(chunk < nlb ? chunk : (nlb > 0 ? nlb : 1)) * kLbLags * kLbWords * 4, bits);
+  ENSURE(B_BITS, (size_t)chunk_max * kLbLags * kLbWords * 4, bits);
   // the stages after the diagonal bound of one chunk: run filter, LB_Keogh, DTW
   auto filter_chunk = [&](int t0, int t1) {
     ph.begin();
-    if (enumerate_all || cascade)
+    if (enumerate_all || cascade) {
       launch_runs(S, Q, lbtiles, t0, t1, bits, masked, !enumerate_all, ctx->num_sms, st);
-    else
-      launch_paa(S, Q, lbtiles, t0, t1, bits, ctx->num_sms, st);
-    ph.end(DTWJ_PHASE_RUNS, 1);
+      ph.end(DTWJ_PHASE_RUNS, 1);
+    } else {
+      if (S.grp) launch_paa_groups(S, Q, F, lbtiles, t0, paa_next, ctx->num_sms, st);
+      launch_paa(S, Q, F, lbtiles, t0, t1, bits, ctx->num_sms, st);
+      ph.end(DTWJ_PHASE_RUNS, S.grp ? 2 : 1);
+    }
     if (!enumerate_all) {
       ph.begin();
       launch_keogh(S, Q, ctx->num_sms, st);
@@ -607,10 +644,14 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   // the counters before the pass, notes[c + 1] those after range c
   using Range = std::pair<int, int>;
   auto sweep_range = [&](const Range& r, ChunkNote* note) {
-    CUDA_OK(cudaMemsetAsync(qc, 0, 32, st));
+    CUDA_OK(cudaMemsetAsync(qc, 0, (size_t)(kQcTiles + r.second - r.first) * 4, st));
     ph.begin();
-    launch_lb(S, Q, lbtiles, r.first, r.second, bits, enumerate_all, lb_next, ctx->num_sms, st);
-    ph.end(DTWJ_PHASE_DIAG, 1);
+    if (S.grp) launch_group(S, Q, F, lbtiles, r.first, r.second, ctx->num_sms, st);
+    launch_lb(S, Q, F, lbtiles, r.first, r.second, bits, enumerate_all, cascade, lb_next,
+              ctx->num_sms, st);
+    if (S.grp && cascade)
+      launch_group_bits(S, Q, F, lbtiles, r.first, ctx->num_sms, bits, st);
+    ph.end(DTWJ_PHASE_DIAG, S.grp ? (cascade ? 4 : 3) : 1);
     filter_chunk(r.first, r.second);
     k_chunk_note<<<1, 32, 0, st>>>(S.status, Q.counters, note);
     return DTWJ_OK;
@@ -706,6 +747,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
                                 (int64_t)(uintptr_t)bits, (int64_t)(uintptr_t)notes};
       put(&S, sizeof S);
       put(&Q, sizeof Q);
+      put(&F, sizeof F);
       put(band_cg, sizeof band_cg);
       put(misc, sizeof misc);
       if (ctx->sweep_exec && key == ctx->sweep_key) {
@@ -1006,7 +1048,7 @@ int dtwj_time_band(int device, int32_t m, int32_t w, int32_t C, int32_t G, int32
     double* dev = nullptr;
     if ((rc = upload(ctx, x.data(), n, &dev))) break;
     DevSeries S;
-    if ((rc = prepare(ctx, dev, n, m, we, false, nullptr, 1, &S))) break;
+    if ((rc = prepare(ctx, dev, n, m, we, false, false, nullptr, 1, &S))) break;
     std::vector<int2> pr((size_t)pairs);
     const int64_t s = n - m + 1;
     for (int q = 0; q < pairs; ++q) {
@@ -1242,8 +1284,8 @@ int dtwj_matrix_profile(const double* x, int64_t n, int32_t m, double* mp, int64
       break;
     }
     DevSeries S, R;
-    if ((rc = prepare(ctx, dev, n, m, 0, false, nullptr, 1, &S))) break;
-    if ((rc = prepare(rev, rdev, n, m, 0, false, nullptr, 1, &R))) break;
+    if ((rc = prepare(ctx, dev, n, m, 0, false, false, nullptr, 1, &S))) break;
+    if ((rc = prepare(rev, rdev, n, m, 0, false, false, nullptr, 1, &R))) break;
     build_lb_tiles(ctx, n, m, nullptr, 1);
     const int nlb = (int)ctx->lbtiles_host.size();
     if ((rc = ensure(ctx, B_LBTILES, (size_t)nlb * sizeof(Tile), &p))) break;
@@ -1333,7 +1375,7 @@ int dtwj_global_mask(const double* x, int64_t n, int32_t m, int32_t w, float* ma
     double* dev = nullptr;
     if ((rc = upload(ctx, x, n, &dev))) break;
     DevSeries S;
-    if ((rc = prepare(ctx, dev, n, m, we, true, nullptr, 1, &S))) break;
+    if ((rc = prepare(ctx, dev, n, m, we, true, false, nullptr, 1, &S))) break;
     if (cudaMemcpyAsync(mask, S.mask, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream) !=
             cudaSuccess ||
         cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
@@ -1379,7 +1421,7 @@ int dtwj_pair_dtw(const double* x, int64_t n, int32_t m, int32_t w, const int64_
     double* dev = nullptr;
     if ((rc = upload(ctx, x, n, &dev))) break;
     DevSeries S;
-    if ((rc = prepare(ctx, dev, n, m, we, false, nullptr, 1, &S))) break;
+    if ((rc = prepare(ctx, dev, n, m, we, false, false, nullptr, 1, &S))) break;
     void* p;
     if ((rc = ensure(ctx, B_PAIRS, (size_t)count * sizeof(int2), &p))) break;
     int2* dp = (int2*)p;
@@ -1422,7 +1464,7 @@ int dtwj_pair_lb_petitjean(const double* x, int64_t n, int32_t m, int32_t w, con
     double* dev = nullptr;
     if ((rc = upload(ctx, x, n, &dev))) break;
     DevSeries S;
-    if ((rc = prepare(ctx, dev, n, m, we, false, nullptr, 1, &S))) break;
+    if ((rc = prepare(ctx, dev, n, m, we, false, false, nullptr, 1, &S))) break;
     void* p;
     if ((rc = ensure(ctx, B_PAIRS, (size_t)count * sizeof(int2), &p))) break;
     int2* dp = (int2*)p;

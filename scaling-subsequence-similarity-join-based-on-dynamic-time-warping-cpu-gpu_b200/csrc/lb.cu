@@ -1,5 +1,5 @@
-// Diagonal lower-bound sweep: the first stage of the reference's GLOBAL_DIAG
-// kernel (GPU_version1/lib/GLOBAL_DIAG.cu:29-73), diag_fast
+// Diagonal lower-bound sweep of the tiles the group filter (group.cu) leaves
+// dense: the first stage of the reference's GLOBAL_DIAG kernel (GPU_version1/lib/GLOBAL_DIAG.cu:29-73), diag_fast
 // (GPU_version1/lib/diag_fast.cu:13-90, CPU_version1/diag_fast.cpp:12-88).
 //
 // For pair (i, j), j = i + L, and the raw-series envelope U, L (radius w)
@@ -210,16 +210,20 @@ __device__ __forceinline__ void lb_tile(const DevSeries& S, const DevSearch& Q, 
 }
 
 // Persistent sweep: each CTA takes tiles from the work counter *next until
-// the chunk is exhausted; tile k of the chunk writes its bits to slot k.
+// the chunk is exhausted; tile k of the chunk writes its bits to slot k.  A
+// tile the group filter left sparse only has its pairs counted (all of them
+// as pruned: the pairs that survive their group are taken out again when they
+// are looked at) and, for the masked cascade, its bits cleared.
 __global__ void __launch_bounds__(kLbThreads, kLbCtasPerSm) k_lb(DevSeries S, DevSearch Q,
-                                                      const Tile* tiles, int ntiles,
+                                                      GroupFilter F, const Tile* tiles, int ntiles,
                                                       unsigned int* bits, bool enumerate_all,
-                                                      unsigned int* next) {
+                                                      bool clear_sparse, unsigned int* next) {
   extern __shared__ __align__(16) unsigned char smraw[];
   LbShared& sh = *reinterpret_cast<LbShared*>(smraw);
   __shared__ unsigned int tile_idx;
   const int lane = threadIdx.x & 31;
   unsigned int npairs = 0, nfast = 0;
+  unsigned long long sparse = 0;
   for (;;) {
     __syncthreads();  // every thread has read tile_idx and left the previous tile's staging
     if (threadIdx.x == 0) tile_idx = atomicAdd(next, 1u);
@@ -227,9 +231,17 @@ __global__ void __launch_bounds__(kLbThreads, kLbCtasPerSm) k_lb(DevSeries S, De
     const unsigned int k = tile_idx;
     if (k >= (unsigned int)ntiles) break;
     const Tile T = tiles[k];
-    lb_tile(S, Q, T, bits + (size_t)k * kLbLags * kLbWords, enumerate_all, sh, npairs, nfast);
+    unsigned int* out = bits + (size_t)k * kLbLags * kLbWords;
+    if (F.tcount && !group_tile_dense(T, S.grp_g, F.tcount[k])) {
+      if (threadIdx.x == 0) sparse += (unsigned long long)tile_pairs(T);
+      if (clear_sparse)
+        for (int x = threadIdx.x; x < kLbLags * kLbWords; x += kLbThreads) out[x] = 0u;
+      continue;
+    }
+    if (threadIdx.x == 0) F.dense[atomicAdd(F.ndense, 1u)] = k;
+    lb_tile(S, Q, T, out, enumerate_all, sh, npairs, nfast);
   }
-  unsigned long long np = npairs, nf = nfast;
+  unsigned long long np = npairs + sparse, nf = nfast + sparse;
   for (int o = 16; o > 0; o >>= 1) {
     np += __shfl_xor_sync(0xffffffffu, np, o);
     nf += __shfl_xor_sync(0xffffffffu, nf, o);
@@ -244,15 +256,15 @@ __global__ void __launch_bounds__(kLbThreads, kLbCtasPerSm) k_lb(DevSeries S, De
 
 size_t lb_smem_bytes() { return sizeof(LbShared); }
 
-void launch_lb(const DevSeries& S, const DevSearch& Q, const Tile* tiles, int tile_begin,
-               int tile_end, unsigned int* bits, bool enumerate_all, unsigned int* next,
-               int num_sms, cudaStream_t st) {
+void launch_lb(const DevSeries& S, const DevSearch& Q, const GroupFilter& F, const Tile* tiles,
+               int tile_begin, int tile_end, unsigned int* bits, bool enumerate_all,
+               bool clear_sparse, unsigned int* next, int num_sms, cudaStream_t st) {
   if (tile_end <= tile_begin) return;
   cudaFuncSetAttribute(k_lb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LbShared));
   const int ntiles = tile_end - tile_begin;
   const int resident = kLbCtasPerSm * num_sms;  // launch bounds, 64.5 KB shared each
   k_lb<<<ntiles < resident ? ntiles : resident, kLbThreads, sizeof(LbShared), st>>>(
-      S, Q, tiles + tile_begin, ntiles, bits, enumerate_all, next);
+      S, Q, F, tiles + tile_begin, ntiles, bits, enumerate_all, clear_sparse, next);
 }
 
 }  // namespace dtwj

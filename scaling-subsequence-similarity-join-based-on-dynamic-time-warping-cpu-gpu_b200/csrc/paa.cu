@@ -51,12 +51,6 @@ namespace {
 
 constexpr int kPaaWarps = 8;
 
-__device__ __forceinline__ float max3f(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-
 // Centers of the two copies of the block means for windows of at most 1024
 // samples: block b of copy 0 is [2048 b, 2048 b + 2048), block b of copy 1 is
 // [2048 b - 1024, 2048 b + 1024); each is centered on the mean of the two
@@ -198,6 +192,48 @@ struct Ends6 {
   __device__ double operator[](int k) const { return v[k]; }
 };
 
+// Endpoint bound (FP64, the end samples normalised) of the pairs (i, j) of
+// the lanes that are alive; those it keeps go to the LB_Keogh queue.  Called
+// by every lane of the warp.
+__device__ __forceinline__ void push_survivor(const DevSeries& S, const DevSearch& Q,
+                                              const Tile& T, bool alive, int i, int j, float thr,
+                                              int lane, unsigned int& nkim) {
+  if (!__any_sync(0xffffffffu, alive)) return;
+  const int m = S.m;
+  float kim = 0.0f;
+  if (alive) {
+    const double mi = S.mu[i], si = S.isg[i], mj = S.mu[j], sj = S.isg[j];
+    double qv[6], tv[6];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      qv[k] = (S.a[i + k] - mi) * si;
+      qv[3 + k] = (S.a[i + m - 3 + k] - mi) * si;
+      tv[k] = (S.a[j + k] - mj) * sj;
+      tv[3 + k] = (S.a[j + m - 3 + k] - mj) * sj;
+    }
+    double dl, dr;
+    kim_bound<double>(Ends6{qv}, Ends6{tv}, 6, &dl, &dr);
+    kim = (float)(dl + dr);
+    if (dl + dr > (double)thr) {
+      alive = false;
+      ++nkim;
+    }
+  }
+  const unsigned int sv = __ballot_sync(0xffffffffu, alive);
+  if (!sv) return;
+  unsigned int base = 0;
+  if (lane == 0) base = atomicAdd(Q.kq_count, (unsigned int)__popc(sv));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (alive) {
+    const unsigned int slot = base + __popc(sv & ((1u << lane) - 1u));
+    if (slot < Q.kq_cap) {
+      Q.kq[slot] = make_int4(i, j, __float_as_int(kim), T.series);
+    } else {
+      atomicOr(S.status, 2);
+    }
+  }
+}
+
 // One block term of both directions: query i (block mean qi) against the
 // envelope of j (uj, lj) and query j against the envelope of i, with
 // q - U = P - U s and L - q = L s - P, P = q s + (offset of q - offset of U).
@@ -213,9 +249,8 @@ __device__ __forceinline__ void block_terms(const float4 bi, const float4 bj, fl
 
 template <int B>
 __global__ void __launch_bounds__(kPaaWarps * 32, 3) k_paa(DevSeries S, DevSearch Q,
-                                                           const Tile* tiles,
-                                                           const unsigned int* bits,
-                                                           unsigned int total_items) {
+                                                           GroupFilter F, const Tile* tiles,
+                                                           const unsigned int* bits) {
   __shared__ unsigned long long cnt_paa, cnt_kim;
   if (threadIdx.x == 0) cnt_paa = cnt_kim = 0;
   __syncthreads();
@@ -223,13 +258,15 @@ __global__ void __launch_bounds__(kPaaWarps * 32, 3) k_paa(DevSeries S, DevSearc
   const int m = S.m;
   constexpr int kSpan = 1 << kBlkShift;
   unsigned int npaa = 0, nkim = 0;
+  const unsigned int total_items = *F.ndense * (unsigned int)(kLbWords * kLbGroups);
   for (;;) {
     unsigned int item = 0;
     if (lane == 0) item = atomicAdd(Q.run_next, 1u);
     item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= total_items) break;
-    const unsigned int tk = item / (kLbWords * kLbGroups);
-    const unsigned int rem = item - tk * (kLbWords * kLbGroups);
+    const unsigned int dk = item / (kLbWords * kLbGroups);
+    const unsigned int rem = item - dk * (kLbWords * kLbGroups);
+    const unsigned int tk = F.dense[dk];
     const int wi = (int)(rem / kLbGroups), g = (int)(rem % kLbGroups);
     const unsigned int word = bits[((size_t)tk * kLbWords + wi) * kLbLags + g * 32 + lane];
     unsigned int nz = __ballot_sync(0xffffffffu, word != 0u);
@@ -390,9 +427,8 @@ __global__ void __launch_bounds__(kPaaWarps * 32, 3) k_paa(DevSeries S, DevSearc
 // groups); the lanes vote every four blocks.
 template <int B>
 __global__ void __launch_bounds__(kPaaWarps * 32, 3) k_paa_lags(DevSeries S, DevSearch Q,
-                                                                const Tile* tiles,
-                                                                const unsigned int* bits,
-                                                                unsigned int total_items) {
+                                                                GroupFilter F, const Tile* tiles,
+                                                                const unsigned int* bits) {
   __shared__ unsigned long long cnt_paa, cnt_kim;
   if (threadIdx.x == 0) cnt_paa = cnt_kim = 0;
   __syncthreads();
@@ -401,13 +437,15 @@ __global__ void __launch_bounds__(kPaaWarps * 32, 3) k_paa_lags(DevSeries S, Dev
   const int nb = m / B;  // blocks per window (a short tail past nb B is left out)
   const float INF = __int_as_float(0x7f800000);
   unsigned int npaa = 0, nkim = 0;
+  const unsigned int total_items = *F.ndense * (unsigned int)(kLbWords * kLbGroups);
   for (;;) {
     unsigned int item = 0;
     if (lane == 0) item = atomicAdd(Q.run_next, 1u);
     item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= total_items) break;
-    const unsigned int tk = item / (kLbWords * kLbGroups);
-    const unsigned int rem = item - tk * (kLbWords * kLbGroups);
+    const unsigned int dk = item / (kLbWords * kLbGroups);
+    const unsigned int rem = item - dk * (kLbWords * kLbGroups);
+    const unsigned int tk = F.dense[dk];
     const int wi = (int)(rem / kLbGroups), g = (int)(rem % kLbGroups);
     // lane l holds lag L0 + 32 g + l: bit r is row i0 + 32 wi + r
     const unsigned int word = bits[((size_t)tk * kLbWords + wi) * kLbLags + g * 32 + lane];
@@ -462,42 +500,8 @@ __global__ void __launch_bounds__(kPaaWarps * 32, 3) k_paa_lags(DevSeries S, Dev
           if (__all_sync(0xffffffffu, pruned)) break;
         }
       }
-      bool alive = live && !pruned;
       npaa += (live && pruned) ? 1u : 0u;
-      float kim = 0.0f;
-      if (alive) {
-        // endpoint bound on the survivors (FP64, the end samples normalised)
-        const double mi = S.mu[i], si = S.isg[i], mj = S.mu[j], sj = S.isg[j];
-        double qv[6], tv[6];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          qv[k] = (S.a[i + k] - mi) * si;
-          qv[3 + k] = (S.a[i + m - 3 + k] - mi) * si;
-          tv[k] = (S.a[j + k] - mj) * sj;
-          tv[3 + k] = (S.a[j + m - 3 + k] - mj) * sj;
-        }
-        double dl, dr;
-        kim_bound<double>(Ends6{qv}, Ends6{tv}, 6, &dl, &dr);
-        kim = (float)(dl + dr);
-        if (dl + dr > (double)thr) {
-          alive = false;
-          ++nkim;
-        }
-      }
-      const unsigned int sv = __ballot_sync(0xffffffffu, alive);
-      if (sv) {
-        unsigned int base = 0;
-        if (lane == 0) base = atomicAdd(Q.kq_count, (unsigned int)__popc(sv));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (alive) {
-          const unsigned int slot = base + __popc(sv & ((1u << lane) - 1u));
-          if (slot < Q.kq_cap) {
-            Q.kq[slot] = make_int4(i, j, __float_as_int(kim), T.series);
-          } else {
-            atomicOr(S.status, 2);
-          }
-        }
-      }
+      push_survivor(S, Q, T, live && !pruned, i, j, thr, lane, nkim);
     }
   }
   unsigned long long a = npaa, b = nkim;
@@ -513,6 +517,142 @@ __global__ void __launch_bounds__(kPaaWarps * 32, 3) k_paa_lags(DevSeries S, Dev
   if (threadIdx.x == 0) {
     if (cnt_paa) atomicAdd(&Q.counters[kPrunedPaa], cnt_paa);
     if (cnt_kim) atomicAdd(&Q.counters[kPrunedKim], cnt_kim);
+  }
+}
+
+// The block-mean bound over the pairs of the group filter's surviving groups,
+// in the tiles that did not go through the diagonal bound.  A warp takes one
+// entry of the group list at a time (up to 16 group pairs), and of it one
+// group pair (g = 8: 64 pairs, two per lane, rows r and r + 4 of the row group
+// against one window of the column group) or two (g = 4: 16 pairs each, one
+// per lane); consecutive windows read consecutive block means.  The block
+// terms, their order and the endpoint bound are those of k_paa_lags.
+template <int B, int G>
+__global__ void __launch_bounds__(kPaaWarps * 32, 3) k_paa_groups(DevSeries S, DevSearch Q,
+                                                                  GroupFilter F, const Tile* tiles,
+                                                                  unsigned int* next) {
+  constexpr int R = G == 8 ? 2 : 1;  // pairs per lane
+  __shared__ unsigned long long cnt_paa, cnt_kim, cnt_seen;
+  if (threadIdx.x == 0) cnt_paa = cnt_kim = cnt_seen = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int m = S.m;
+  const int nb = m / B;
+  const float INF = __int_as_float(0x7f800000);
+  const unsigned int total = *F.nlist;
+  unsigned int npaa = 0, nkim = 0, nseen = 0;
+  for (;;) {
+    unsigned int e = 0;
+    if (lane == 0) e = atomicAdd(next, 1u);
+    e = __shfl_sync(0xffffffffu, e, 0);
+    if (e >= total) break;
+    const uint2 en = F.list[e];
+    const unsigned int tk = group_code_tile(en.x);
+    const Tile T = tiles[tk];
+    if (group_tile_dense(T, G, F.tcount[tk])) continue;
+    const GroupPair gp = group_code_pair(en.x, T, kGrpFan * G);
+    const float thr = prune_threshold_now(Q.bsf2 + T.series, m);
+    const float r_ok = fp32_bound_radius(thr, m);
+    unsigned int wv = en.y;
+    while (wv) {
+      int b = __ffs(wv) - 1;
+      wv &= wv - 1u;
+      bool on = true;
+      if (G == 4) {
+        // the upper half warp takes the next group pair, if there is one
+        const int b2 = wv ? __ffs(wv) - 1 : -1;
+        if (wv) wv &= wv - 1u;
+        if (lane >= 16) {
+          on = b2 >= 0;
+          if (on) b = b2;
+        }
+      }
+      const int j = (gp.J * kGrpFan + (b & 3)) * G + (lane & (G - 1));
+      const int ir = (gp.I * kGrpFan + (b >> 2)) * G + (G == 8 ? lane >> 3 : (lane & 15) >> 2);
+      bool live[R], pruned[R];
+      int i[R];
+      float thr_lane[R], o[R], fsi[R], acc1[R], acc2[R];
+      const float4* pi[R];
+      // a lane without a pair reads a valid address and ignores the result
+      const int jv = j < T.send ? j : T.send - 1;
+      const float4 wrj = S.wrec[jv];
+      const float fsj = wrj.z;
+      const double oj = __hiloint2double(__float_as_int(wrj.y), __float_as_int(wrj.x));
+      const float4* pj = S.pq2 + (win_copy(jv, m) ? S.n : 0) + jv;
+      bool all = true;
+#pragma unroll
+      for (int x = 0; x < R; ++x) {
+        const int ix = ir + 4 * x;
+        const int row = ix - T.i0, lag = j - ix - T.L0;
+        live[x] = on && row >= 0 && row < T.rows && j < T.send && lag >= 0 && lag < kLbLags;
+        i[x] = live[x] ? ix : T.i0;
+        const float4 wri = S.wrec[i[x]];
+        if (wri.z == 0.0f || fsj == 0.0f) live[x] = false;  // a flat window: no pair
+        nseen += live[x] ? 1u : 0u;
+        thr_lane[x] = live[x] && wri.w <= r_ok && wrj.w <= r_ok ? thr : INF;
+        o[x] = (float)(__hiloint2double(__float_as_int(wri.y), __float_as_int(wri.x)) - oj);
+        fsi[x] = wri.z;
+        pi[x] = S.pq2 + (win_copy(i[x], m) ? S.n : 0) + i[x];
+        acc1[x] = acc2[x] = 0.0f;
+        pruned[x] = !live[x];
+        all = all && pruned[x];
+      }
+      if (__all_sync(0xffffffffu, all)) continue;
+      // stride-4 order, a vote after every four blocks
+#pragma unroll 1
+      for (int r4 = 0; r4 < 4; ++r4) {
+        int k = r4;
+        const float4* qj = pj + r4 * B;
+        const float4* qi[R];
+#pragma unroll
+        for (int x = 0; x < R; ++x) qi[x] = pi[x] + r4 * B;
+        for (; k < nb; k += 16) {
+          // the group's four blocks (fewer at the end)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (k + 4 * u < nb) {
+              const float4 bj = qj[4 * u * B];
+#pragma unroll
+              for (int x = 0; x < R; ++x)
+                block_terms(qi[x][4 * u * B], bj, fsi[x], fsj, o[x], acc1[x], acc2[x]);
+            }
+          }
+          all = true;
+          qj += 16 * B;
+#pragma unroll
+          for (int x = 0; x < R; ++x) {
+            qi[x] += 16 * B;
+            pruned[x] = pruned[x] || (float)B * fmaxf(acc1[x], acc2[x]) > thr_lane[x];
+            all = all && pruned[x];
+          }
+          if (__all_sync(0xffffffffu, all)) break;
+        }
+        if (k < nb) break;  // every lane pruned
+      }
+#pragma unroll
+      for (int x = 0; x < R; ++x) {
+        npaa += (live[x] && pruned[x]) ? 1u : 0u;
+        push_survivor(S, Q, T, live[x] && !pruned[x], i[x], j, thr, lane, nkim);
+      }
+    }
+  }
+  unsigned long long a = npaa, b = nkim, c = nseen;
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+    c += __shfl_xor_sync(0xffffffffu, c, o);
+  }
+  if (lane == 0) {
+    if (a) atomicAdd(&cnt_paa, a);
+    if (b) atomicAdd(&cnt_kim, b);
+    if (c) atomicAdd(&cnt_seen, c);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (cnt_paa) atomicAdd(&Q.counters[kPrunedPaa], cnt_paa);
+    if (cnt_kim) atomicAdd(&Q.counters[kPrunedKim], cnt_kim);
+    // the sweep counted every pair of a sparse tile as pruned
+    if (cnt_seen) atomicAdd(&Q.counters[kPrunedFast], 0ull - cnt_seen);
   }
 }
 
@@ -535,15 +675,15 @@ int launch_paa_prep(const DevSeries& S, cudaStream_t st) {
   return 5;
 }
 
-void launch_paa(const DevSeries& S, const DevSearch& Q, const Tile* tiles, int tile_begin,
-                int tile_end, const unsigned int* bits, int num_sms, cudaStream_t st) {
+void launch_paa(const DevSeries& S, const DevSearch& Q, const GroupFilter& F, const Tile* tiles,
+                int tile_begin, int tile_end, const unsigned int* bits, int num_sms,
+                cudaStream_t st) {
   if (tile_end <= tile_begin) return;
-  const unsigned int items = (unsigned int)(tile_end - tile_begin) * kLbWords * kLbGroups;
   auto go = [&](auto kern) {
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPaaWarps * 32, 0);
     if (per_sm < 1) per_sm = 1;
-    kern<<<num_sms * per_sm, kPaaWarps * 32, 0, st>>>(S, Q, tiles + tile_begin, bits, items);
+    kern<<<num_sms * per_sm, kPaaWarps * 32, 0, st>>>(S, Q, F, tiles + tile_begin, bits);
   };
   // windows of at most 1024 samples: lanes on lags (window-relative blocks,
   // no per-lane window ends); longer windows: lanes on rows
@@ -556,6 +696,21 @@ void launch_paa(const DevSeries& S, const DevSearch& Q, const Tile* tiles, int t
     else if (S.paa_b == 16) go(k_paa<16>);
     else go(k_paa<8>);
   }
+}
+
+void launch_paa_groups(const DevSeries& S, const DevSearch& Q, const GroupFilter& F,
+                       const Tile* tiles, int tile_begin, unsigned int* next, int num_sms,
+                       cudaStream_t st) {
+  auto go = [&](auto kern) {
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPaaWarps * 32, 0);
+    if (per_sm < 1) per_sm = 1;
+    kern<<<num_sms * per_sm, kPaaWarps * 32, 0, st>>>(S, Q, F, tiles + tile_begin, next);
+  };
+  // group_windows and paa_block change at the same window lengths
+  if (S.paa_b == 32) go(k_paa_groups<32, 8>);
+  else if (S.paa_b == 16) go(k_paa_groups<16, 8>);
+  else go(k_paa_groups<8, 4>);
 }
 
 }  // namespace dtwj
