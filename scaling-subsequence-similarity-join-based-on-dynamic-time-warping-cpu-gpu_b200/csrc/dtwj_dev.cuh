@@ -236,6 +236,9 @@ struct GroupFilter {
                          //   kGrpFan x kGrpFan group pairs)
   unsigned int* nlist;
   unsigned int* tcount;  // surviving group pairs per tile (nullptr: no filter, every tile dense)
+  unsigned int sup_cap, list_cap;
+  const float* cut;      // seeds only: the cutoff on ED^2 ...
+  unsigned int* walk;    // ... and whether the diagonals must be walked after all
   unsigned int* dense;   // tiles the diagonal sweep ran on
   unsigned int* ndense;
   int nib, nw;           // first-level work items per tile: blocks of row groups x column words
@@ -371,8 +374,19 @@ void launch_seed_select(const DevSeries& S, const unsigned long long* keys, int2
 // Row minima for the join's seeds on the rows of a kSeedGrid grid: FP64
 // anchors and stage carries, FP32 increments within a stage (keys only rank
 // the seed candidates).
+// walk (nullptr: always): the kernel returns at once while *walk is zero, and
+// adds to the keys instead of starting from empty ones.
 void launch_mp_seed(const DevSeries& S, const Tile* tiles, int ntiles, unsigned long long* keys,
-                    cudaStream_t st);
+                    const unsigned int* walk, int num_sms, cudaStream_t st);
+// The same keys for the rows that can be among the kSeeds smallest, by the
+// group bound (group.cu).  F: lists of sup_cap and list_cap entries, nsup,
+// nlist, tcount (one word: the group pair count) consecutive, cut and walk;
+// samples: kSeedSamples floats.  Single series.
+constexpr int kSeedSamples = 2048;
+constexpr int kSeedSlab = 16384;  // tiles per pass
+void launch_seed_groups(const DevSeries& S, GroupFilter F, const Tile* tiles, int ntiles,
+                        int world, float* samples, unsigned long long* keys, int num_sms,
+                        cudaStream_t st);
 // Series of a sample (0 for a single series).
 __device__ __forceinline__ int series_of(const DevSeries& S, int64_t x) {
   return S.sid ? S.sid[x] : 0;

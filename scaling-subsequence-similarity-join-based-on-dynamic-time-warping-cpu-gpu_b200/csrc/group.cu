@@ -88,8 +88,16 @@ __global__ void k_group_rec(DevSeries S, const double* gm, SegOrder ord) {
   S.grp[(int64_t)slot * S.grp_n + G] = rec;
 }
 
-// Both directions of one segment of a group pair.
+// One segment of a group pair: both directions of the block-mean bound, or
+// (ED) the bound on the z-normalised Euclidean distance of the group's pairs,
+// whose envelopes are the windows themselves.
+template <bool ED>
 __device__ __forceinline__ void group_terms(const float4 i, const float4 j, float& a1, float& a2) {
+  if (ED) {
+    const float d = max3f(i.x - j.y, j.x - i.y, 0.0f);
+    a1 = fmaf(d, d, a1);
+    return;
+  }
   const float d1 = max3f(i.x - j.z, j.w - i.y, 0.0f);
   a1 = fmaf(d1, d1, a1);
   const float d2 = max3f(j.x - i.z, i.w - j.y, 0.0f);
@@ -111,6 +119,7 @@ __device__ __forceinline__ unsigned int append_slot(bool on, int lane, unsigned 
 // row, the I loads are broadcasts.  The slots are in an order that spreads
 // the first ones over the window; the warp votes every four.
 constexpr int kSupRows = 4;
+template <bool ED>
 __global__ void __launch_bounds__(kThreads) k_group_super(DevSeries S, DevSearch Q, GroupFilter F,
                                                           const Tile* tiles, unsigned int total) {
   const int lane = threadIdx.x & 31;
@@ -131,7 +140,7 @@ __global__ void __launch_bounds__(kThreads) k_group_super(DevSeries S, DevSearch
   for (int r = 0; r < kSupRows; ++r)
     if (group_pair_in_tile(T, g, I0 + r, J0 + r)) alive |= 1u << r;
   if (!__any_sync(0xffffffffu, alive != 0u)) return;
-  const float thr = prune_threshold_now(Q.bsf2 + T.series, S.m);
+  const float thr = ED ? *F.cut : prune_threshold_now(Q.bsf2 + T.series, S.m);
   const float fb = (float)S.grp_b;
   const int64_t n = S.sup_n;
   // addresses past the last record repeat it (those group pairs are not
@@ -149,7 +158,7 @@ __global__ void __launch_bounds__(kThreads) k_group_super(DevSeries S, DevSearch
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
 #pragma unroll
-      for (int r = 0; r < kSupRows; ++r) group_terms(pi[u * n + r], pj[r][u * n], a1[r], a2[r]);
+      for (int r = 0; r < kSupRows; ++r) group_terms<ED>(pi[u * n + r], pj[r][u * n], a1[r], a2[r]);
     }
     pi += 4 * n;
 #pragma unroll
@@ -163,17 +172,18 @@ __global__ void __launch_bounds__(kThreads) k_group_super(DevSeries S, DevSearch
   for (int r = 0; r < kSupRows; ++r) {
     const bool on = (alive >> r) & 1u;
     const unsigned int slot = append_slot(on, lane, F.nsup);
-    if (on) F.sup[slot] = group_code(tk, row0 + r, col);
+    if (on && slot < F.sup_cap) F.sup[slot] = group_code(tk, row0 + r, col);
   }
 }
 
 // Second level: half a warp per surviving super-group pair, one lane per
 // pair of its kGrpFan x kGrpFan groups.
+template <bool ED>
 __global__ void __launch_bounds__(kThreads) k_group(DevSeries S, DevSearch Q, GroupFilter F,
                                                     const Tile* tiles) {
   static_assert(kGrpFan == 4, "16 group pairs, half a warp");
   const int lane = threadIdx.x & 31, h = lane & 15;
-  const unsigned int total = *F.nsup;
+  const unsigned int total = *F.nsup < F.sup_cap ? *F.nsup : F.sup_cap;
   const int g = S.grp_g, G = kGrpFan * g;
   const float fb = (float)S.grp_b;
   const int64_t n = S.grp_n;
@@ -186,14 +196,14 @@ __global__ void __launch_bounds__(kThreads) k_group(DevSeries S, DevSearch Q, Gr
     const GroupPair p = group_code_pair(code, T, G);
     const int I = p.I * kGrpFan + (h >> 2), J = p.J * kGrpFan + (h & 3);
     bool alive = e < total && group_pair_in_tile(T, g, I, J);
-    const float thr = prune_threshold_now(Q.bsf2 + T.series, S.m);
+    const float thr = ED ? *F.cut : prune_threshold_now(Q.bsf2 + T.series, S.m);
     const float4* pi = S.grp + (I < n ? I : n - 1);
     const float4* pj = S.grp + (J < n ? J : n - 1);
     float a1 = 0.0f, a2 = 0.0f;
 #pragma unroll 1
     for (int s0 = 0; s0 < S.grp_d && __any_sync(0xffffffffu, alive); s0 += 4) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) group_terms(pi[u * n], pj[u * n], a1, a2);
+      for (int u = 0; u < 4; ++u) group_terms<ED>(pi[u * n], pj[u * n], a1, a2);
       pi += 4 * n;
       pj += 4 * n;
       alive = alive && !(fb * fmaxf(a1, a2) > thr);
@@ -201,10 +211,8 @@ __global__ void __launch_bounds__(kThreads) k_group(DevSeries S, DevSearch Q, Gr
     const unsigned int mask = (__ballot_sync(0xffffffffu, alive) >> (lane & 16)) & 0xffffu;
     const bool on = h == 0 && mask != 0u;
     const unsigned int slot = append_slot(on, lane, F.nlist);
-    if (on) {
-      F.list[slot] = make_uint2(code, mask);
-      atomicAdd(&F.tcount[tk], (unsigned int)__popc(mask));
-    }
+    if (on && slot < F.list_cap) F.list[slot] = make_uint2(code, mask);
+    if (on) atomicAdd(ED ? F.tcount : F.tcount + tk, (unsigned int)__popc(mask));
   }
 }
 
@@ -299,19 +307,212 @@ size_t group_items(int g, GroupFilter* F) {
   return (size_t)rows * cols;
 }
 
+namespace {
+template <bool ED>
+void run_group(const DevSeries& S, const DevSearch& Q, const GroupFilter& F, const Tile* tiles,
+               int ntiles, int num_sms, cudaStream_t st) {
+  const unsigned int items = (unsigned int)ntiles * (unsigned)(F.nib * F.nw);
+  k_group_super<ED><<<(items + kThreads / 32 - 1) / (kThreads / 32), kThreads, 0, st>>>(
+      S, Q, F, tiles, items);
+  k_group<ED><<<num_sms * 8, kThreads, 0, st>>>(S, Q, F, tiles);
+}
+}  // namespace
+
 void launch_group(const DevSeries& S, const DevSearch& Q, const GroupFilter& F, const Tile* tiles,
                   int tile_begin, int tile_end, int num_sms, cudaStream_t st) {
-  if (tile_end <= tile_begin) return;
-  const unsigned int items = (unsigned int)(tile_end - tile_begin) * (unsigned)(F.nib * F.nw);
-  k_group_super<<<(items + kThreads / 32 - 1) / (kThreads / 32), kThreads, 0, st>>>(
-      S, Q, F, tiles + tile_begin, items);
-  k_group<<<num_sms * 8, kThreads, 0, st>>>(S, Q, F, tiles + tile_begin);
+  if (tile_end > tile_begin)
+    run_group<false>(S, Q, F, tiles + tile_begin, tile_end - tile_begin, num_sms, st);
 }
 
 void launch_group_bits(const DevSeries& S, const DevSearch& Q, const GroupFilter& F,
                        const Tile* tiles, int tile_begin, int num_sms, unsigned int* bits,
                        cudaStream_t st) {
   k_group_bits<<<num_sms * 8, kThreads, 0, st>>>(S, Q, F, tiles + tile_begin, bits);
+}
+
+// ---- seeds of a large join ----
+//
+// The seeds are the kSeeds grid rows with the smallest ED to a later window
+// (mp.cu).  Walking every diagonal for them (k_mp_seed) takes 0.2 ps per pair:
+// 100 ms of the 1M-sample bench join once the sweep takes 30.  The group
+// bound finds the same rows: with a cutoff c on ED^2, every pair below c lies
+// in a group pair whose bound is at most c, and only those pairs are measured.
+// c comes from a sample of row groups: each one's closest pair among its best
+// group pair, and of these values the one that should leave a few times kSeeds
+// rows below it.  Where the bound settles too little (it would cost more than
+// walking the diagonals: quasi-periodic series) or a list overflows,
+// *F.walk is set and k_mp_seed walks them after all.
+
+namespace {
+
+// Smallest group-pair bound of sampled row groups (one block each) over all
+// later column groups, then the smallest ED^2 of the pairs of that group pair.
+__global__ void __launch_bounds__(kThreads) k_seed_sample(DevSeries S, int64_t stride,
+                                                          float* best_ed) {
+  const int t = threadIdx.x, lane = t & 31;
+  const int g = S.grp_g, m = S.m;
+  const int64_t I = (int64_t)blockIdx.x * stride, n = S.grp_n;
+  const int64_t ng = (S.s + g - 1) / g;
+  __shared__ unsigned long long red[kThreads / 32];
+  __shared__ float4 rec[kGrpSlots];
+  if (t < S.grp_d) rec[t] = S.grp[t * n + I];
+  __syncthreads();
+  const float fb = (float)S.grp_b;
+  float best = __int_as_float(0x7f800000);
+  int64_t at = -1;
+  for (int64_t J = (I * g + m + g - 1) / g + t; J < ng; J += kThreads) {
+    float acc = 0.0f, unused = 0.0f;
+    for (int s0 = 0; s0 < S.grp_d; s0 += 4) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) group_terms<true>(rec[s0 + u], S.grp[(s0 + u) * n + J], acc, unused);
+      if (fb * acc >= best) break;
+    }
+    if (fb * acc < best) {
+      best = fb * acc;
+      at = J;
+    }
+  }
+  unsigned long long k = at < 0 ? ~0ull
+                                : ((unsigned long long)__float_as_uint(best) << 32) | (unsigned int)at;
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long v = __shfl_xor_sync(0xffffffffu, k, o);
+    k = v < k ? v : k;
+  }
+  if (lane == 0) red[t >> 5] = k;
+  __syncthreads();
+  if (t == 0) {
+    for (int w = 1; w < kThreads / 32; ++w) red[0] = red[w] < red[0] ? red[w] : red[0];
+  }
+  __syncthreads();
+  k = red[0];
+  __syncthreads();
+  float ed = __int_as_float(0x7f800000);
+  if (k != ~0ull) {
+    const int64_t j0 = (int64_t)(k & 0xffffffffu) * g;
+    for (int x = t >> 5; x < g * g; x += kThreads / 32) {
+      const int64_t i = I * g + x / g, j = j0 + x % g;
+      if (i >= S.s || j >= S.s || S.flat[i] || S.flat[j]) continue;
+      const double mi = S.mu[i], si = S.isg[i], mj = S.mu[j], sj = S.isg[j];
+      double d2 = 0.0;
+      for (int q = lane; q < m; q += 32) {
+        const double d = (S.a[i + q] - mi) * si - (S.a[j + q] - mj) * sj;
+        d2 = fma(d, d, d2);
+      }
+      for (int o = 16; o > 0; o >>= 1) d2 += __shfl_xor_sync(0xffffffffu, d2, o);
+      ed = fminf(ed, (float)d2);
+    }
+  }
+  if (lane == 0) red[t >> 5] = __float_as_uint(ed);
+  __syncthreads();
+  if (t == 0) {
+    for (int w = 1; w < kThreads / 32; ++w) red[0] = red[w] < red[0] ? red[w] : red[0];
+    best_ed[blockIdx.x] = __uint_as_float((unsigned int)red[0]);
+  }
+}
+
+// cut = the rank-th smallest of the count sampled values (lowest index on
+// ties), rounded up past the FP32 error of the bound.
+__global__ void __launch_bounds__(1024) k_seed_cut(const float* v, int count, int rank, float* cut) {
+  for (int x = threadIdx.x; x < count; x += blockDim.x) {
+    const float mine = v[x];
+    int below = 0;
+    for (int y = 0; y < count; ++y) below += v[y] < mine || (v[y] == mine && y < x) ? 1 : 0;
+    if (below == rank) *cut = mine * (1.0f + 1.0f / 4096.0f) + 1e-6f;
+  }
+}
+
+// Exact ED^2 (FP64 centered dot product) of the grid rows of the surviving
+// group pairs against their column windows, one warp per row and column
+// group; the row's key takes the smallest, in the format of k_mp.
+template <int G>
+__global__ void __launch_bounds__(kThreads) k_seed_exact(DevSeries S, GroupFilter F,
+                                                         const Tile* tiles, unsigned int budget,
+                                                         unsigned long long* keys) {
+  const int lane = threadIdx.x & 31;
+  const unsigned int total = *F.nlist;
+  // too many group pairs, or some were dropped: the diagonals are walked instead
+  if (total > F.list_cap || *F.nsup > F.sup_cap || *F.tcount > budget) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *F.walk = 1u;
+    return;
+  }
+  const int m = S.m;
+  const double two_m = 2.0 * m;
+  for (unsigned int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < total;
+       e += (gridDim.x * blockDim.x) >> 5) {
+    const uint2 en = F.list[e];
+    const Tile T = tiles[group_code_tile(en.x)];
+    const GroupPair p = group_code_pair(en.x, T, kGrpFan * G);
+    for (unsigned int mask = en.y; mask; mask &= mask - 1u) {
+      const int b = __ffs(mask) - 1;
+      const int ia = (p.I * kGrpFan + (b >> 2)) * G, j0 = (p.J * kGrpFan + (b & 3)) * G;
+      // rows of the series' grid (a single series starts at window 0)
+      for (int i = (ia + kSeedGrid - 1) / kSeedGrid * kSeedGrid; i < ia + G; i += kSeedGrid) {
+        if (i < T.i0 || i >= T.i0 + T.rows || S.flat[i]) continue;
+        const double mi = S.mu[i];
+        double c[G], mj[G];
+#pragma unroll
+        for (int x = 0; x < G; ++x) {
+          c[x] = 0.0;
+          mj[x] = S.mu[j0 + x < T.send ? j0 + x : T.send - 1];
+        }
+        for (int k = lane; k < m; k += 32) {
+          const double ai = S.a[i + k] - mi;
+#pragma unroll
+          for (int x = 0; x < G; ++x) {
+            const int64_t q = (int64_t)j0 + x + k;
+            c[x] = fma(ai, S.a[q < S.n ? q : S.n - 1] - mj[x], c[x]);
+          }
+        }
+#pragma unroll
+        for (int x = 0; x < G; ++x)
+          for (int o = 16; o > 0; o >>= 1) c[x] += __shfl_xor_sync(0xffffffffu, c[x], o);
+        // lane x finishes pair x
+        double mine = 0.0;
+#pragma unroll
+        for (int x = 0; x < G; ++x)
+          if (lane == x) mine = c[x];
+        const int j = j0 + lane, lag = j - i - T.L0;
+        if (lane < G && j < T.send && lag >= 0 && lag < kLbLags && !S.flat[j]) {
+          const double e2 = fmax(two_m - 2.0 * mine * S.isg[i] * S.isg[j], 0.0);
+          const unsigned int hi = (unsigned int)__double2hiint(e2) & ~7u;
+          atomicMin(&keys[i], ((unsigned long long)hi << 32) | (unsigned int)j);
+        }
+      }
+    }
+  }
+}
+
+}  // namespace
+
+void launch_seed_groups(const DevSeries& S, GroupFilter F, const Tile* tiles, int ntiles,
+                        int world, float* samples, unsigned long long* keys, int num_sms,
+                        cudaStream_t st) {
+  cudaMemsetAsync(keys, 0xff, (size_t)S.s * 8, st);
+  cudaMemsetAsync(F.walk, 0, 4, st);
+  // one row group in `stride`, at most kSeedSamples; the rank that should
+  // leave 4 kSeeds grid rows (of this shard) below the cutoff, at least 4 deep
+  const int64_t ng = (S.s + S.grp_g - 1) / S.grp_g, rows = (S.s + kSeedGrid - 1) / kSeedGrid;
+  int64_t stride = 64;
+  while ((ng + stride - 1) / stride > kSeedSamples) stride *= 2;
+  const int count = (int)((ng + stride - 1) / stride);
+  int64_t rank = 4ll * kSeeds * world * count / rows;
+  if (rank < 4) rank = 4;
+  if (rank > count - 1) rank = count - 1;
+  k_seed_sample<<<count, kThreads, 0, st>>>(S, stride, samples);
+  k_seed_cut<<<1, 1024, 0, st>>>(samples, count, (int)rank, const_cast<float*>(F.cut));
+  for (int b = 0; b < ntiles; b += kSeedSlab) {
+    const int cnt = ntiles - b < kSeedSlab ? ntiles - b : kSeedSlab;
+    cudaMemsetAsync(F.nsup, 0, 12, st);  // nsup, nlist and the group pair count
+    run_group<true>(S, DevSearch{}, F, tiles + b, cnt, num_sms, st);
+    // a group pair costs about 1000 (g = 8) or 300 (g = 4) warp instructions,
+    // walking a diagonal about 0.23 per pair: the budget is half of that
+    const double pairs = (double)cnt * kLbLags * kLbRows;
+    const unsigned int budget = (unsigned int)(pairs / (S.grp_g == 8 ? 8192.0 : 4096.0));
+    if (S.grp_g == 8)
+      k_seed_exact<8><<<num_sms * 8, kThreads, 0, st>>>(S, F, tiles + b, budget, keys);
+    else
+      k_seed_exact<4><<<num_sms * 8, kThreads, 0, st>>>(S, F, tiles + b, budget, keys);
+  }
 }
 
 }  // namespace dtwj

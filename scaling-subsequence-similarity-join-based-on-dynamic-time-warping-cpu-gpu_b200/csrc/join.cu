@@ -51,6 +51,14 @@ constexpr int kLbChunkRounds = 4;
 // million per tile by that join's stage counts, so 32 tiles fit the LB_Keogh
 // queue (2^27 entries) and 55 would not.
 constexpr int kResweepTiles = 32;
+// Tiles from which the seeds come from the group bound instead of a walk over
+// every diagonal.
+constexpr int kSeedGroupTiles = 1024;
+// Their lists of group pairs, and with the samples and five words the bytes
+// they take.
+constexpr unsigned int kSeedSupCap = 1u << 24, kSeedListCap = 1u << 22;
+constexpr size_t kSeedScratch =
+    (size_t)kSeedSupCap * 4 + (size_t)kSeedListCap * sizeof(uint2) + kSeedSamples * 4 + 64;
 // (m, w) groups of a batch joined at the same time, one context each.
 constexpr int kBatchWorkers = 4;
 
@@ -510,6 +518,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     const size_t pairs = (size_t)chunk_max * group_items(S.grp_g, &F);
     ENSURE(B_GSUP, pairs * 4, F.sup);
     ENSURE(B_GLIST, pairs * sizeof(uint2), F.list);
+    F.sup_cap = F.list_cap = (unsigned int)pairs;
     F.tcount = qc + kQcTiles;
   }
   Q.queue_cap = qcap;
@@ -533,6 +542,9 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   unsigned int* seed_bsf;
   ENSURE(B_SEEDBSF, (size_t)nslots * 4, seed_bsf);
 
+  unsigned int* bits;
+  ENSURE(B_BITS, (size_t)chunk_max * kLbLags * kLbWords * 4, bits);
+
   // ---- ED matrix profile (row minima; per tile for the tile minima) ----
   const bool want_features = learned || (tq && tq->features);
   unsigned long long* keys = nullptr;
@@ -547,10 +559,34 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     // a join only ranks seed candidates by these keys (mixed precision, one
     // row in kSeedGrid); the per-tile minima and the exported features take
     // the exact FP64 profile of every row
-    if (tq) launch_mp(S, lbtiles, nlb, keys, st, tbest);
-    else launch_mp_seed(S, lbtiles, nlb, keys, st);
+    int launches = 2;
+    if (tq) {
+      launch_mp(S, lbtiles, nlb, keys, st, tbest);
+    } else if (S.grp && !sbeg && !learned && nlb >= kSeedGroupTiles &&
+               (size_t)chunk_max * kLbLags * kLbWords * 4 >= kSeedScratch) {
+      // a large join: the group bound finds the rows; its lists lie in the
+      // survivor bits' buffer, which the sweep uses later
+      GroupFilter E = F;
+      E.sup_cap = kSeedSupCap;
+      E.list_cap = kSeedListCap;
+      E.sup = bits;
+      E.list = reinterpret_cast<uint2*>(bits + kSeedSupCap);
+      float* samples = reinterpret_cast<float*>(E.list + kSeedListCap);
+      unsigned int* word = reinterpret_cast<unsigned int*>(samples + kSeedSamples);
+      E.nsup = word;
+      E.nlist = word + 1;
+      E.tcount = word + 2;
+      E.walk = word + 3;
+      E.cut = reinterpret_cast<const float*>(word + 4);
+      launch_seed_groups(S, E, lbtiles, nlb, ctx->shard_world, samples, keys, ctx->num_sms, st);
+      launch_mp_seed(S, lbtiles, nlb, keys, E.walk, ctx->num_sms, st);
+      launches = 3 + 3 * ((nlb + kSeedSlab - 1) / kSeedSlab);
+    } else {
+      launch_mp_seed(S, lbtiles, nlb, keys, nullptr, ctx->num_sms, st);
+      launches = 1;
+    }
     if (tile_mode) launch_tile_bound(tbest, nlb, Q.bsf2, st);
-    ph.end(DTWJ_PHASE_PROFILE, 2);
+    ph.end(DTWJ_PHASE_PROFILE, launches);
   }
   // ---- tile features; the learned order sorts the tiles by their score ----
   if (want_features && nlb > 0) {
@@ -616,8 +652,6 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   CUDA_OK(cudaMemcpyAsync(seed_bsf, Q.bsf2, (size_t)nslots * 4, cudaMemcpyDeviceToDevice, st));
 
   // ---- diagonal sweep in chunks of LB tiles ----
-  unsigned int* bits;
-  ENSURE(B_BITS, (size_t)chunk_max * kLbLags * kLbWords * 4, bits);
   // the stages after the diagonal bound of one chunk: run filter, LB_Keogh, DTW
   auto filter_chunk = [&](int t0, int t1) {
     ph.begin();

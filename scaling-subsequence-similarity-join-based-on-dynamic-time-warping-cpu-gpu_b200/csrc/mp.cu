@@ -221,6 +221,8 @@ __global__ void __launch_bounds__(kLbThreads, 4) k_mp(DevSeries S, const Tile* t
 static_assert(kSeedGrid == kLbPerThread, "grid rows are the first of each unrolled group");
 static_assert(kLbRows % kSeedGrid == 0 && kStage % kSeedGrid == 0, "tiles and stages on the grid");
 
+constexpr int kSeedCtasPerSm = 6;  // launch bounds of k_mp_seed
+
 struct MpSeedShared {
   float2 p[kCols];   // (dfa, dga) of column j - 1: one 8-byte read per row and thread
   float is[kCols], c2[kCols];
@@ -228,36 +230,80 @@ struct MpSeedShared {
   unsigned long long rowbest[kStage / kSeedGrid];
 };
 
-__global__ void __launch_bounds__(kLbThreads, 6) k_mp_seed(DevSeries S, const Tile* tiles,
-                                                           unsigned long long* keys) {
+// A block takes `part` stages of a tile (blockIdx.x: tile, blockIdx.y: part of
+// it), all 18 when the tiles alone fill the GPU.  Each part starts from its
+// own exact anchors, so a tile is cut only as far as that pays: a series of
+// 20,000 samples has 74 tiles, and one block per tile walked 4,032 rows one
+// after another on half of the SMs (0.26 ms).
+__global__ void __launch_bounds__(kLbThreads, kSeedCtasPerSm) k_mp_seed(DevSeries S,
+                                                                      const Tile* tiles, int part,
+                                                                      unsigned long long* keys,
+                                                                      const unsigned int* walk) {
   extern __shared__ __align__(16) unsigned char smraw[];
   MpSeedShared& sh = *reinterpret_cast<MpSeedShared*>(smraw);
-  const Tile T = tiles[blockIdx.x];
+  if (walk && *walk == 0u) return;
+  Tile T = tiles[blockIdx.x];
+  {
+    const int first = (int)blockIdx.y * part * kStage;
+    if (first >= T.rows) return;
+    T.i0 += first;
+    T.rows = T.rows - first < part * kStage ? T.rows - first : part * kStage;
+  }
   const int64_t s = T.send;
   const int m = S.m;
   const int t = threadIdx.x, lane = t & 31;
   const int64_t L0 = T.L0, i0 = T.i0;
   const int64_t Lt = L0 + (int64_t)t * kLbPerThread;
-  // exact anchors C(i0, i0 + L) for the thread's lags (FP64)
+  // exact anchors C(i0, i0 + L) = sum_k (a[i0+k] - mu_i) (a[j+k] - mu_j) for the
+  // thread's lags (FP64), the samples staged kStage at a time.  The columns
+  // are centered on one value c0 near their means when staged, which leaves
+  // one multiply-add per lag and sample; sum_k (a[i0+k] - mu_i), zero up to
+  // rounding, takes the rest of the centering.
   double C[kLbPerThread];
   {
-    double mj[kLbPerThread], wa[kLbPerThread];
-    const int64_t jb = i0 + Lt;
+    double* col = reinterpret_cast<double*>(sh.p);
+    double* row = reinterpret_cast<double*>(sh.r);
+    static_assert(sizeof sh.p >= kCols * sizeof(double) && sizeof sh.r >= kStage * sizeof(double),
+                  "staging fits");
+    const double mi = S.mu[i0];
+    const double c0 = S.mu[i0 + L0 + kLbLags / 2 < s ? i0 + L0 + kLbLags / 2 : s - 1];
+    const int cb = t * kLbPerThread;
+    double wa[kLbPerThread], rsum = 0.0;
+#pragma unroll
+    for (int l = 0; l < kLbPerThread; ++l) C[l] = 0.0;
+    for (int k0 = 0; k0 < m; k0 += kStage) {
+      const int cnt = m - k0 < kStage ? m - k0 : kStage;
+      __syncthreads();
+      for (int x = t; x < kCols; x += kLbThreads) {
+        const int64_t q = i0 + L0 + k0 + x;
+        col[x] = S.a[q < S.n ? q : S.n - 1] - c0;
+      }
+      for (int x = t; x < cnt; x += kLbThreads) row[x] = S.a[i0 + k0 + x] - mi;
+      __syncthreads();
+#pragma unroll
+      for (int l = 0; l < kLbPerThread; ++l) wa[l] = col[cb + l];
+      int k = 0;
+      for (; k + kLbPerThread <= cnt; k += kLbPerThread) {
+#pragma unroll
+        for (int u = 0; u < kLbPerThread; ++u) {
+          const double ai = row[k + u];
+          rsum += ai;
+#pragma unroll
+          for (int l = 0; l < kLbPerThread; ++l) C[l] = fma(ai, wa[(u + l) % kLbPerThread], C[l]);
+          wa[u] = col[cb + k + u + kLbPerThread];
+        }
+      }
+      for (; k < cnt; ++k) {
+        const double ai = row[k];
+        rsum += ai;
+#pragma unroll
+        for (int l = 0; l < kLbPerThread; ++l) C[l] = fma(ai, col[cb + k + l], C[l]);
+      }
+    }
 #pragma unroll
     for (int l = 0; l < kLbPerThread; ++l) {
-      C[l] = 0.0;
-      mj[l] = S.mu[jb + l < s ? jb + l : s - 1];
-      wa[l] = S.a[jb + l < S.n ? jb + l : S.n - 1];
-    }
-    const double mi = S.mu[i0];
-    for (int k = 0; k < m; ++k) {
-      const double ai = S.a[i0 + k] - mi;
-#pragma unroll
-      for (int l = 0; l < kLbPerThread; ++l) C[l] = fma(ai, wa[l] - mj[l], C[l]);
-#pragma unroll
-      for (int l = 0; l < kLbPerThread - 1; ++l) wa[l] = wa[l + 1];
-      const int64_t x = jb + kLbPerThread + k < S.n ? jb + kLbPerThread + k : S.n - 1;
-      wa[kLbPerThread - 1] = S.a[x];
+      const int64_t j = i0 + Lt + l < s ? i0 + Lt + l : s - 1;
+      C[l] = fma(c0 - S.mu[j], rsum, C[l]);
     }
   }
   float w1[kLbPerThread], w2[kLbPerThread];
@@ -461,97 +507,108 @@ __global__ void k_mp_want(int64_t s, const unsigned long long* up, const unsigne
 }
 
 constexpr int kSelThreads = 1024;
-constexpr int kLocal = 8;
 
-// kSeeds smallest row minima (by ED^2 key, then row index).  Each thread
-// keeps the kLocal best of a strided slice; kSeeds rounds of block minimum
-// then pop the global order.  Writes each seed pair with its diagonal
-// neighbours (kSeedSpread slots per seed, (-1, -1) where a neighbour leaves
-// the series) and the seed count.
+// kSeeds smallest row minima of a series (by ED^2 key, then row index), among
+// the rows of the seed grid: the keys' high words are narrowed to the kSeeds-th
+// smallest by four rounds of an 8-bit radix select in shared memory, then the
+// keys below it are taken, and of those equal to it the lowest rows.  Writes
+// each seed pair with its diagonal neighbours (kSeedSpread slots per seed,
+// (-1, -1) where a neighbour leaves the series) and the seed count.
 __global__ void __launch_bounds__(kSelThreads) k_seed_select(DevSeries S,
                                                               const unsigned long long* keys,
                                                               int2* seeds, unsigned int* nseeds) {
   // block b selects the seeds of series b (windows [wb, we))
-  const int b = blockIdx.x;
+  const int b = blockIdx.x, t = threadIdx.x, lane = t & 31;
   const int64_t wb = S.sbeg ? S.sbeg[b] : 0;
   const int64_t we = S.sbeg ? S.sbeg[b + 1] - S.m + 1 : S.s;
+  const int64_t rows = (we - wb + kSeedGrid - 1) / kSeedGrid;  // of the grid
   seeds += (size_t)b * kSeedSlots;
-  for (int x = threadIdx.x; x < kSeedSlots; x += blockDim.x) seeds[x] = make_int2(-1, -1);
-  unsigned long long loc[kLocal];
-  int part[kLocal];
+  for (int x = t; x < kSeedSlots; x += kSelThreads) seeds[x] = make_int2(-1, -1);
+  __shared__ unsigned int hist[256];
+  __shared__ unsigned int bin, below, taken, equal_base, wcount[kSelThreads / 32];
+  // prefix = the digits of the kSeeds-th smallest high word found so far;
+  // need = how many of the keys with that prefix are still to take
+  unsigned int prefix = 0, need = kSeeds;
+  for (int shift = 24; shift >= 0; shift -= 8) {
+    if (t < 256) hist[t] = 0;
+    __syncthreads();
+    for (int64_t r = t; r < rows; r += 4 * kSelThreads) {
+      unsigned int h[4];  // four loads in flight
 #pragma unroll
-  for (int q = 0; q < kLocal; ++q) { loc[q] = ULLONG_MAX; part[q] = -1; }
-  for (int64_t i = wb + threadIdx.x; i < we; i += blockDim.x) {
-    const unsigned long long k = keys[i];
-    if (k == ULLONG_MAX) continue;
-    const unsigned long long sk = (k & 0xffffffff00000000ull) | (unsigned long long)(unsigned int)i;
-    if (sk >= loc[kLocal - 1]) continue;
-    const int pj = (int)(k & 0xffffffffu);
-    // insertion into the ascending local list
-    bool done = false;
+      for (int u = 0; u < 4; ++u) {
+        const int64_t ru = r + u * kSelThreads;
+        h[u] = ru < rows ? (unsigned int)(keys[wb + ru * kSeedGrid] >> 32) : 0xffffffffu;
+      }
 #pragma unroll
-    for (int q = kLocal - 1; q > 0; --q) {
-      if (!done) {
-        if (loc[q - 1] > sk) {
-          loc[q] = loc[q - 1];
-          part[q] = part[q - 1];
-        } else {
-          loc[q] = sk;
-          part[q] = pj;
-          done = true;
-        }
+      for (int u = 0; u < 4; ++u) {
+        if (h[u] == 0xffffffffu) continue;  // no neighbour
+        if (shift == 24 || (h[u] >> (shift + 8)) == prefix)
+          atomicAdd(&hist[(h[u] >> shift) & 255u], 1u);
       }
     }
-    if (!done) {
-      loc[0] = sk;
-      part[0] = pj;
+    __syncthreads();
+    if (t < 32) {
+      // lane l sums bins 8 l .. 8 l + 7, a scan finds the lane and bin that
+      // reach `need` (none: fewer keys than that, the last bin stands)
+      unsigned int c[8], sum = 0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) sum += (c[q] = hist[8 * t + q]);
+      unsigned int inc = sum;
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (t >= o) inc += v;
+      }
+      const unsigned int reach = __ballot_sync(0xffffffffu, inc >= need);
+      const int who = reach ? __ffs(reach) - 1 : 31;
+      if (t == who) {
+        unsigned int acc = inc - sum;
+        int q = 0;
+        while (q < 7 && acc + c[q] < need) acc += c[q++];
+        bin = 8u * (unsigned int)t + (unsigned int)q;
+        below = acc;
+      }
     }
+    __syncthreads();
+    prefix = (prefix << 8) | bin;
+    need = need > below ? need - below : 0u;
+    __syncthreads();
   }
-  __shared__ unsigned long long red[kSelThreads / 32];
-  __shared__ unsigned long long winner;
-  int head = 0;
-  unsigned int count = 0;
-  for (int round = 0; round < kSeeds; ++round) {
-    // head of the local list (select through the unrolled registers)
-    unsigned long long v = ULLONG_MAX;
-#pragma unroll
-    for (int q = 0; q < kLocal; ++q) if (q == head) v = loc[q];
-    unsigned long long wv = v;
-    for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long t = __shfl_xor_sync(0xffffffffu, wv, o);
-      wv = t < wv ? t : wv;
+  if (t == 0) taken = 0, equal_base = 0;
+  __syncthreads();
+  // every key below the threshold, and the first `need` rows equal to it
+  unsigned long long ahead = t < rows ? keys[wb + (int64_t)t * kSeedGrid] : ULLONG_MAX;
+  for (int64_t r0 = 0; r0 < rows; r0 += kSelThreads) {
+    const int64_t r = r0 + t, rn = r + kSelThreads;
+    const unsigned long long k = ahead;
+    ahead = rn < rows ? keys[wb + rn * kSeedGrid] : ULLONG_MAX;
+    const unsigned int h = (unsigned int)(k >> 32);
+    const bool eq = h == prefix && h != 0xffffffffu;
+    bool take = h < prefix;
+    if (__syncthreads_or(eq)) {
+      const unsigned int eb = __ballot_sync(0xffffffffu, eq);
+      if (lane == 0) wcount[t >> 5] = __popc(eb);
+      __syncthreads();
+      unsigned int rank = equal_base + __popc(eb & ((1u << lane) - 1u));
+      for (int w = 0; w < (t >> 5); ++w) rank += wcount[w];
+      take = take || (eq && rank < need);
+      __syncthreads();
+      if (t == 0)
+        for (int w = 0; w < kSelThreads / 32; ++w) equal_base += wcount[w];
     }
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = wv;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      unsigned long long t = red[threadIdx.x];
-      for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long u = __shfl_xor_sync(0xffffffffu, t, o);
-        t = u < t ? u : t;
-      }
-      if (threadIdx.x == 0) winner = t;
-    }
-    __syncthreads();
-    const unsigned long long wn = winner;
-    if (wn == ULLONG_MAX) break;
-    if (v == wn) {
-      int pj = -1;
-#pragma unroll
-      for (int q = 0; q < kLocal; ++q) if (q == head) pj = part[q];
-      const int i = (int)(wn & 0xffffffffu);
+    if (take) {
+      const unsigned int slot = atomicAdd(&taken, 1u);
+      const int i = (int)(wb + r * kSeedGrid), pj = (int)(k & 0xffffffffu);
       const int lo = i < pj ? i : pj, hi = i < pj ? pj : i;
       // the pair and its diagonal neighbours that lie in the series
       for (int d = 0; d < kSeedSpread; ++d) {
         const int off = d - kSeedSpread / 2;
         const bool ok = lo + off >= wb && hi + off < we;
-        seeds[round * kSeedSpread + d] = ok ? make_int2(lo + off, hi + off) : make_int2(-1, -1);
+        seeds[slot * kSeedSpread + d] = ok ? make_int2(lo + off, hi + off) : make_int2(-1, -1);
       }
-      ++head;
     }
-    ++count;
-    __syncthreads();
   }
-  if (threadIdx.x == 0) nseeds[b] = count;
+  __syncthreads();
+  if (t == 0) nseeds[b] = taken;
 }
 
 __global__ void k_reverse(const double* a, int64_t n, double* out) {
@@ -586,15 +643,32 @@ void launch_mp(const DevSeries& S, const Tile* tiles, int ntiles, unsigned long 
 }
 
 void launch_mp_seed(const DevSeries& S, const Tile* tiles, int ntiles, unsigned long long* keys,
-                    cudaStream_t st) {
-  k_fill_u64<<<1024, 256, 0, st>>>(keys, S.s, ULLONG_MAX);
+                    const unsigned int* walk, int num_sms, cudaStream_t st) {
+  if (!walk) cudaMemsetAsync(keys, 0xff, (size_t)S.s * 8, st);
   if (ntiles <= 0) return;
   cudaFuncSetAttribute(k_mp_seed, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(MpSeedShared));
+  // parts per tile by the rounds of resident blocks and the work of one:
+  // anchors (m rows of 7 FP64 multiply-adds) against `part` stages (kStage
+  // rows of 14 FP32 ones at twice the rate, and the keyed rows)
+  constexpr int kStages = kLbRows / kStage;
+  const int64_t resident = (int64_t)kSeedCtasPerSm * num_sms;
+  int part = kStages;
+  double best = 0.0;
+  for (int p = kStages; p >= 1; --p) {
+    const int64_t units = (int64_t)ntiles * ((kStages + p - 1) / p);
+    // fewer blocks than the GPU holds run faster, up to one per scheduler
+    const double rounds = units >= resident ? (double)((units + resident - 1) / resident)
+                                            : (units * 4 >= resident ? (double)units / resident : 0.25);
+    const double cost = rounds * ((double)S.m + 1.5 * kStage * p);
+    if (p == kStages || cost < 0.95 * best) best = cost, part = p;
+  }
+  const int parts = (kStages + part - 1) / part;
   const int slab = 1 << 20;
   for (int b = 0; b < ntiles; b += slab) {
     const int cnt = ntiles - b < slab ? ntiles - b : slab;
-    k_mp_seed<<<cnt, kLbThreads, sizeof(MpSeedShared), st>>>(S, tiles + b, keys);
+    k_mp_seed<<<dim3((unsigned)cnt, (unsigned)parts), kLbThreads, sizeof(MpSeedShared), st>>>(
+        S, tiles + b, part, keys, walk);
   }
 }
 
