@@ -189,6 +189,12 @@ struct DevSeries {
   float4* sup;      // the same for kGrpFan consecutive groups, sup_n records per slot
   int64_t grp_n, sup_n;
   int grp_g, grp_b, grp_d;
+  // Window table of the DTW stage (nullptr: too large): the z-normalised
+  // windows and their envelopes as FP32 rows of zm values, filled by
+  // launch_window_table once a chunk queues enough pairs (*zready).
+  float *zt, *zu, *zl;
+  int zm;
+  unsigned int* zready;  // [0] filled, [1] blocks done
   int* status;      // device status word (0 ok, else error bits)
 };
 
@@ -288,7 +294,7 @@ __host__ __device__ inline bool group_tile_dense(const Tile& T, int g, unsigned 
 // reference's fourth option adds the corner cell twice (lb_kim.cpp:55,62);
 // here it is added once so that the bound stays admissible.
 template <typename V, typename Seq>
-__device__ __forceinline__ void kim_bound(const Seq& q, const Seq& t, int m, V* left, V* right) {
+__device__ __forceinline__ V kim_side(const Seq& q, const Seq& t) {
   auto D2 = [](V x, V y) { return (x - y) * (x - y); };
   auto mn = [](V x, V y) { return x < y ? x : y; };
   const V o = D2(t[0], q[0]);
@@ -298,16 +304,19 @@ __device__ __forceinline__ void kim_bound(const Seq& q, const Seq& t, int m, V* 
   d = mn(d, D2(q[1], t[1]) + D2(q[2], t[2]));
   d = mn(d, l1 + D2(q[2], t[1]));
   d = mn(d, D2(q[1], t[0]) + D2(q[2], t[0]));
-  *left = o + d;
-  const int e = m - 1;
-  const V o2 = D2(t[e], q[e]);
-  const V rw = mn(D2(t[e - 1], q[e]), D2(t[e - 1], q[e - 1]));
-  const V r1 = mn(rw, D2(t[e], q[e - 1]));
-  d = mn(D2(t[e - 1], q[e]) + D2(t[e - 2], q[e]), rw + D2(t[e - 2], q[e - 1]));
-  d = mn(d, D2(q[e - 1], t[e - 1]) + D2(q[e - 2], t[e - 2]));
-  d = mn(d, r1 + D2(q[e - 2], t[e - 1]));
-  d = mn(d, D2(q[e - 1], t[e]) + D2(q[e - 2], t[e]));
-  *right = o2 + d;
+  return o + d;
+}
+template <typename Seq>
+struct Reversed {
+  const Seq& s;
+  int e;
+  __device__ auto operator[](int k) const { return s[e - k]; }
+};
+// left from the windows' first three samples, right from their last three.
+template <typename V, typename Seq>
+__device__ __forceinline__ void kim_bound(const Seq& q, const Seq& t, int m, V* left, V* right) {
+  *left = kim_side<V>(q, t);
+  *right = kim_side<V>(Reversed<Seq>{q, m - 1}, Reversed<Seq>{t, m - 1});
 }
 
 struct BandShape {
@@ -315,9 +324,12 @@ struct BandShape {
   int G;  // lanes per pair
   int warps = 0;  // CTA size of the join's DTW kernel in warps (0: the default, 4)
 };
-// The join's layout: one pair per warp (G = 32) with the fewest cells per
-// lane C in [2, 16] covering 2w+1 diagonals.  Returns false if w > 255.
+// One pair per warp (G = 32) with the fewest cells per lane C in [2, 16]
+// covering 2w+1 diagonals.  Returns false if w > 255.
 bool choose_band(int w, BandShape* out);
+// The join's layout: several pairs to a warp where the band and the windows
+// are small enough, else choose_band.
+bool choose_band_join(int m, int w, BandShape* out);
 // Exact DTW lists (no early abandoning): G in {4, 8, 16, 32} and C in
 // [2, 16] covering 2w+1 diagonals with the least waste.
 bool choose_band_list(int w, BandShape* out);
@@ -456,10 +468,20 @@ void launch_petitjean(const DevSeries& S, const DevSearch& Q, unsigned int* next
 size_t lbp_list_bytes(int m, int w, bool own_env);
 void launch_lbp_list(const DevSeries& S, const int2* pairs, int count, bool own_env,
                      double* keogh_mid, double* terms, int num_sms, cudaStream_t st);
-// bounds = false: DTW only (the seeds); true: endpoint bound + LB_Keogh first
+// bounds = false: DTW only (the seeds); true: endpoint bound + LB_Keogh first.
+// Layouts with G < 32 and bounds run several pairs to a warp (dtw_slots.cuh).
 void launch_pairs(const DevSeries& S, const DevSearch& Q, const int2* pairs,
                   const unsigned int* npairs, bool bounds, BandShape band, int num_sms,
                   cudaStream_t st);
+void launch_dtw_slots4(int cells, const DevSeries& S, const DevSearch& Q, const int2* pairs,
+                       const unsigned int* npairs, int num_sms, int warps, cudaStream_t st);
+void launch_dtw_slots8(int cells, const DevSeries& S, const DevSearch& Q, const int2* pairs,
+                       const unsigned int* npairs, int num_sms, int warps, cudaStream_t st);
+void launch_dtw_slots16(int cells, const DevSeries& S, const DevSearch& Q, const int2* pairs,
+                        const unsigned int* npairs, int num_sms, int warps, cudaStream_t st);
+// Fills the window table if the queue holds more than half as many pairs as
+// the series has windows and it is not filled yet.
+void launch_window_table(const DevSeries& S, const DevSearch& Q, int num_sms, cudaStream_t st);
 // FP64 re-verification of the candidates, then per series the lexicographic
 // minimum (d2, i, j): best_d2[series] (FP64 squared distance, +inf if none),
 // best_ij[series] = i << 32 | j, best_f32[series] = the search's FP32 d2.

@@ -59,6 +59,8 @@ constexpr int kSeedGroupTiles = 1024;
 constexpr unsigned int kSeedSupCap = 1u << 24, kSeedListCap = 1u << 22;
 constexpr size_t kSeedScratch =
     (size_t)kSeedSupCap * 4 + (size_t)kSeedListCap * sizeof(uint2) + kSeedSamples * 4 + 64;
+// Largest window table (three FP32 rows per window).
+constexpr size_t kWindowTableMax = (size_t)2 << 30;
 // (m, w) groups of a batch joined at the same time, one context each.
 constexpr int kBatchWorkers = 4;
 
@@ -154,7 +156,7 @@ enum BufId {
   B_MP, B_MPI, B_CB, B_AF, B_ULF, B_BITS, B_LBTILES, B_KQ, B_SBEG, B_SID, B_SEEDBSF,
   B_BEST_IJ, B_BEST_F32, B_QSER, B_TILEBEST, B_FEAT, B_SCORE, B_PA, B_CMAX, B_RW,
   B_MPX_WANT, B_MPX_WREV, B_MPX_MIN, B_MPX_IDX, B_MPX_CAND, B_MPX_CNT, B_NOTES, B_NOTES2,
-  B_SORT, B_SORT_TEMP, B_LBTILES2, B_CMAX2, B_WREC, B_GRP, B_SUP, B_GMEANS, B_GSUP, B_GLIST, B_DENSE,
+  B_SORT, B_SORT_TEMP, B_LBTILES2, B_CMAX2, B_WREC, B_GRP, B_SUP, B_GMEANS, B_GSUP, B_GLIST, B_DENSE, B_ZT, B_ZREADY,
   B_COUNT_
 };
 
@@ -432,10 +434,13 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   Timer wall;
   const int w = effective_band(m, w_in);
   BandShape band;
-  if (!choose_band(w, &band)) return DTWJ_ERR_BAND;
+  if (!choose_band_join(m, w, &band)) return DTWJ_ERR_BAND;
   for (const auto& bo : ctx->band_override)
     if (bo.first == w) band = bo.second;
   band.warps = ctx->dtw_warps;
+  // the seeds and the verification: few pairs, each as fast as one can go
+  BandShape wide;
+  choose_band(w, &wide);
   const bool learned = (flags & DTWJ_F_LEARNED) && !tq;
   if (learned && !ctx->model) return DTWJ_ERR_NOMODEL;
   if (learned && mlp_device(ctx->model) != ctx->device) return DTWJ_ERR_ARG;
@@ -478,6 +483,22 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   if (nlb > 0)
     CUDA_OK(cudaMemcpyAsync(lbtiles, th.data(), (size_t)nlb * sizeof(Tile),
                             cudaMemcpyHostToDevice, st));
+
+  // the window table of the slot DTW, where it fits its limit and the device
+  if (band.G < 32) {
+    const int64_t zm = (m + 3) / 4 * 4;
+    const size_t row = (size_t)S.s * zm * sizeof(float);
+    void *zt = nullptr, *zr = nullptr;
+    if (3 * row <= kWindowTableMax && ensure(ctx, B_ZT, 3 * row, &zt) == DTWJ_OK &&
+        ensure(ctx, B_ZREADY, 8, &zr) == DTWJ_OK) {
+      S.zt = static_cast<float*>(zt);
+      S.zu = S.zt + S.s * zm;
+      S.zl = S.zu + S.s * zm;
+      S.zm = (int)zm;
+      S.zready = static_cast<unsigned int*>(zr);
+      CUDA_OK(cudaMemsetAsync(S.zready, 0, 8, st));
+    }
+  }
 
   // search state
   DevSearch Q;
@@ -646,7 +667,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     Qs.qser = nullptr;
     Qs.queue_next = nseeds + nseries + 1;
     Qs.queue_cap = (unsigned int)(nseries * kSeedSlots);
-    launch_pairs(S, Qs, seeds, nseeds + nseries, false, band, ctx->num_sms, st);
+    launch_pairs(S, Qs, seeds, nseeds + nseries, false, wide, ctx->num_sms, st);
     ph.end(DTWJ_PHASE_SEEDS, 2);
   }
   CUDA_OK(cudaMemcpyAsync(seed_bsf, Q.bsf2, (size_t)nslots * 4, cudaMemcpyDeviceToDevice, st));
@@ -670,8 +691,9 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
       ph.end(DTWJ_PHASE_KEOGH, petitjean ? 2 : 1);
     }
     ph.begin();
+    if (S.zt) launch_window_table(S, Q, ctx->num_sms, st);
     launch_pairs(S, Q, Q.queue, Q.queue_count, true, band, ctx->num_sms, st);
-    ph.end(DTWJ_PHASE_PAIRS, 1);
+    ph.end(DTWJ_PHASE_PAIRS, S.zt ? 2 : 1);
   };
   // one pass over tile ranges: bound sweep, run filter, LB_Keogh, DTW, and a
   // note of each range (queue overflow, counters after it); notes[0] holds
@@ -881,7 +903,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   ENSURE(B_BEST_IJ, (size_t)nslots * 8, best_ij);
   ENSURE(B_BEST_F32, (size_t)nslots * 4, best_f32);
   ph.begin();
-  launch_verify(S, Q, band, vd2, best_d2, best_ij, best_f32, st);
+  launch_verify(S, Q, wide, vd2, best_d2, best_ij, best_f32, st);
   ph.end(DTWJ_PHASE_VERIFY, 4);
   CUDA_OK(cudaEventRecord(ctx->ev1, st));
 

@@ -22,6 +22,7 @@
 // are z-normalised in shared memory with finite sentinels outside [0, m) so
 // out-of-range cells are effectively infinite without branches; a lane keeps
 // the q and t values of C consecutive steps in registers.
+#include "dtw_slots.cuh"
 #include "dtwj_dev.cuh"
 
 #include <cfloat>
@@ -439,6 +440,42 @@ __global__ void __launch_bounds__(256) k_pairs(DevSeries S, DevSearch Q, const i
     if (cnt[x]) atomicAdd(&Q.counters[x], cnt[x]);
 }
 
+// The window table (DevSeries::zt, zu, zl): each pair of the DTW stage needs
+// two z-normalised windows and the second one's envelope, 4 m values
+// normalised in FP64; a queue of more than s / 2 pairs repeats windows enough
+// that normalising every window once is cheaper.  A thread writes four
+// samples of a window.
+__global__ void __launch_bounds__(256) k_window_table(DevSeries S, DevSearch Q) {
+  if (S.zready[0] != 0u || 2ll * *Q.queue_count <= S.s) return;
+  const int per = S.zm / 4;
+  const int64_t total = S.s * per;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = e / per;
+    const int k = (int)(e - i * per) * 4;
+    const double mu = S.mu[i], is = S.isg[i];
+    float a[4], u[4], l[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const int64_t p = i + k + x < S.n ? i + k + x : S.n - 1;  // past the window: never read
+      a[x] = (float)((S.a[p] - mu) * is);
+      u[x] = (float)((S.U[p] - mu) * is);
+      l[x] = (float)((S.L[p] - mu) * is);
+    }
+    const int64_t at = i * S.zm + k;
+    *reinterpret_cast<float4*>(S.zt + at) = make_float4(a[0], a[1], a[2], a[3]);
+    *reinterpret_cast<float4*>(S.zu + at) = make_float4(u[0], u[1], u[2], u[3]);
+    *reinterpret_cast<float4*>(S.zl + at) = make_float4(l[0], l[1], l[2], l[3]);
+  }
+  // the last block to finish marks the table as filled
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(&S.zready[1], 1u) == gridDim.x - 1) {
+    S.zready[1] = 0u;
+    S.zready[0] = 1u;
+  }
+}
+
 // Exact DTW of a list of pairs (no bounds, no abandoning), FP32 or FP64.
 // With `cands`, pairs come from the candidate list and any candidate above
 // the final best-so-far (plus slack) is skipped with +inf.
@@ -594,7 +631,8 @@ void run_pairs_band(const DevSeries& S, const DevSearch& Q, const int2* pairs,
                     const unsigned int* npairs, int flags, int num_sms, cudaStream_t st,
                     int warps) {
   if constexpr (G == 32 && C <= 8) {
-    if (run_pairs_hi<C, G, 0>((2 * S.w + 1) % C, S, Q, pairs, npairs, flags, num_sms, st, warps))
+    if (slot_mask_ok(S.w, C, G) &&
+        run_pairs_hi<C, G, 0>((2 * S.w + 1) % C, S, Q, pairs, npairs, flags, num_sms, st, warps))
       return;
   }
   run_pairs<C, G, -2>(S, Q, pairs, npairs, flags, num_sms, st, warps);
@@ -662,14 +700,6 @@ int band_shapes(int w, BandShape* out, int max) {
 }
 
 bool choose_band(int w, BandShape* out) {
-  // One pair per warp (G = 32), with the fewest cells per lane that cover
-  // the band.  The groups of a warp that hold different pairs leave the band
-  // loop at different steps (early abandoning) and the warp then runs their
-  // loops one after the other, which costs more than the lanes' cells
-  // outside the band: measured in joins of ECG-like series at w = 3, 13, 52
-  // and 103, G = 32 was fastest at every w, up to 4.9x ahead of the layout
-  // with the fewest wasted cells (w = 13: (7, 4) 58.9 s against (2, 32)
-  // 12.0 s of DTW).
   int C = (2 * w + 1 + 31) / 32;
   if (C < 2) C = 2;
   while (C <= 16 && !band_supported(C, 32)) ++C;
@@ -704,17 +734,52 @@ bool choose_band_list(int w, BandShape* out) {
   return true;
 }
 
+bool choose_band_join(int m, int w, BandShape* out) {
+  // Lanes per pair by the band: a slot's row step costs the same whatever it
+  // holds, so a narrow band takes few lanes with several cells each.  DTW
+  // stage of ECG-like joins, (cells, lanes): w = 20 (6, 8) 9.2 ms, (3, 16)
+  // 16.1; w = 13 (4, 8) 13.3, (2, 16) 29.0, (7, 4) 18.7; w = 7 (4, 4) 10.8,
+  // (2, 8) 13.5; w = 52 (7, 16) 150, one pair per warp (4, 32) 224.  A warp's
+  // windows must leave room for about 11 warps per SM.
+  const int first = w <= 7 ? 4 : (w <= 27 ? 8 : 16);
+  for (int G = first; G <= 16; G *= 2) {
+    const int C = slot_cells(w, G);
+    if (C == 0 || slot_bytes(m, w, C, G) > kSlotSmemPerWarp) continue;
+    out->C = C;
+    out->G = G;
+    return true;
+  }
+  return choose_band(w, out);
+}
+
 void launch_pairs(const DevSeries& S, const DevSearch& Q, const int2* pairs,
                   const unsigned int* npairs, bool bounds, BandShape band, int num_sms,
                   cudaStream_t st) {
+  if (bounds && band.G < 32 && slot_bytes(S.m, S.w, band.C, band.G) <= 200 * 1024) {
+    auto go = band.G == 4 ? launch_dtw_slots4 : (band.G == 8 ? launch_dtw_slots8 : launch_dtw_slots16);
+    go(band.C, S, Q, pairs, npairs, num_sms, band.warps, st);
+    return;
+  }
+  // one pair per warp: wide bands, the seeds, windows whose slots do not fit
+  if (band.G < 32) {
+    const int warps = band.warps;
+    choose_band(S.w, &band);
+    band.warps = warps;
+  }
   const int flags = bounds ? 1 : 0;
 #define X(c, g) \
-  if (band.C == c && band.G == g) {                                               \
-    run_pairs_band<c, g>(S, Q, pairs, npairs, flags, num_sms, st, band.warps);     \
-    return;                                                                        \
+  if constexpr (g == 32) {                                                          \
+    if (band.C == c) {                                                              \
+      run_pairs_band<c, g>(S, Q, pairs, npairs, flags, num_sms, st, band.warps);     \
+      return;                                                                       \
+    }                                                                               \
   }
   DTWJ_BAND_CASES(X)
 #undef X
+}
+
+void launch_window_table(const DevSeries& S, const DevSearch& Q, int num_sms, cudaStream_t st) {
+  k_window_table<<<num_sms * 8, 256, 0, st>>>(S, Q);
 }
 
 void launch_verify(const DevSeries& S, const DevSearch& Q, BandShape band, double* out_d2,
