@@ -24,6 +24,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I" + INCLUDE]
 CU_SOURCES = ["prep.cu", "mp.cu", "group.cu", "lb.cu", "runs.cu", "paa.cu", "pairs.cu", "dtw_slots4.cu", "dtw_slots8.cu", "dtw_slots16.cu",
+              "dtw_slots32.cu",
               "petitjean.cu", "join.cu", "noalloc.cu", "mlp.cu",
               "features.cu", "load.cpp"]
 

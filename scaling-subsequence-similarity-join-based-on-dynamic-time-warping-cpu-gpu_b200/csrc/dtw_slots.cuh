@@ -1,7 +1,8 @@
 // LB_Keogh's cumulative bound and the banded DTW of the join's queue, several
 // pairs to a warp.
 //
-// A warp holds 32 / G slots of G lanes, one pair each; a lane owns C
+// A warp holds 32 / G slots of G lanes (one slot of the whole warp for wide
+// bands), one pair each; a lane owns C
 // consecutive diagonals of its pair's band (the layout of pairs.cu).  A row
 // step costs a warp two shuffles, two shared loads and 3 C + 1 arithmetic
 // instructions whatever it holds, and shuffles and shared loads issue at one
@@ -263,12 +264,19 @@ __device__ __forceinline__ float prepare_pair(const DevSeries& S, const Next& nx
   return whole;
 }
 
+// Blocks per SM asked of the compiler: 3 (80 registers) where that measured
+// faster than its own choice of 64 with a few spills: wide bands (walk of 131k,
+// m = 512, w = 103: 168 -> 141 ms, one pair per warp without slots and table
+// 288) and few cells per lane (w = 7 and 13: 4 %); at 6 and 7 cells in slots 64
+// registers win by 3 to 6 %.
+constexpr int slot_blocks(int C, int G) { return G == 32 || C <= 4 ? 3 : 0; }
+
 template <int C, int G, int HI>
-__global__ void __launch_bounds__(256) k_dtw_slots(DevSeries S, DevSearch Q, const int2* pairs,
+__global__ void __launch_bounds__(256, slot_blocks(C, G)) k_dtw_slots(DevSeries S, DevSearch Q, const int2* pairs,
                                                    const unsigned int* npairs) {
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int NS = 32 / G;
-  constexpr unsigned int kGroup = (1u << G) - 1u;  // a slot's lanes
+  constexpr unsigned int kGroup = 0xffffffffu >> (32 - G);  // a slot's lanes
   constexpr int kIters = (16 + 2 * C - 1) / (2 * C);  // iterations between abandon checks
   const int m = S.m, w = S.w;
   const int lane = threadIdx.x & 31, slot = lane / G, g = lane & (G - 1);

@@ -178,7 +178,10 @@ struct DevSeries {
   // copy 1 on [2048 b - 1024, 2048 b + 1024), so every window lies inside one
   // block of one copy and has a single block offset (else all nullptr).
   float4* pq2;      // 2n, copy c at [c n, c n + n)
-  float* cmax2;     // 2 kCopyBlocks(n), largest |value| of each copy block
+  float* fq;        // the same over fine blocks of paa_b / 4 samples, a apart from
+  float2* ful;      //    (U, L) and phase-major (fine_at): a window's blocks are consecutive
+  int64_t fine_n;   // entries per phase
+  float* cmax2;     // 2 kCopyBlocks(n), largest |value| of each copy block (both lengths)
   float4* wrec;     // s, window record: block offset (FP64 in .x/.y), isg as
                     //    FP32 (.z) and the error scale for pq2 (.w)
   // Window groups of the group bound (nullptr: not built): grp_d slots of
@@ -198,6 +201,17 @@ struct DevSeries {
   int* status;      // device status word (0 ok, else error bits)
 };
 
+// The copy whose blocks hold window [i, i + m), m <= 1024: copy 0 when the
+// window ends inside its 2048-sample block, else copy 1 (then i mod 2048 >
+// 1024 and the window lies in [2048 b + 1024, 2048 b + 3072)).
+__device__ __forceinline__ int win_copy(int64_t i, int m) { return (int)(i & 2047) + m > 2048 ? 1 : 0; }
+// Fine block [p, p + F) of copy c, F = paa_b / 4; the next block of the same
+// window, at p + F, follows it.
+__device__ __forceinline__ int64_t fine_at(const DevSeries& S, int c, int64_t p) {
+  const int F = S.paa_b / 4;
+  return ((int64_t)c * F + p % F) * S.fine_n + p / F;
+}
+
 // Global search state of one join.
 struct DevSearch {
   unsigned int* bsf2;           // per series: float bits of the best squared DTW so far
@@ -214,7 +228,8 @@ struct DevSearch {
   unsigned int* queue_count;
   unsigned int* queue_next;
   unsigned int queue_cap;
-  int4* kq;                     // LB_Keogh candidates: (i, j, endpoint bound bits, series)
+  int4* kq;                     // LB_Keogh candidates: (query, envelope, endpoint bound bits,
+                                //   series), the more promising direction first
   unsigned int* kq_count;
   unsigned int* kq_next;
   unsigned int kq_cap;
@@ -469,7 +484,7 @@ size_t lbp_list_bytes(int m, int w, bool own_env);
 void launch_lbp_list(const DevSeries& S, const int2* pairs, int count, bool own_env,
                      double* keogh_mid, double* terms, int num_sms, cudaStream_t st);
 // bounds = false: DTW only (the seeds); true: endpoint bound + LB_Keogh first.
-// Layouts with G < 32 and bounds run several pairs to a warp (dtw_slots.cuh).
+// Layouts with up to 8 cells per lane and bounds run in slots (dtw_slots.cuh).
 void launch_pairs(const DevSeries& S, const DevSearch& Q, const int2* pairs,
                   const unsigned int* npairs, bool bounds, BandShape band, int num_sms,
                   cudaStream_t st);
@@ -478,6 +493,8 @@ void launch_dtw_slots4(int cells, const DevSeries& S, const DevSearch& Q, const 
 void launch_dtw_slots8(int cells, const DevSeries& S, const DevSearch& Q, const int2* pairs,
                        const unsigned int* npairs, int num_sms, int warps, cudaStream_t st);
 void launch_dtw_slots16(int cells, const DevSeries& S, const DevSearch& Q, const int2* pairs,
+                        const unsigned int* npairs, int num_sms, int warps, cudaStream_t st);
+void launch_dtw_slots32(int cells, const DevSeries& S, const DevSearch& Q, const int2* pairs,
                         const unsigned int* npairs, int num_sms, int warps, cudaStream_t st);
 // Fills the window table if the queue holds more than half as many pairs as
 // the series has windows and it is not filled yet.

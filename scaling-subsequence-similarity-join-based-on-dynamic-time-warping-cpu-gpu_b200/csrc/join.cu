@@ -156,7 +156,7 @@ enum BufId {
   B_MP, B_MPI, B_CB, B_AF, B_ULF, B_BITS, B_LBTILES, B_KQ, B_SBEG, B_SID, B_SEEDBSF,
   B_BEST_IJ, B_BEST_F32, B_QSER, B_TILEBEST, B_FEAT, B_SCORE, B_PA, B_CMAX, B_RW,
   B_MPX_WANT, B_MPX_WREV, B_MPX_MIN, B_MPX_IDX, B_MPX_CAND, B_MPX_CNT, B_NOTES, B_NOTES2,
-  B_SORT, B_SORT_TEMP, B_LBTILES2, B_CMAX2, B_WREC, B_GRP, B_SUP, B_GMEANS, B_GSUP, B_GLIST, B_DENSE, B_ZT, B_ZREADY,
+  B_SORT, B_SORT_TEMP, B_LBTILES2, B_CMAX2, B_WREC, B_GRP, B_SUP, B_GMEANS, B_GSUP, B_GLIST, B_DENSE, B_ZT, B_ZREADY, B_FQ, B_FUL,
   B_COUNT_
 };
 
@@ -337,6 +337,10 @@ int prepare(dtwj_ctx* ctx, const double* x_dev, int64_t n, int m, int w, bool ma
   ENSURE(B_ULF, n * 8, S.ulf);
   if (m <= (1 << kBlkShift)) {
     ENSURE(B_PA, (size_t)n * 32, S.pq2);
+    const int fine = paa_block(m) / 4;
+    S.fine_n = n / fine + 2;
+    ENSURE(B_FQ, (size_t)S.fine_n * fine * 2 * sizeof(float), S.fq);
+    ENSURE(B_FUL, (size_t)S.fine_n * fine * 2 * sizeof(float2), S.ful);
     ENSURE(B_CMAX2, (size_t)kCopyBlocks(n) * 8, S.cmax2);
     ENSURE(B_WREC, (size_t)s * 16, S.wrec);
   } else {
@@ -485,7 +489,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
                             cudaMemcpyHostToDevice, st));
 
   // the window table of the slot DTW, where it fits its limit and the device
-  if (band.G < 32) {
+  if (band.C <= 8) {
     const int64_t zm = (m + 3) / 4 * 4;
     const size_t row = (size_t)S.s * zm * sizeof(float);
     void *zt = nullptr, *zr = nullptr;
@@ -508,9 +512,10 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     const long v = atol(env);
     if (v >= 1024 && v < (long)kQueueCapMax) qcap = (unsigned int)v;
   }
-  ENSURE(B_QUEUE, (size_t)qcap * sizeof(int2), Q.queue);
-  // LB_Keogh candidates of one chunk: twice the DTW queue (most are pruned)
+  // LB_Keogh candidates of one chunk, and those that go on to DTW (nearly all
+  // of them on quasi-periodic series)
   ENSURE(B_KQ, (size_t)qcap * 2 * sizeof(int4), Q.kq);
+  ENSURE(B_QUEUE, (size_t)qcap * 2 * sizeof(int2), Q.queue);
   const bool enumerate_all = flags & DTWJ_F_NO_DIAG;
   const double tile_pairs = (double)kLbLags * kLbRows;
   int chunk = ctx->chunk_tiles > 0 ? ctx->chunk_tiles
@@ -542,7 +547,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     F.sup_cap = F.list_cap = (unsigned int)pairs;
     F.tcount = qc + kQcTiles;
   }
-  Q.queue_cap = qcap;
+  Q.queue_cap = qcap * 2;
   Q.kq_cap = qcap * 2;
   Q.runs = nullptr;
   Q.run_cap = 0;
@@ -554,7 +559,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   ENSURE(B_CAND, (size_t)cand_cap * sizeof(Candidate), Q.cand);
   ENSURE(B_CCOUNT, 4, Q.cand_count);
   Q.cand_cap = cand_cap;
-  if (tile_mode) ENSURE(B_QSER, (size_t)qcap * sizeof(int), Q.qser);
+  if (tile_mode) ENSURE(B_QSER, (size_t)qcap * 2 * sizeof(int), Q.qser);
   CUDA_OK(cudaMemsetAsync(Q.counters, 0, kNumCounters * 8, st));
   CUDA_OK(cudaMemsetAsync(Q.cand_count, 0, 4, st));
   ctx->host_u32.assign((size_t)nslots + 1, 0x7f800000u);  // +inf per slot

@@ -60,45 +60,45 @@ __device__ __forceinline__ double copy_center(const DevSeries& S, int copy, int6
   const int64_t k = 2 * b - copy;
   return k < 0 ? S.cb[0] : 0.5 * (S.cb[k] + S.cb[k + 1]);
 }
-// The copy whose blocks hold window [i, i + m), m <= 1024: copy 0 when the
-// window ends inside its 2048-sample block, else copy 1 (then i mod 2048 >
-// 1024 and the window lies in [2048 b + 1024, 2048 b + 3072)).
-__device__ __forceinline__ int win_copy(int64_t i, int m) { return (int)(i & 2047) + m > 2048 ? 1 : 0; }
-
 // Sliding block means over [p, p + B) of a, U and L, centered: on the
 // 1024-sample block of p (pq, windows longer than 1024 samples), or on the
-// block of p in each of the two copies (pq2).  Entries whose block runs past
-// the series are zero (never read: a window's blocks end inside it).
+// block of p in each of the two copies (pq2), there also over [p, p + B / 4)
+// (fq, ful).  Entries whose block runs past the series are zero (never read: a
+// window's blocks end inside it).
 __global__ void k_slide_means(DevSeries S, int B) {
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (p >= S.n) return;
-  if (p + B > S.n) {
-    const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (S.pq2) {
-      S.pq2[p] = z;
-      S.pq2[S.n + p] = z;
-    } else {
-      S.pq[p] = z;
-    }
-    return;
-  }
-  double sa = 0.0, su = 0.0, sl = 0.0;
-  for (int k = 0; k < B; ++k) {
+  const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const int F = B / 4;
+  double sa = 0.0, su = 0.0, sl = 0.0, fa = 0.0, fu = 0.0, fl = 0.0;
+  const int cnt = p + B <= S.n ? B : (p + F <= S.n ? F : 0);
+  for (int k = 0; k < cnt; ++k) {
     sa += S.a[p + k];
     su += S.U[p + k];
     sl += S.L[p + k];
+    if (k == F - 1) {
+      fa = sa;
+      fu = su;
+      fl = sl;
+    }
   }
   const double ib = 1.0 / (double)B;
-  const double ma = sa * ib, mu = su * ib, ml = sl * ib;
   if (S.pq2) {
+    const double jf = 1.0 / (double)F;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       const double x = copy_center(S, c, copy_block(c, p));
-      S.pq2[c * S.n + p] = make_float4((float)(ma - x), (float)(mu - x), (float)(ml - x), 0.0f);
+      S.pq2[c * S.n + p] = cnt < B ? z : make_float4((float)(sa * ib - x), (float)(su * ib - x),
+                                                     (float)(sl * ib - x), 0.0f);
+      const int64_t at = fine_at(S, c, p);
+      S.fq[at] = cnt < F ? 0.0f : (float)(fa * jf - x);
+      S.ful[at] = cnt < F ? make_float2(0.0f, 0.0f)
+                          : make_float2((float)(fu * jf - x), (float)(fl * jf - x));
     }
   } else {
     const double x = S.cb[p >> kBlkShift];
-    S.pq[p] = make_float4((float)(ma - x), (float)(mu - x), (float)(ml - x), 0.0f);
+    S.pq[p] = cnt < B ? z : make_float4((float)(sa * ib - x), (float)(su * ib - x),
+                                        (float)(sl * ib - x), 0.0f);
   }
 }
 
@@ -133,8 +133,8 @@ __global__ void k_block_max(DevSeries S, int nb) {
   if (threadIdx.x == 0) S.cmax[b] = t;
 }
 
-// cmax2[c * kCopyBlocks + b] = the largest magnitude of pq2 over block b of
-// copy c (grid: 2 kCopyBlocks(n) blocks).
+// cmax2[c * kCopyBlocks + b] = the largest magnitude of pq2, fq and ful over
+// block b of copy c (grid: 2 kCopyBlocks(n) blocks).
 __global__ void k_block_max2(DevSeries S) {
   const int64_t nbc = kCopyBlocks(S.n);
   const int c = (int)(blockIdx.x / nbc);
@@ -146,7 +146,10 @@ __global__ void k_block_max2(DevSeries S) {
   float v = 0.0f;
   for (int64_t p = lo + threadIdx.x; p < hi; p += blockDim.x) {
     const float4 x = q[p];
+    const int64_t at = fine_at(S, c, p);
+    const float2 y = S.ful[at];
     v = fmaxf(v, fmaxf(fabsf(x.x), fmaxf(fabsf(x.y), fabsf(x.z))));
+    v = fmaxf(v, fmaxf(fabsf(S.fq[at]), fmaxf(fabsf(y.x), fabsf(y.y))));
   }
   const float t = block_max_reduce(v);
   if (threadIdx.x == 0) S.cmax2[blockIdx.x] = t;
@@ -193,11 +196,13 @@ struct Ends6 {
 };
 
 // Endpoint bound (FP64, the end samples normalised) of the pairs (i, j) of
-// the lanes that are alive; those it keeps go to the LB_Keogh queue.  Called
-// by every lane of the warp.
+// the lanes that are alive; those it keeps go to the LB_Keogh queue, as (j, i)
+// when `second`: the direction whose block-mean bound came closer, the query
+// first, which LB_Keogh then takes first.  Called by every lane of the warp.
 __device__ __forceinline__ void push_survivor(const DevSeries& S, const DevSearch& Q,
-                                              const Tile& T, bool alive, int i, int j, float thr,
-                                              int lane, unsigned int& nkim) {
+                                              const Tile& T, bool alive, int i, int j,
+                                              bool second, float thr, int lane,
+                                              unsigned int& nkim) {
   if (!__any_sync(0xffffffffu, alive)) return;
   const int m = S.m;
   float kim = 0.0f;
@@ -227,7 +232,7 @@ __device__ __forceinline__ void push_survivor(const DevSeries& S, const DevSearc
   if (alive) {
     const unsigned int slot = base + __popc(sv & ((1u << lane) - 1u));
     if (slot < Q.kq_cap) {
-      Q.kq[slot] = make_int4(i, j, __float_as_int(kim), T.series);
+      Q.kq[slot] = make_int4(second ? j : i, second ? i : j, __float_as_int(kim), T.series);
     } else {
       atomicOr(S.status, 2);
     }
@@ -501,7 +506,7 @@ __global__ void __launch_bounds__(kPaaWarps * 32, 3) k_paa_lags(DevSeries S, Dev
         }
       }
       npaa += (live && pruned) ? 1u : 0u;
-      push_survivor(S, Q, T, live && !pruned, i, j, thr, lane, nkim);
+      push_survivor(S, Q, T, live && !pruned, i, j, acc2 > acc1, thr, lane, nkim);
     }
   }
   unsigned long long a = npaa, b = nkim;
@@ -632,7 +637,8 @@ __global__ void __launch_bounds__(kPaaWarps * 32, 3) k_paa_groups(DevSeries S, D
 #pragma unroll
       for (int x = 0; x < R; ++x) {
         npaa += (live[x] && pruned[x]) ? 1u : 0u;
-        push_survivor(S, Q, T, live[x] && !pruned[x], i[x], j, thr, lane, nkim);
+        push_survivor(S, Q, T, live[x] && !pruned[x], i[x], j, acc2[x] > acc1[x], thr, lane,
+                      nkim);
       }
     }
   }

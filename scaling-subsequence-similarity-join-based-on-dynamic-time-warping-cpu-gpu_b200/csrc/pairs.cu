@@ -606,38 +606,6 @@ void run_pairs(const DevSeries& S, const DevSearch& Q, const int2* pairs,
                                                               lay.total);
 }
 
-// The one-pair-per-warp layouts with at most 8 cells per lane run with the
-// single-cell band mask (HI = (2w + 1) mod C, -1 for 0; an even C only sees
-// odd values); the others mask every cell.
-template <int C, int G, int K>
-bool run_pairs_hi(int hi, const DevSeries& S, const DevSearch& Q, const int2* pairs,
-                  const unsigned int* npairs, int flags, int num_sms, cudaStream_t st,
-                  int warps) {
-  if constexpr (K < C) {
-    if constexpr (C % 2 == 1 || K % 2 == 1) {
-      if (hi == K) {
-        run_pairs<C, G, K == 0 ? -1 : K>(S, Q, pairs, npairs, flags, num_sms, st, warps);
-        return true;
-      }
-    }
-    return run_pairs_hi<C, G, K + 1>(hi, S, Q, pairs, npairs, flags, num_sms, st, warps);
-  } else {
-    return false;
-  }
-}
-
-template <int C, int G>
-void run_pairs_band(const DevSeries& S, const DevSearch& Q, const int2* pairs,
-                    const unsigned int* npairs, int flags, int num_sms, cudaStream_t st,
-                    int warps) {
-  if constexpr (G == 32 && C <= 8) {
-    if (slot_mask_ok(S.w, C, G) &&
-        run_pairs_hi<C, G, 0>((2 * S.w + 1) % C, S, Q, pairs, npairs, flags, num_sms, st, warps))
-      return;
-  }
-  run_pairs<C, G, -2>(S, Q, pairs, npairs, flags, num_sms, st, warps);
-}
-
 template <typename T, int C, int G>
 void run_list(const DevSeries& S, const int2* pairs, const Candidate* cands,
               const unsigned int* count_ptr, int count, const unsigned int* bsf2, double* out,
@@ -755,12 +723,16 @@ bool choose_band_join(int m, int w, BandShape* out) {
 void launch_pairs(const DevSeries& S, const DevSearch& Q, const int2* pairs,
                   const unsigned int* npairs, bool bounds, BandShape band, int num_sms,
                   cudaStream_t st) {
-  if (bounds && band.G < 32 && slot_bytes(S.m, S.w, band.C, band.G) <= 200 * 1024) {
-    auto go = band.G == 4 ? launch_dtw_slots4 : (band.G == 8 ? launch_dtw_slots8 : launch_dtw_slots16);
+  if (bounds && band.C <= 8 && slot_bytes(S.m, S.w, band.C, band.G) <= 200 * 1024) {
+    auto go = band.G == 4    ? launch_dtw_slots4
+              : band.G == 8  ? launch_dtw_slots8
+              : band.G == 16 ? launch_dtw_slots16
+                             : launch_dtw_slots32;
     go(band.C, S, Q, pairs, npairs, num_sms, band.warps, st);
     return;
   }
-  // one pair per warp: wide bands, the seeds, windows whose slots do not fit
+  // one pair per warp, every cell masked: bands past 127, the seeds, windows
+  // whose slots do not fit
   if (band.G < 32) {
     const int warps = band.warps;
     choose_band(S.w, &band);
@@ -770,7 +742,7 @@ void launch_pairs(const DevSeries& S, const DevSearch& Q, const int2* pairs,
 #define X(c, g) \
   if constexpr (g == 32) {                                                          \
     if (band.C == c) {                                                              \
-      run_pairs_band<c, g>(S, Q, pairs, npairs, flags, num_sms, st, band.warps);     \
+      run_pairs<c, g, -2>(S, Q, pairs, npairs, flags, num_sms, st, band.warps);      \
       return;                                                                       \
     }                                                                               \
   }

@@ -32,7 +32,7 @@ namespace {
 constexpr int kRunWarps = 4;
 constexpr int kKeoghCheck = 128;  // samples between two best-so-far checks of LB_Keogh
 constexpr int kKeoghWarps = 8;    // warps per block of the LB_Keogh kernel
-constexpr int kKeoghBatch = 8;    // consecutive queue entries a warp takes at once
+constexpr int kKeoghBatch = 8;    // entries a warp prepares at once for the exact bound
 
 // Masked bound for env = r, query = c from the raw FP64 sums
 // F1 = sum_T M_r a_c, F2 = sum_T M_r a_c^2, F3 = sum_T M_r E_r a_c.
@@ -88,12 +88,6 @@ __device__ __forceinline__ double warp_iscan(double v, int lane) {
 }
 
 // max(a, b, c) in one instruction (three-input max.f32, sm_100).
-__device__ __forceinline__ float max3f(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-
 // Adds one LB_Keogh term: query sample a (block-centered, scale sq, offset o
 // = query block offset - envelope block offset, both already scaled) against
 // the block-centered envelope ul = (U, L) (scale se).  With q = a sq + o,
@@ -362,83 +356,177 @@ __global__ void __launch_bounds__(kRunWarps * 32, 8) k_runs(DevSeries S, DevSear
     if (cnt[x]) atomicAdd(&Q.counters[x], cnt[x]);
 }
 
+// Sums over the warp of four values at once: lane l returns that of v[l / 8].
+__device__ __forceinline__ float warp_sum4(const float (&v)[4], int lane) {
+  const bool hi = lane & 16, odd = lane & 8;
+  float a = hi ? v[2] : v[0], b = hi ? v[3] : v[1];
+  a += __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], 16);
+  b += __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], 16);
+  float c = odd ? b : a;
+  c += __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  return c;
+}
+
 // LB_Keogh over the queued candidates.  Entries sit in the order the run
-// filter found them, so the kKeoghBatch consecutive pairs a warp takes are
-// mostly neighbours on one diagonal and share L1 lines.  Lane e prefetches
-// entry e of the batch (indices, endpoint bound, window statistics, block
-// offsets) into shared memory, so the dependent loads are paid once per
-// batch; then the lanes run over the samples of one pair at a time.  The
-// first direction (query i against the envelope of j) decides most pairs,
-// the second runs only when the first stays within the best-so-far.
+// filter found them, so the consecutive pairs a warp takes share windows and
+// L1 lines.
+//
+// First, for windows of at most 1024 samples, the endpoint bound plus the
+// block-mean bound over the fine blocks (paa_b / 4 samples) between the end
+// samples, in the direction that came closer with the
+// coarse ones: the lanes take consecutive blocks, which are consecutive in
+// memory, four pairs at a time (12 bytes per block and pair against 12 per
+// sample of the exact bound).  It settles 86 % of the pairs on the 1M-sample
+// bench series and 69 % on walks at m = 512, w = 52.  What it leaves is split
+// by how close it came: the exact bound is larger by the variance within the
+// blocks and prunes few of the pairs well below the threshold (CPU measurement
+// at half the threshold: 8 of 620 on walks at m = 512, none of 31,600 on an
+// ECG-like series, 37 of 18,000 at m = 200), so those go to DTW as they are;
+// the DTW stage has one direction of the bound for its abandoning anyway.
+// Where the line lies: at 0.8 of the threshold the ECG-like 16k join (m = 512)
+// takes 158.5 ms, at 0.5 165.8, at 0.3 169.4; walks of 131k with w = 103 209,
+// 224 and 235 ms.  In windows below 192 samples single samples weigh more
+// (m = 128: 15.0 ms at 0.5, 15.7 at 0.3, 18.2 at 0.1).  Without the window table
+// a DTW costs more to start: 0.5 (1M-sample join 98.8 ms, at 0.7 99.8, 0.85 104).
+//
+// For the others, eight at a time, lane (e, d) prefetches window d of entry e
+// (statistics, block offsets, end samples) into shared memory, so the
+// dependent loads are paid once; then the lanes run over the samples of one
+// pair at a time.  The first direction decides most pairs, the second runs
+// only when the first stays within the best-so-far.
 __global__ void __launch_bounds__(kKeoghWarps * 32, 5) k_keogh(DevSeries S, DevSearch Q) {
   __shared__ KeoghSide side[kKeoghWarps][kKeoghBatch][2];
   __shared__ float endsv[kKeoghWarps][kKeoghBatch][2];
-  __shared__ int serv[kKeoghWarps][kKeoghBatch];
   __shared__ float errv[kKeoghWarps][kKeoghBatch];  // FP32 error scale of the pair
   __shared__ unsigned long long pruned_block;
   if (threadIdx.x == 0) pruned_block = 0;
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned int total = *Q.kq_count < Q.kq_cap ? *Q.kq_count : Q.kq_cap;
+  // a short queue is dealt out in smaller batches, so that every warp gets some
+  const unsigned int batch = total >= gridDim.x * kKeoghWarps * 64u ? 32u : kKeoghBatch;
+  // fine blocks between the end samples
+  const int F = S.paa_b / 4, kb = (kBias + F - 1) / F, ke = (S.m - kBias) / F;
+  const float skip = !S.zt ? 0.5f : (S.m >= 192 ? 0.8f : 0.6f);
   unsigned long long pruned = 0;
   for (;;) {
     unsigned int idx = 0;
-    if (lane == 0) idx = atomicAdd(Q.kq_next, (unsigned int)kKeoghBatch);
+    if (lane == 0) idx = atomicAdd(Q.kq_next, batch);
     idx = __shfl_sync(0xffffffffu, idx, 0);
     if (idx >= total) break;
-    const int cnt = total - idx < (unsigned int)kKeoghBatch ? (int)(total - idx) : kKeoghBatch;
-    __syncwarp();  // the previous batch is no longer read
-    if (lane < 2 * cnt) {
-      // lane (e, d): window d of entry e, and the end samples of direction d
-      // (query = window d, envelope = the other window) in FP64
-      const int e = lane >> 1, d = lane & 1;
-      const int4 r = Q.kq[idx + e];
-      const unsigned int xe = (unsigned int)(d ? r.x : r.y);
-      KeoghSide w;
-      w.x = (unsigned int)(d ? r.y : r.x);
-      w.mu = S.mu[w.x];
-      w.is = S.isg[w.x];
-      const unsigned int b0 = w.x >> kBlkShift;
-      w.o0 = block_offset(S, b0, w.mu, w.is);
-      w.o1 = block_offset(S, b0 + 1, w.mu, w.is);
-      w.pad = 0;
-      side[warp][e][d] = w;
-      const double me = S.mu[xe], ie = S.isg[xe];
-      double t = 0.0;
+    const int cnt = total - idx < batch ? (int)(total - idx) : (int)batch;
+    // lane e holds entry e of the batch
+    const int4 r = Q.kq[idx + (lane < cnt ? lane : cnt - 1)];
+    const float thr_e = prune_threshold_now(Q.bsf2 + r.w, S.m);
+    const unsigned int all = cnt == 32 ? 0xffffffffu : (1u << cnt) - 1u;
+    unsigned int alive = all, exact = all;
+    if (S.fq) {
+      const float4 wx = S.wrec[r.x], wy = S.wrec[r.y];
+      const float o_e = (float)(__hiloint2double(__float_as_int(wx.y), __float_as_int(wx.x)) -
+                                __hiloint2double(__float_as_int(wy.y), __float_as_int(wy.x)));
+      const bool sure = fmaxf(wx.w, wy.w) <= fp32_bound_radius(thr_e, S.m);
+      // the bound that prunes, and the one below which the exact bound is not tried
+      const float over_e = sure ? thr_e : __int_as_float(0x7f800000);
+      const unsigned int ax = (unsigned int)fine_at(S, win_copy(r.x, S.m), r.x);
+      const unsigned int ay = (unsigned int)fine_at(S, win_copy(r.y, S.m), r.y);
+      for (int e0 = 0; e0 < cnt; e0 += 4) {
+        float acc[4];
 #pragma unroll
-      for (int c = 0; c < 2 * kBias; ++c) {
-        const int k = c < kBias ? c : S.m - 2 * kBias + c;
-        const double z = (S.a[w.x + k] - w.mu) * w.is;
-        const double u = (S.U[xe + k] - me) * ie, l = (S.L[xe + k] - me) * ie;
-        const double dd = fmax(fmax(z - u, l - z), 0.0);
-        t = fma(dd, dd, t);
-      }
-      endsv[warp][e][d] = (float)fmax((double)__int_as_float(r.z), t);
-      if (d == 0) {
-        serv[warp][e] = r.w;
-        errv[warp][e] = fmaxf(S.rw[r.x], S.rw[r.y]);
+        for (int u = 0; u < 4; ++u) {
+          const int e = e0 + u < cnt ? e0 + u : cnt - 1;
+          const float* q = S.fq + __shfl_sync(0xffffffffu, ax, e);
+          const float2* ul = S.ful + __shfl_sync(0xffffffffu, ay, e);
+          const float sx = __shfl_sync(0xffffffffu, wx.z, e);
+          const float sy = __shfl_sync(0xffffffffu, wy.z, e);
+          const float o = __shfl_sync(0xffffffffu, o_e, e);
+          acc[u] = 0.0f;
+#pragma unroll 4
+          for (int k = kb + lane; k < ke; k += 32)
+            acc[u] = keogh_acc(q[k], ul[k], sx, sy, o, acc[u]);
+        }
+        const int e = e0 + (lane >> 3);
+        const float kim = __int_as_float(__shfl_sync(0xffffffffu, r.z, e < cnt ? e : cnt - 1));
+        const float lb = (float)F * warp_sum4(acc, lane) + kim;
+        const float over = __shfl_sync(0xffffffffu, over_e, e < cnt ? e : cnt - 1);
+        const bool mine = (lane & 7) == 0 && e < cnt;
+        unsigned int dead = __ballot_sync(0xffffffffu, mine && lb > over);
+        unsigned int low = __ballot_sync(0xffffffffu, mine && lb < skip * over);
+        // bits 0, 8, 16, 24 -> entries e0 .. e0 + 3
+        dead = (dead & 1u) | (dead >> 7 & 2u) | (dead >> 14 & 4u) | (dead >> 21 & 8u);
+        low = (low & 1u) | (low >> 7 & 2u) | (low >> 14 & 4u) | (low >> 21 & 8u);
+        alive &= ~(dead << e0);
+        exact &= ~((dead | low) << e0);
       }
     }
-    __syncwarp();
-    for (int e = 0; e < cnt; ++e) {
-      float thr = prune_threshold_now(Q.bsf2 + serv[warp][e], S.m);
-      // a pair whose FP32 error bound does not fit the slack is never pruned here
-      if (!fp32_bound_ok(errv[warp][e], thr, S.m)) thr = __int_as_float(0x7f800000);
-      const KeoghSide& wi = side[warp][e][0];
-      const KeoghSide& wj = side[warp][e][1];
-      bool live = keogh_within(S, wi, wj, endsv[warp][e][0], thr, lane);
-      if (live) live = keogh_within(S, wj, wi, endsv[warp][e][1], thr, lane);
-      if (lane == 0) {
-        if (!live) {
-          ++pruned;
+    while (exact) {
+      // the next (up to) eight entries; lane (q, d) owns window d of the q-th
+      unsigned int rest = exact, group = 0;
+      int mine = -1;
+#pragma unroll
+      for (int q = 0; q < kKeoghBatch; ++q) {
+        const int e = rest ? __ffs(rest) - 1 : -1;
+        rest &= rest - 1u;
+        if (e >= 0) group |= 1u << e;
+        if (q == (lane >> 1)) mine = e;
+      }
+      exact &= ~group;
+      const int src = mine < 0 ? 0 : mine, d = lane & 1, q = lane >> 1;
+      const int rx = __shfl_sync(0xffffffffu, r.x, src), ry = __shfl_sync(0xffffffffu, r.y, src);
+      const int rz = __shfl_sync(0xffffffffu, r.z, src);
+      __syncwarp();  // the previous entries are no longer read
+      if (q < kKeoghBatch && mine >= 0) {
+        // window d of the entry, and the end samples of direction d (query =
+        // window d, envelope = the other window) in FP64
+        const unsigned int xe = (unsigned int)(d ? rx : ry);
+        KeoghSide w;
+        w.x = (unsigned int)(d ? ry : rx);
+        w.mu = S.mu[w.x];
+        w.is = S.isg[w.x];
+        const unsigned int b0 = w.x >> kBlkShift;
+        w.o0 = block_offset(S, b0, w.mu, w.is);
+        w.o1 = block_offset(S, b0 + 1, w.mu, w.is);
+        w.pad = 0;
+        side[warp][q][d] = w;
+        const double me = S.mu[xe], ie = S.isg[xe];
+        double t = 0.0;
+#pragma unroll
+        for (int c = 0; c < 2 * kBias; ++c) {
+          const int k = c < kBias ? c : S.m - 2 * kBias + c;
+          const double z = (S.a[w.x + k] - w.mu) * w.is;
+          const double u = (S.U[xe + k] - me) * ie, l = (S.L[xe + k] - me) * ie;
+          const double dd = fmax(fmax(z - u, l - z), 0.0);
+          t = fma(dd, dd, t);
+        }
+        endsv[warp][q][d] = (float)fmax((double)__int_as_float(rz), t);
+        if (d == 0) errv[warp][q] = fmaxf(S.rw[rx], S.rw[ry]);
+      }
+      __syncwarp();
+      for (int x = 0; group; ++x, group &= group - 1u) {
+        const int e = __ffs(group) - 1;
+        float thr = __shfl_sync(0xffffffffu, thr_e, e);
+        // a pair whose FP32 error bound does not fit the slack is never pruned here
+        if (!fp32_bound_ok(errv[warp][x], thr, S.m)) thr = __int_as_float(0x7f800000);
+        const KeoghSide& wi = side[warp][x][0];
+        const KeoghSide& wj = side[warp][x][1];
+        if (!keogh_within(S, wi, wj, endsv[warp][x][0], thr, lane) ||
+            !keogh_within(S, wj, wi, endsv[warp][x][1], thr, lane))
+          alive &= ~(1u << e);
+      }
+    }
+    if (lane == 0) pruned += (unsigned long long)(cnt - __popc(alive));
+    if (alive) {
+      unsigned int base = 0;
+      if (lane == 0) base = atomicAdd(Q.queue_count, (unsigned int)__popc(alive));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if ((alive >> lane) & 1u) {
+        const unsigned int slot = base + __popc(alive & ((1u << lane) - 1u));
+        if (slot < Q.queue_cap) {
+          Q.queue[slot] = make_int2(min(r.x, r.y), max(r.x, r.y));
+          if (Q.qser) Q.qser[slot] = r.w;
         } else {
-          const unsigned int slot = atomicAdd(Q.queue_count, 1u);
-          if (slot < Q.queue_cap) {
-            Q.queue[slot] = make_int2((int)wi.x, (int)wj.x);
-            if (Q.qser) Q.qser[slot] = serv[warp][e];
-          } else {
-            atomicOr(S.status, 2);
-          }
+          atomicOr(S.status, 2);
         }
       }
     }
