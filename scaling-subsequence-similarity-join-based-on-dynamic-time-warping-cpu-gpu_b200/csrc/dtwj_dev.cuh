@@ -359,6 +359,9 @@ void launch_check_finite(const double* a, int64_t n, int* status, cudaStream_t s
 // sid[p] = series of sample p for a batch with series offsets sbeg[0..nseries].
 void launch_series_ids(const int64_t* sbeg, int nseries, int* sid, int64_t n, cudaStream_t st);
 void launch_prep(const DevSeries& S, cudaStream_t st);
+void launch_stats(const DevSeries& S, cudaStream_t st);
+// Update terms of the series alone (dfa, dga); returns the kernels launched.
+int launch_diffs(const DevSeries& S, cudaStream_t st);
 void launch_rowterms(const DevSeries& S, bool masked, cudaStream_t st);
 // Largest CDF length the mask can need: max |z| <= sqrt(m - 1).
 int mask_table_max(int m);
@@ -501,7 +504,8 @@ void launch_dtw_slots32(int cells, const DevSeries& S, const DevSearch& Q, const
 void launch_window_table(const DevSeries& S, const DevSearch& Q, int num_sms, cudaStream_t st);
 // FP64 re-verification of the candidates, then per series the lexicographic
 // minimum (d2, i, j): best_d2[series] (FP64 squared distance, +inf if none),
-// best_ij[series] = i << 32 | j, best_f32[series] = the search's FP32 d2.
+// best_ij[series] = i << 32 | j, best_f32[series] = the search's FP32 d2 (the
+// three arrays follow one another).
 void launch_verify(const DevSeries& S, const DevSearch& Q, BandShape band, double* out_d2,
                    unsigned long long* best_d2, unsigned long long* best_ij, float* best_f32,
                    cudaStream_t st);

@@ -64,6 +64,13 @@ constexpr size_t kWindowTableMax = (size_t)2 << 30;
 // (m, w) groups of a batch joined at the same time, one context each.
 constexpr int kBatchWorkers = 4;
 
+// Status bits: 1 input not finite, 2 a queue overflowed in the current chunk,
+// 8 one did in an earlier chunk of this sweep.
+constexpr int kOverflowSeen = 8;
+// Pinned staging of a join's results; larger ones (per-tile minima) go to
+// pageable memory.
+constexpr size_t kPinBytes = 64 * 1024;
+
 struct Buf {
   void* p = nullptr;
   size_t cap = 0;
@@ -113,7 +120,25 @@ __global__ void k_chunk_note(int* status, const unsigned long long* counters, Ch
   if (t == 0) {
     const int s = *status;
     note->overflow = (s & 2) ? 1u : 0u;
-    *status = s & ~2;
+    *status = (s & 2) ? (s & ~2) | kOverflowSeen : s;
+  }
+}
+
+// The search state of a join before its first DTW: best-so-far +inf per slot,
+// counters, candidates and the seeds' work counter zero.
+__global__ void k_init_search(unsigned int* bsf2, int nslots, unsigned long long* counters,
+                              unsigned int* cand_count, unsigned int* nseeds, int nseries,
+                              int seed_slots, unsigned int* zready) {
+  for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < nslots; x += gridDim.x * blockDim.x)
+    bsf2[x] = 0x7f800000u;
+  if (blockIdx.x == 0) {
+    if (threadIdx.x < kNumCounters) counters[threadIdx.x] = 0ull;
+    if (threadIdx.x == 0) {
+      *cand_count = 0u;
+      nseeds[nseries] = (unsigned int)seed_slots;
+      nseeds[nseries + 1] = 0u;
+      zready[0] = zready[1] = 0u;  // the window table: not filled
+    }
   }
 }
 
@@ -124,10 +149,20 @@ struct dtwj_ctx {
   cudaStream_t stream = nullptr;
   int num_sms = 0;
   std::vector<Buf> bufs;
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_check = nullptr;
   std::vector<Tile> lbtiles_host;    // kLbLags-lag tiles of the diagonal sweep
   int64_t lbtiles_n = -1, lbtiles_m = -1;  // single-series shape the tiles were built for
-  std::vector<unsigned int> host_u32;      // staging of small host -> device copies
+  // what the plain tiles on the device are those of (a single series' join)
+  struct TilesKey {
+    const void* p;
+    int64_t n, m;
+    int rank, world;
+  } tiles_dev = {nullptr, -1, -1, 0, 1};
+  // staging of small device -> host copies: pageable on a context's first call
+  // (pinning costs more than a call can gain), pinned from then on
+  unsigned char* pin = nullptr;
+  std::vector<unsigned char> staging;
+  int calls = 0;
   std::vector<Tile> tiles_run;             // the tiles in the order of the current call
   dtwj_mlp* model = nullptr;               // scores tiles for DTWJ_F_LEARNED (not owned)
   std::vector<std::pair<int, BandShape>> band_override;  // band w -> DTW layout (autotuner)
@@ -142,6 +177,7 @@ struct dtwj_ctx {
   // launch argument is unchanged (same buffers, tiles, band, flags)
   cudaGraphExec_t sweep_exec = nullptr;
   std::vector<unsigned char> sweep_key;
+  std::vector<unsigned char> sweep_seen;  // the last launches made directly
   std::vector<int> sweep_marks;  // phase marks of the capture: (phase, a, b, launches)
   size_t sweep_ev0 = 0, sweep_ev1 = 0;
 };
@@ -149,14 +185,8 @@ struct dtwj_ctx {
 namespace {
 
 enum BufId {
-  B_A = 0, B_MU, B_SIG, B_ISG, B_FLAT, B_U, B_L, B_E, B_NU, B_DFA, B_DGA, B_DFE, B_DGE,
-  B_AC, B_DUL, B_QSIG, B_MASK, B_MN, B_MDUL2, B_MDUL, B_SM, B_SME, B_STATUS,
-  B_COUNTS, B_DIFF, B_MEAN, B_ZMAX, B_KEYS_UP, B_QUEUE, B_QCOUNT,
-  B_BSF2, B_COUNTERS, B_CAND, B_CCOUNT, B_SEEDS, B_NSEEDS, B_VERIFY, B_BEST, B_PAIRS, B_OUT,
-  B_MP, B_MPI, B_CB, B_AF, B_ULF, B_BITS, B_LBTILES, B_KQ, B_SBEG, B_SID, B_SEEDBSF,
-  B_BEST_IJ, B_BEST_F32, B_QSER, B_TILEBEST, B_FEAT, B_SCORE, B_PA, B_CMAX, B_RW,
-  B_MPX_WANT, B_MPX_WREV, B_MPX_MIN, B_MPX_IDX, B_MPX_CAND, B_MPX_CNT, B_NOTES, B_NOTES2,
-  B_SORT, B_SORT_TEMP, B_LBTILES2, B_CMAX2, B_WREC, B_GRP, B_SUP, B_GMEANS, B_GSUP, B_GLIST, B_DENSE, B_ZT, B_ZREADY, B_FQ, B_FUL,
+  B_A = 0, B_WORK, B_KEYS_UP, B_RESULT, B_PAIRS, B_OUT, B_MP, B_MPI, B_LBTILES, B_TILEBEST, B_FEAT, B_SCORE, B_MPX_WANT, B_MPX_WREV, B_MPX_MIN, B_MPX_IDX, B_MPX_CAND,
+  B_MPX_CNT, B_NOTES2, B_SORT, B_SORT_TEMP, B_LBTILES2,
   B_COUNT_
 };
 
@@ -185,6 +215,33 @@ int ensure(dtwj_ctx* c, int id, size_t bytes, void** out) {
     if (_rc) return _rc;                                             \
     ptr = reinterpret_cast<decltype(ptr)>(_p);                       \
   } while (0)
+
+// Several arrays in one device buffer, each on a 256-byte boundary.  An
+// allocation and its release cost 0.7 ms at 10 MB and 2.3 ms at 2 GB, which a
+// one-shot call pays every time: with one buffer, and queues no longer than
+// the series has pairs, the one-shot ECG-like join of 9,001 samples takes 12.8
+// ms (10.6 of them on the device), with a buffer per array it took 17, and 22
+// with pinned staging made for a single call.
+struct Arena {
+  std::vector<std::pair<void**, size_t>> parts;
+  template <typename T>
+  void add(T** p, size_t bytes) {
+    parts.push_back({reinterpret_cast<void**>(p), bytes});
+  }
+  int place(dtwj_ctx* ctx, int id) {
+    size_t total = 0;
+    for (auto& q : parts) total += (q.second + 255) / 256 * 256;
+    void* base = nullptr;
+    const int rc = ensure(ctx, id, total, &base);
+    if (rc) return rc;
+    unsigned char* at = static_cast<unsigned char*>(base);
+    for (auto& q : parts) {
+      *q.first = at;
+      at += (q.second + 255) / 256 * 256;
+    }
+    return DTWJ_OK;
+  }
+};
 
 #define CUDA_OK(expr)                                                 \
   do {                                                                \
@@ -283,138 +340,195 @@ void build_lb_tiles(dtwj_ctx* ctx, int64_t n, int m, const int64_t* sbeg, int ns
   ctx->lbtiles_m = sbeg ? -1 : m;
 }
 
-// Allocates and prepares every per-series array; returns the DevSeries.  A
-// batch (sbeg != nullptr) holds nseries series back to back in x_dev, series
-// r on samples [sbeg[r], sbeg[r + 1]).  groups: also the records of the group
-// filter, where the single-pair block-mean bound reads one offset per window
-// (m <= 1024) and they fit the device (S.grp stays nullptr otherwise: every
-// tile then goes through the diagonal bound).
-int prepare(dtwj_ctx* ctx, const double* x_dev, int64_t n, int m, int w, bool masked, bool groups,
-            const int64_t* sbeg_host, int nseries, DevSeries* out, Phases* ph = nullptr) {
-  const int64_t s = n - m + 1;
-  DevSeries S;
-  memset(&S, 0, sizeof S);
-  S.a = x_dev;
-  S.n = n;
-  S.s = s;
-  S.m = m;
-  S.w = w;
-  S.nseries = nseries;
-  if (sbeg_host) {
-    int64_t* sbeg;
-    int* sid;
-    ENSURE(B_SBEG, (size_t)(nseries + 1) * 8, sbeg);
-    ENSURE(B_SID, (size_t)n * 4, sid);
-    CUDA_OK(cudaMemcpyAsync(sbeg, sbeg_host, (size_t)(nseries + 1) * 8, cudaMemcpyHostToDevice,
-                            ctx->stream));
-    launch_series_ids(sbeg, nseries, sid, n, ctx->stream);
-    S.sbeg = sbeg;
-    S.sid = sid;
+// Host memory for a copy of `bytes` from the device, valid until the next one.
+unsigned char* staging(dtwj_ctx* ctx, size_t bytes) {
+  if (!ctx->pin && ctx->calls > 1 &&
+      cudaHostAlloc(reinterpret_cast<void**>(&ctx->pin), kPinBytes, cudaHostAllocDefault) !=
+          cudaSuccess) {
+    cudaGetLastError();
+    ctx->pin = nullptr;
   }
-  ENSURE(B_MU, s * 8, S.mu);
-  ENSURE(B_SIG, s * 8, S.sig);
-  ENSURE(B_ISG, s * 8, S.isg);
-  ENSURE(B_FLAT, s, S.flat);
-  ENSURE(B_U, n * 8, S.U);
-  ENSURE(B_L, n * 8, S.L);
-  ENSURE(B_E, n * 8, S.E);
-  ENSURE(B_NU, s * 8, S.nu);
-  ENSURE(B_DFA, s * 8, S.dfa);
-  ENSURE(B_DGA, s * 8, S.dga);
-  ENSURE(B_DFE, s * 8, S.dfE);
-  ENSURE(B_DGE, s * 8, S.dgE);
-  ENSURE(B_AC, s * 8, S.A);
-  ENSURE(B_DUL, s * 8, S.DUL);
-  ENSURE(B_QSIG, s * 8, S.qsig);
-  ENSURE(B_MASK, n * 4, S.mask);
-  ENSURE(B_MN, s * 4, S.MN);
-  ENSURE(B_MDUL2, s * 4, S.MDUL2);
-  ENSURE(B_MDUL, s * 4, S.MDUL);
-  ENSURE(B_SM, s * 8, S.SM);
-  ENSURE(B_SME, s * 8, S.SME);
-  ENSURE(B_CB, ((n >> kBlkShift) + 4) * 8, S.cb);
-  ENSURE(B_AF, n * 4, S.af);
-  ENSURE(B_ULF, n * 8, S.ulf);
-  if (m <= (1 << kBlkShift)) {
-    ENSURE(B_PA, (size_t)n * 32, S.pq2);
-    const int fine = paa_block(m) / 4;
-    S.fine_n = n / fine + 2;
-    ENSURE(B_FQ, (size_t)S.fine_n * fine * 2 * sizeof(float), S.fq);
-    ENSURE(B_FUL, (size_t)S.fine_n * fine * 2 * sizeof(float2), S.ful);
-    ENSURE(B_CMAX2, (size_t)kCopyBlocks(n) * 8, S.cmax2);
-    ENSURE(B_WREC, (size_t)s * 16, S.wrec);
-  } else {
-    ENSURE(B_PA, (size_t)n * 16, S.pq);
-  }
-  ENSURE(B_CMAX, ((n >> kBlkShift) + 4) * 4, S.cmax);
-  ENSURE(B_RW, s * 4, S.rw);
-  S.paa_b = paa_block(m);
+  if (ctx->pin && bytes <= kPinBytes) return ctx->pin;
+  if (ctx->staging.size() < bytes) ctx->staging.resize(bytes);
+  return ctx->staging.data();
+}
+
+// How much of a series prepare() makes: the window statistics (pair lists),
+// also the update terms of the covariance recurrence (the matrix profile),
+// also the envelopes and everything a sweep reads, also the records of the
+// group filter (joins).
+enum Prep { kPrepStats, kPrepProfile, kPrepSweep, kPrepJoin };
+
+// What the preparation needs besides the DevSeries' own arrays.
+struct PrepScratch {
+  bool masked = false;
+  Prep level = kPrepStats;
+  const int64_t* sbeg_host = nullptr;
+  int64_t* sbeg = nullptr;
+  int* sid = nullptr;
   double* gmeans = nullptr;
-  if (groups && m <= (1 << kBlkShift)) {
-    group_shape(m, s, &S);
-    void *recs = nullptr, *sups = nullptr, *means = nullptr;
-    if (ensure(ctx, B_GRP, (size_t)S.grp_n * S.grp_d * sizeof(float4), &recs) == DTWJ_OK &&
-        ensure(ctx, B_SUP, (size_t)S.sup_n * S.grp_d * sizeof(float4), &sups) == DTWJ_OK &&
-        ensure(ctx, B_GMEANS, (size_t)n * 24, &means) == DTWJ_OK) {
-      S.grp = static_cast<float4*>(recs);
-      S.sup = static_cast<float4*>(sups);
-      gmeans = static_cast<double*>(means);
-    }
+  unsigned int* counts = nullptr;
+  double *diff = nullptr, *mean = nullptr;
+  float* zmax = nullptr;
+};
+
+// Lays out the per-series arrays in A (not placed yet).  A batch (sbeg !=
+// nullptr) holds nseries series back to back in x_dev, series r on samples
+// [sbeg[r], sbeg[r + 1]).  The group filter's records are made where the
+// single-pair block-mean bound reads one offset per window (m <= 1024);
+// without them every tile goes through the diagonal bound.
+void plan_series(Arena& A, const double* x_dev, int64_t n, int m, int w, bool masked, Prep level,
+                 const int64_t* sbeg_host, int nseries, DevSeries* S, PrepScratch* P) {
+  const int64_t s = n - m + 1;
+  memset(S, 0, sizeof *S);
+  S->a = x_dev;
+  S->n = n;
+  S->s = s;
+  S->m = m;
+  S->w = w;
+  S->nseries = nseries;
+  P->masked = masked;
+  P->level = level;
+  P->sbeg_host = sbeg_host;
+  if (sbeg_host) {
+    A.add(&P->sbeg, (size_t)(nseries + 1) * 8);
+    A.add(&P->sid, (size_t)n * 4);
   }
-  ENSURE(B_STATUS, 4, S.status);
-  cudaStream_t st = ctx->stream;
-  CUDA_OK(cudaMemsetAsync(S.status, 0, 4, st));
-  launch_check_finite(S.a, n, S.status, st);
-  int status = 0;
-  CUDA_OK(cudaMemcpyAsync(&status, S.status, 4, cudaMemcpyDeviceToHost, st));
-  CUDA_OK(cudaStreamSynchronize(st));
-  if (status & 1) return DTWJ_ERR_NAN;
-  if (ph) ph->begin();
-  launch_prep(S, st);
-  if (masked) {
-    const int lt_max = mask_table_max(m);
-    unsigned int* counts;
-    double* diff;
-    double* mean;
-    float* zmax;
-    ENSURE(B_COUNTS, (size_t)m * lt_max * 4, counts);
-    ENSURE(B_DIFF, n * 8, diff);
-    ENSURE(B_MEAN, 8, mean);
-    ENSURE(B_ZMAX, 4, zmax);
-    if (!sbeg_host) {
-      launch_mask(S, counts, lt_max, diff, mean, zmax, st);
+  A.add(&S->mu, s * 8);
+  A.add(&S->sig, s * 8);
+  A.add(&S->isg, s * 8);
+  A.add(&S->flat, s);
+  if (level >= kPrepProfile) {
+    A.add(&S->dfa, s * 8);
+    A.add(&S->dga, s * 8);
+  }
+  if (level >= kPrepSweep) {
+    A.add(&S->U, n * 8);
+    A.add(&S->L, n * 8);
+    A.add(&S->E, n * 8);
+    A.add(&S->nu, s * 8);
+    A.add(&S->dfE, s * 8);
+    A.add(&S->dgE, s * 8);
+    A.add(&S->A, s * 8);
+    A.add(&S->DUL, s * 8);
+    A.add(&S->qsig, s * 8);
+    A.add(&S->cb, ((n >> kBlkShift) + 4) * 8);
+    A.add(&S->af, n * 4);
+    A.add(&S->ulf, n * 8);
+    S->paa_b = paa_block(m);
+    if (m <= (1 << kBlkShift)) {
+      A.add(&S->pq2, (size_t)n * 32);
+      const int fine = S->paa_b / 4;
+      S->fine_n = n / fine + 2;
+      A.add(&S->fq, (size_t)S->fine_n * fine * 2 * sizeof(float));
+      A.add(&S->ful, (size_t)S->fine_n * fine * 2 * sizeof(float2));
+      A.add(&S->cmax2, (size_t)kCopyBlocks(n) * 8);
+      A.add(&S->wrec, (size_t)s * 16);
     } else {
-      // the mask's CDF tables are per series: build it on a view of each one
-      for (int r = 0; r < nseries; ++r) {
-        const int64_t b = sbeg_host[r], nr = sbeg_host[r + 1] - b;
-        DevSeries V = S;
-        V.a = S.a + b;
-        V.n = nr;
-        V.s = nr - m + 1;
-        V.mu = S.mu + b;
-        V.sig = S.sig + b;
-        V.isg = S.isg + b;
-        V.flat = S.flat + b;
-        V.U = S.U + b;
-        V.L = S.L + b;
-        V.mask = S.mask + b;
-        V.sid = nullptr;
-        V.sbeg = nullptr;
-        V.nseries = 1;
-        launch_mask(V, counts, lt_max, diff, mean, zmax, st);
+      A.add(&S->pq, (size_t)n * 16);
+    }
+    A.add(&S->cmax, ((n >> kBlkShift) + 4) * 4);
+    A.add(&S->rw, s * 4);
+  }
+  if (masked) {
+    A.add(&S->mask, n * 4);
+    A.add(&S->MN, s * 4);
+    A.add(&S->MDUL2, s * 4);
+    A.add(&S->MDUL, s * 4);
+    A.add(&S->SM, s * 8);
+    A.add(&S->SME, s * 8);
+    A.add(&P->zmax, 4);
+    A.add(&P->counts, (size_t)m * mask_table_max(m) * 4);
+    A.add(&P->diff, n * 8);
+    A.add(&P->mean, 8);
+  }
+  if (level >= kPrepJoin && m <= (1 << kBlkShift)) {
+    group_shape(m, s, S);
+    A.add(&S->grp, (size_t)S->grp_n * S->grp_d * sizeof(float4));
+    A.add(&S->sup, (size_t)S->sup_n * S->grp_d * sizeof(float4));
+    A.add(&P->gmeans, (size_t)n * 24);
+  }
+  A.add(&S->status, 4);
+}
+
+// Prepares the planned and placed arrays.
+int prepare(dtwj_ctx* ctx, DevSeries& S, const PrepScratch& P, Phases* ph = nullptr) {
+  const int m = S.m;
+  const bool masked = P.masked;
+  const Prep level = P.level;
+  const int64_t* sbeg_host = P.sbeg_host;
+  if (sbeg_host) {
+    CUDA_OK(cudaMemcpyAsync(P.sbeg, sbeg_host, (size_t)(S.nseries + 1) * 8, cudaMemcpyHostToDevice,
+                            ctx->stream));
+    launch_series_ids(P.sbeg, S.nseries, P.sid, S.n, ctx->stream);
+    S.sbeg = P.sbeg;
+    S.sid = P.sid;
+  }
+  cudaStream_t st = ctx->stream;
+  // the check of the input: its verdict travels while the preparation runs
+  int* verdict = reinterpret_cast<int*>(staging(ctx, 4));
+  CUDA_OK(cudaMemsetAsync(S.status, 0, 4, st));
+  launch_check_finite(S.a, S.n, S.status, st);
+  CUDA_OK(cudaMemcpyAsync(verdict, S.status, 4, cudaMemcpyDeviceToHost, st));
+  CUDA_OK(cudaEventRecord(ctx->ev_check, st));
+  if (ph) ph->begin();
+  int launches = 1;
+  if (level < kPrepSweep) {
+    launch_stats(S, st);
+    if (level == kPrepProfile) launches += launch_diffs(S, st);
+  } else {
+    launch_prep(S, st);
+    if (masked) {
+      const int lt_max = mask_table_max(m);
+      unsigned int* counts = P.counts;
+      double *diff = P.diff, *mean = P.mean;
+      float* zmax = P.zmax;
+      if (!sbeg_host) {
+        launch_mask(S, counts, lt_max, diff, mean, zmax, st);
+      } else {
+        // the mask's CDF tables are per series: build it on a view of each one
+        for (int r = 0; r < S.nseries; ++r) {
+          const int64_t b = sbeg_host[r], nr = sbeg_host[r + 1] - b;
+          DevSeries V = S;
+          V.a = S.a + b;
+          V.n = nr;
+          V.s = nr - m + 1;
+          V.mu = S.mu + b;
+          V.sig = S.sig + b;
+          V.isg = S.isg + b;
+          V.flat = S.flat + b;
+          V.U = S.U + b;
+          V.L = S.L + b;
+          V.mask = S.mask + b;
+          V.sid = nullptr;
+          V.sbeg = nullptr;
+          V.nseries = 1;
+          launch_mask(V, counts, lt_max, diff, mean, zmax, st);
+        }
       }
     }
-  } else {
-    CUDA_OK(cudaMemsetAsync(S.mask, 0, n * 4, st));
+    launch_rowterms(S, masked, st);
+    launch_center(S, st);
+    launches = (masked ? 11 : 6) + launch_paa_prep(S, st);
+    if (S.grp) launches += launch_group_prep(S, P.gmeans, st);
   }
-  launch_rowterms(S, masked, st);
-  launch_center(S, st);
-  int paa_launches = launch_paa_prep(S, st);
-  if (S.grp) paa_launches += launch_group_prep(S, gmeans, st);
-  if (ph) ph->end(DTWJ_PHASE_PREP, (masked ? 11 : 6) + paa_launches);
+  if (ph) ph->end(DTWJ_PHASE_PREP, launches);
   CUDA_OK(cudaGetLastError());
-  *out = S;
+  CUDA_OK(cudaEventSynchronize(ctx->ev_check));
+  if (*verdict & 1) {
+    CUDA_OK(cudaStreamSynchronize(st));  // nothing reads the caller's series any more
+    return DTWJ_ERR_NAN;
+  }
   return DTWJ_OK;
+}
+
+// The same in one, for calls that need no other buffers of the arena.
+int plan_and_prepare(dtwj_ctx* ctx, const double* x_dev, int64_t n, int m, int w, bool masked,
+                     Prep level, DevSeries* S, PrepScratch* P) {
+  Arena A;
+  plan_series(A, x_dev, n, m, w, masked, level, nullptr, 1, S, P);
+  const int rc = A.place(ctx, B_WORK);
+  return rc ? rc : prepare(ctx, *S, *P);
 }
 
 int effective_band(int m, int w) { return w > m - 1 ? m - 1 : w; }
@@ -461,121 +575,171 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   Phases ph(ctx, (flags & DTWJ_F_PROFILE) != 0);
   CUDA_OK(cudaEventRecord(ctx->ev0, st));
 
-  DevSeries S;
-  int rc = prepare(ctx, x_dev, n, m, w, masked, !(flags & DTWJ_F_NO_DIAG), sbeg, nseries, &S, &ph);
-  if (rc) return rc;
-
-  build_lb_tiles(ctx, n, m, sbeg, nseries);
+  // tiles of the sweep; a single series' stay on the device while its shape and
+  // shard do
+  const int world = tq ? 1 : ctx->shard_world, rank = tq ? 0 : ctx->shard_rank;
   std::vector<Tile>& th = ctx->tiles_run;
-  th = ctx->lbtiles_host;
-  if (ctx->shard_world > 1 && !tq) {
-    // one shard of the tiles (round robin): the profile, the seeds and the
-    // sweep only see these; the shards' results combine by their minimum
-    size_t k = 0;
-    for (size_t t = 0; t < th.size(); ++t)
-      if ((int)(t % (size_t)ctx->shard_world) == ctx->shard_rank) th[k++] = th[t];
-    th.resize(k);
+  const auto& tk = ctx->tiles_dev;
+  const bool keep_tiles = !sbeg && !tile_mode && tk.p && tk.p == ctx->bufs[B_LBTILES].p &&
+                          tk.n == n && tk.m == m && tk.rank == rank && tk.world == world;
+  if (!keep_tiles) {
+    ctx->tiles_dev.p = nullptr;  // until the new ones are on their way
+    build_lb_tiles(ctx, n, m, sbeg, nseries);
+    th = ctx->lbtiles_host;
+    if (world > 1) {
+      // one shard of the tiles (round robin): the profile, the seeds and the
+      // sweep only see these; the shards' results combine by their minimum
+      size_t k = 0;
+      for (size_t t = 0; t < th.size(); ++t)
+        if ((int)(t % (size_t)world) == rank) th[k++] = th[t];
+      th.resize(k);
+    }
   }
   const int nlb = (int)th.size();
   // best-so-far slots: one per series, or one per tile for the tile minima
   const int nslots = tile_mode ? (nlb > 0 ? nlb : 1) : nseries;
-  S.nseries = nslots;
-  if (tile_mode)
-    for (int t = 0; t < nlb; ++t) th[t].series = t;
-  Tile* lbtiles;
-  ENSURE(B_LBTILES, (size_t)(nlb > 0 ? nlb : 1) * sizeof(Tile), lbtiles);
-  if (nlb > 0)
-    CUDA_OK(cudaMemcpyAsync(lbtiles, th.data(), (size_t)nlb * sizeof(Tile),
-                            cudaMemcpyHostToDevice, st));
 
-  // the window table of the slot DTW, where it fits its limit and the device
-  if (band.C <= 8) {
-    const int64_t zm = (m + 3) / 4 * 4;
-    const size_t row = (size_t)S.s * zm * sizeof(float);
-    void *zt = nullptr, *zr = nullptr;
-    if (3 * row <= kWindowTableMax && ensure(ctx, B_ZT, 3 * row, &zt) == DTWJ_OK &&
-        ensure(ctx, B_ZREADY, 8, &zr) == DTWJ_OK) {
-      S.zt = static_cast<float*>(zt);
-      S.zu = S.zt + S.s * zm;
-      S.zl = S.zu + S.s * zm;
-      S.zm = (int)zm;
-      S.zready = static_cast<unsigned int*>(zr);
-      CUDA_OK(cudaMemsetAsync(S.zready, 0, 8, st));
-    }
-  }
-
-  // search state
+  // what the call returns, in one block: [nslots] best_d2, best_ij, best_f32,
+  // seed_bsf, then the counters, the candidate count and the status word
+  unsigned long long *best_d2, *best_ij;
+  float* best_f32;
+  unsigned int* seed_bsf;
   DevSearch Q;
   memset(&Q, 0, sizeof Q);
+  int* status_dev;
+  const size_t at_counters = ((size_t)nslots * 24 + 7) / 8 * 8;
+  const size_t result_bytes = at_counters + kNumCounters * 8 + 8;
+  unsigned char* result_dev;
+  ENSURE(B_RESULT, result_bytes, result_dev);
+  best_d2 = reinterpret_cast<unsigned long long*>(result_dev);
+  best_ij = best_d2 + nslots;
+  best_f32 = reinterpret_cast<float*>(best_ij + nslots);
+  seed_bsf = reinterpret_cast<unsigned int*>(best_f32 + nslots);
+  Q.counters = reinterpret_cast<unsigned long long*>(result_dev + at_counters);
+  Q.cand_count = reinterpret_cast<unsigned int*>(Q.counters + kNumCounters);
+  status_dev = reinterpret_cast<int*>(Q.cand_count + 1);
+
+  // every buffer of the call in one allocation, the group filter's and the
+  // window table's only where they fit the device
+  DevSeries S;
+  PrepScratch P;
+  // search state
   unsigned int qcap = kQueueCapMax;
   if (const char* env = getenv("DTWJ_QUEUE_CAP")) {  // smaller queue (profiling, tests)
     const long v = atol(env);
     if (v >= 1024 && v < (long)kQueueCapMax) qcap = (unsigned int)v;
   }
-  // LB_Keogh candidates of one chunk, and those that go on to DTW (nearly all
-  // of them on quasi-periodic series)
-  ENSURE(B_KQ, (size_t)qcap * 2 * sizeof(int4), Q.kq);
-  ENSURE(B_QUEUE, (size_t)qcap * 2 * sizeof(int2), Q.queue);
   const bool enumerate_all = flags & DTWJ_F_NO_DIAG;
-  const double tile_pairs = (double)kLbLags * kLbRows;
+  const double full_tile = (double)kLbLags * kLbRows;
   int chunk = ctx->chunk_tiles > 0 ? ctx->chunk_tiles
                                    : kLbChunkRounds * kLbCtasPerSm * ctx->num_sms;
-  if (enumerate_all) chunk = (int)((double)qcap / tile_pairs) > 0 ? (int)((double)qcap / tile_pairs) : 1;
+  if (enumerate_all) chunk = (int)((double)qcap / full_tile) > 0 ? (int)((double)qcap / full_tile) : 1;
   const int chunk_max = chunk < nlb ? chunk : (nlb > 0 ? nlb : 1);  // tiles of the largest chunk
-  // counters of a chunk, then the group filter's surviving group pairs per tile
-  constexpr int kQcTiles = 16;
-  unsigned int* qc;
-  ENSURE(B_QCOUNT, (size_t)(kQcTiles + chunk_max) * 4, qc);
-  Q.queue_count = qc;
-  Q.queue_next = qc + 1;
-  Q.run_count = qc + 2;
-  Q.run_next = qc + 3;
-  Q.kq_count = qc + 4;
-  Q.kq_next = qc + 5;
-  unsigned int* lb_next = qc + 6;
-  GroupFilter F;
-  memset(&F, 0, sizeof F);
-  F.nsup = qc + 8;
-  F.nlist = qc + 9;
-  F.ndense = qc + 10;
-  unsigned int* paa_next = qc + 11;
-  ENSURE(B_DENSE, (size_t)chunk_max * 4, F.dense);
-  if (S.grp) {
-    const size_t pairs = (size_t)chunk_max * group_items(S.grp_g, &F);
-    ENSURE(B_GSUP, pairs * 4, F.sup);
-    ENSURE(B_GLIST, pairs * sizeof(uint2), F.list);
-    F.sup_cap = F.list_cap = (unsigned int)pairs;
-    F.tcount = qc + kQcTiles;
+  // LB_Keogh candidates of one chunk, and those that go on to DTW (nearly all
+  // of them on quasi-periodic series): no more than the call has pairs
+  double pairs_bound = 1024.0;
+  for (int r = 0; r < nseries; ++r) {
+    const double k = (double)((sbeg ? sbeg[r + 1] - sbeg[r] : n) - 2 * (int64_t)m + 1);
+    pairs_bound += 0.5 * k * (k + 1.0);
   }
-  Q.queue_cap = qcap * 2;
-  Q.kq_cap = qcap * 2;
-  Q.runs = nullptr;
-  Q.run_cap = 0;
-  ENSURE(B_BSF2, (size_t)nslots * 4, Q.bsf2);
-  ENSURE(B_COUNTERS, kNumCounters * 8, Q.counters);
+  const unsigned int queue_cap =
+      pairs_bound < 2.0 * qcap ? (unsigned int)pairs_bound : qcap * 2;
+  Q.queue_cap = Q.kq_cap = queue_cap;
   // the tile minima keep a few candidates per tile
   const unsigned int cand_cap =
       tile_mode && 16u * (unsigned int)nlb > kCandCap ? 16u * (unsigned int)nlb : kCandCap;
-  ENSURE(B_CAND, (size_t)cand_cap * sizeof(Candidate), Q.cand);
-  ENSURE(B_CCOUNT, 4, Q.cand_count);
   Q.cand_cap = cand_cap;
-  if (tile_mode) ENSURE(B_QSER, (size_t)qcap * 2 * sizeof(int), Q.qser);
-  CUDA_OK(cudaMemsetAsync(Q.counters, 0, kNumCounters * 8, st));
-  CUDA_OK(cudaMemsetAsync(Q.cand_count, 0, 4, st));
-  ctx->host_u32.assign((size_t)nslots + 1, 0x7f800000u);  // +inf per slot
-  CUDA_OK(cudaMemcpyAsync(Q.bsf2, ctx->host_u32.data(), (size_t)nslots * 4,
-                          cudaMemcpyHostToDevice, st));
-  unsigned int* seed_bsf;
-  ENSURE(B_SEEDBSF, (size_t)nslots * 4, seed_bsf);
+  using Range = std::pair<int, int>;
+  std::vector<Range> ranges;
+  for (int t0 = 0; t0 < nlb; t0 += chunk) ranges.push_back({t0, t0 + chunk < nlb ? t0 + chunk : nlb});
+  const bool want_features = learned || (tq && tq->features);
+  const bool want_keys = nlb > 0 && (tile_mode || want_features || !(flags & DTWJ_F_NO_SEED));
+  // counters of a chunk, then the group filter's surviving group pairs per tile
+  constexpr int kQcTiles = 16;
+  unsigned int *qc, *nseeds, *bits;  // nseeds: [nseries] counts, total slots, work counter
+  unsigned long long* keys;          // row minima of the ED profile
+  int2* seeds;
+  ChunkNote* notes;
+  double* vd2;
+  GroupFilter F;
+  memset(&F, 0, sizeof F);
+  const size_t table = 3 * (size_t)(n - m + 1) * ((m + 3) / 4 * 4) * sizeof(float);
+  bool want_table = band.C <= 8 && table <= kWindowTableMax && !(tq && !tile_mode);
+  Prep level = enumerate_all || (tq && !tile_mode) ? kPrepSweep : kPrepJoin;
+  int rc = DTWJ_OK;
+  for (;;) {
+    Arena A;
+    plan_series(A, x_dev, n, m, w, masked, level, sbeg, nseries, &S, &P);
+    if (want_keys) A.add(&keys, S.s * 8);
+    if (!tq || tile_mode) {
+      A.add(&qc, (size_t)(kQcTiles + chunk_max) * 4);
+      A.add(&F.dense, (size_t)chunk_max * 4);
+      A.add(&Q.bsf2, (size_t)nslots * 4);
+      A.add(&S.zready, 8);
+      A.add(&seeds, (size_t)nseries * kSeedSlots * sizeof(int2));
+      A.add(&nseeds, ((size_t)nseries + 2) * 4);
+      A.add(&notes, (ranges.size() + 1) * sizeof(ChunkNote));
+      A.add(&Q.cand, (size_t)cand_cap * sizeof(Candidate));
+      A.add(&vd2, (size_t)cand_cap * 8);
+      if (level == kPrepJoin && m <= (1 << kBlkShift)) {
+        const size_t pairs = (size_t)chunk_max * group_items(S.grp_g, &F);
+        A.add(&F.sup, pairs * 4);
+        A.add(&F.list, pairs * sizeof(uint2));
+        F.sup_cap = F.list_cap = (unsigned int)pairs;
+      }
+      A.add(&bits, (size_t)chunk_max * kLbLags * kLbWords * 4);
+      if (tile_mode) A.add(&Q.qser, (size_t)queue_cap * sizeof(int));
+      if (want_table) A.add(&S.zt, table);
+      A.add(&Q.queue, (size_t)queue_cap * sizeof(int2));
+      A.add(&Q.kq, (size_t)queue_cap * sizeof(int4));
+    }
+    rc = A.place(ctx, B_WORK);
+    if (rc != DTWJ_ERR_OOM) break;
+    if (want_table) want_table = false;
+    else if (level == kPrepJoin) level = kPrepSweep;
+    else break;
+  }
+  if (rc) return rc;
+  S.status = status_dev;
+  if (want_table) {
+    S.zm = (m + 3) / 4 * 4;
+    S.zu = S.zt + S.s * S.zm;
+    S.zl = S.zu + S.s * S.zm;
+  }
+  rc = prepare(ctx, S, P, &ph);
+  if (rc) return rc;
+  S.nseries = nslots;
+  if (tile_mode)
+    for (int t = 0; t < nlb; ++t) th[t].series = t;
+  Tile* lbtiles;
+  ENSURE(B_LBTILES, (size_t)(nlb > 0 ? nlb : 1) * sizeof(Tile), lbtiles);
+  if (!keep_tiles) {
+    if (nlb > 0)
+      CUDA_OK(cudaMemcpyAsync(lbtiles, th.data(), (size_t)nlb * sizeof(Tile),
+                              cudaMemcpyHostToDevice, st));
+    ctx->tiles_dev = {sbeg || tile_mode ? nullptr : lbtiles, n, m, rank, world};
+  }
 
-  unsigned int* bits;
-  ENSURE(B_BITS, (size_t)chunk_max * kLbLags * kLbWords * 4, bits);
+  unsigned int *lb_next = nullptr, *paa_next = nullptr;
+  if (!tq || tile_mode) {
+    Q.queue_count = qc;
+    Q.queue_next = qc + 1;
+    Q.run_count = qc + 2;
+    Q.run_next = qc + 3;
+    Q.kq_count = qc + 4;
+    Q.kq_next = qc + 5;
+    lb_next = qc + 6;
+    F.nsup = qc + 8;
+    F.nlist = qc + 9;
+    F.ndense = qc + 10;
+    paa_next = qc + 11;
+    if (S.grp) F.tcount = qc + kQcTiles;
+    k_init_search<<<(nslots + 255) / 256 < 256 ? (nslots + 255) / 256 : 256, 256, 0, st>>>(
+        Q.bsf2, nslots, Q.counters, Q.cand_count, nseeds, nseries, nseries * kSeedSlots, S.zready);
+  }
 
   // ---- ED matrix profile (row minima; per tile for the tile minima) ----
-  const bool want_features = learned || (tq && tq->features);
-  unsigned long long* keys = nullptr;
-  if (nlb > 0 && (tile_mode || want_features || !(flags & DTWJ_F_NO_SEED))) {
-    ENSURE(B_KEYS_UP, S.s * 8, keys);
+  if (want_keys) {
     unsigned int* tbest = nullptr;
     if (tile_mode) {
       ENSURE(B_TILEBEST, (size_t)nlb * 4, tbest);
@@ -647,8 +811,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
       Tile* sorted;
       ENSURE(B_LBTILES2, (size_t)nlb * sizeof(Tile), sorted);
       k_gather_tiles<<<nb, 256, 0, st>>>(lbtiles, si_out, nlb, sorted);
-      CUDA_OK(cudaMemcpyAsync(lbtiles, sorted, (size_t)nlb * sizeof(Tile),
-                              cudaMemcpyDeviceToDevice, st));
+      lbtiles = sorted;
     }
   }
   if (tq && !tile_mode) {
@@ -658,14 +821,6 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
 
   // ---- ED profile seeds ----
   if (!tile_mode && !(flags & DTWJ_F_NO_SEED) && nlb > 0) {
-    int2* seeds;
-    unsigned int* nseeds;  // [nseries] counts, total slots, work counter
-    ENSURE(B_SEEDS, (size_t)nseries * kSeedSlots * sizeof(int2), seeds);
-    ENSURE(B_NSEEDS, ((size_t)nseries + 2) * 4, nseeds);
-    ctx->host_u32[0] = (unsigned int)(nseries * kSeedSlots);
-    CUDA_OK(cudaMemcpyAsync(nseeds + nseries, ctx->host_u32.data(), 4, cudaMemcpyHostToDevice,
-                            st));
-    CUDA_OK(cudaMemsetAsync(nseeds + nseries + 1, 0, 4, st));
     ph.begin();
     launch_seed_select(S, keys, seeds, nseeds, st);
     DevSearch Qs = Q;
@@ -703,7 +858,6 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   // one pass over tile ranges: bound sweep, run filter, LB_Keogh, DTW, and a
   // note of each range (queue overflow, counters after it); notes[0] holds
   // the counters before the pass, notes[c + 1] those after range c
-  using Range = std::pair<int, int>;
   auto sweep_range = [&](const Range& r, ChunkNote* note) {
     CUDA_OK(cudaMemsetAsync(qc, 0, (size_t)(kQcTiles + r.second - r.first) * 4, st));
     ph.begin();
@@ -723,10 +877,6 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     CUDA_OK(cudaGetLastError());
     return DTWJ_OK;
   };
-  std::vector<Range> ranges;
-  for (int t0 = 0; t0 < nlb; t0 += chunk) ranges.push_back({t0, t0 + chunk < nlb ? t0 + chunk : nlb});
-  ChunkNote* notes;
-  ENSURE(B_NOTES, (ranges.size() + 1) * sizeof(ChunkNote), notes);
   // a sharded join with an exchange sweeps its tiles in phases and lets the
   // caller lower the best-so-far between them (direct launches)
   const bool exchanging = ctx->exchange && ctx->shard_world > 1 && !tq;
@@ -744,6 +894,19 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     CUDA_OK(cudaGetLastError());
     return DTWJ_OK;
   };
+  // FP64 verification of the candidates, the minimum per series, and the
+  // result block on its way to the host
+  unsigned char* result = staging(ctx, result_bytes);
+  auto finish = [&]() -> int {
+    ph.begin();
+    launch_verify(S, Q, wide, vd2, best_d2, best_ij, best_f32, st);
+    ph.end(DTWJ_PHASE_VERIFY, 4);
+    CUDA_OK(cudaEventRecord(ctx->ev1, st));
+    CUDA_OK(cudaMemcpyAsync(result, result_dev, result_bytes, cudaMemcpyDeviceToHost, st));
+    CUDA_OK(cudaStreamSynchronize(st));
+    return DTWJ_OK;
+  };
+  const int* status_h = reinterpret_cast<const int*>(result + at_counters + kNumCounters * 8 + 4);
   // A batch sweeps chunk by chunk and checks each one: its short series put
   // many tiles' survivors into one chunk, and when a chunk's queues
   // overflow, the counters go back to before it, it is swept again in
@@ -780,7 +943,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     CUDA_OK(cudaGetLastError());
     if (verbose && resweeps)
       fprintf(stderr, "dtwj: %zu chunks swept again in smaller chunks\n", resweeps);
-    ranges.clear();
+    if ((rc = finish())) return rc;
   }
   for (int attempt = 0; !adaptive; ++attempt) {
     bool swept = false;
@@ -811,6 +974,9 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
       put(&F, sizeof F);
       put(band_cg, sizeof band_cg);
       put(misc, sizeof misc);
+      // a context's first join launches directly: it may be its only one
+      const bool seen = key == ctx->sweep_seen;
+      if (!seen) ctx->sweep_seen = key;
       if (ctx->sweep_exec && key == ctx->sweep_key) {
         CUDA_OK(cudaGraphLaunch(ctx->sweep_exec, st));
         for (size_t k = 0; k + 3 < ctx->sweep_marks.size(); k += 4)
@@ -818,7 +984,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
                               (size_t)ctx->sweep_marks[k + 2], ctx->sweep_marks[k + 3]});
         ph.used = ctx->sweep_ev1;
         swept = true;
-      } else {
+      } else if (seen) {
         if (ctx->sweep_exec) cudaGraphExecDestroy(ctx->sweep_exec);
         ctx->sweep_exec = nullptr;
         ctx->sweep_key.clear();
@@ -866,9 +1032,11 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
       const int src = sweep(ranges, pass_notes);
       if (src) return src;
     }
+    if ((rc = finish())) return rc;
     // a chunk whose queue overflowed lost pairs: take its counts out and
     // sweep it again in smaller chunks (the other chunks stand)
-    if (ranges.empty()) break;
+    if (ranges.empty() || !(*status_h & kOverflowSeen)) break;
+    CUDA_OK(cudaMemsetAsync(S.status, 0, 4, st));
     std::vector<ChunkNote> nh(ranges.size() + 1);
     CUDA_OK(cudaMemcpyAsync(nh.data(), pass_notes, nh.size() * sizeof(ChunkNote),
                             cudaMemcpyDeviceToHost, st));
@@ -899,33 +1067,15 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     ranges.swap(again);
   }
 
-  // ---- FP64 verification of the candidates, per-series minimum ----
-  double* vd2;
-  ENSURE(B_VERIFY, (size_t)kCandCap * 8, vd2);
-  unsigned long long *best_d2, *best_ij;
-  float* best_f32;
-  ENSURE(B_BEST, (size_t)nslots * 8, best_d2);
-  ENSURE(B_BEST_IJ, (size_t)nslots * 8, best_ij);
-  ENSURE(B_BEST_F32, (size_t)nslots * 4, best_f32);
-  ph.begin();
-  launch_verify(S, Q, wide, vd2, best_d2, best_ij, best_f32, st);
-  ph.end(DTWJ_PHASE_VERIFY, 4);
-  CUDA_OK(cudaEventRecord(ctx->ev1, st));
-
-  std::vector<unsigned long long> d2_h(nslots), ij_h(nslots);
-  std::vector<unsigned int> f32_h(nslots), seed_h(nslots);
-  unsigned long long cnt_h[kNumCounters];
-  unsigned int cand_h = 0;
-  int status_h = 0;
-  CUDA_OK(cudaMemcpyAsync(d2_h.data(), best_d2, (size_t)nslots * 8, cudaMemcpyDeviceToHost, st));
-  CUDA_OK(cudaMemcpyAsync(ij_h.data(), best_ij, (size_t)nslots * 8, cudaMemcpyDeviceToHost, st));
-  CUDA_OK(cudaMemcpyAsync(f32_h.data(), best_f32, (size_t)nslots * 4, cudaMemcpyDeviceToHost, st));
-  CUDA_OK(cudaMemcpyAsync(seed_h.data(), seed_bsf, (size_t)nslots * 4, cudaMemcpyDeviceToHost, st));
-  CUDA_OK(cudaMemcpyAsync(cnt_h, Q.counters, sizeof cnt_h, cudaMemcpyDeviceToHost, st));
-  CUDA_OK(cudaMemcpyAsync(&cand_h, Q.cand_count, 4, cudaMemcpyDeviceToHost, st));
-  CUDA_OK(cudaMemcpyAsync(&status_h, S.status, 4, cudaMemcpyDeviceToHost, st));
-  CUDA_OK(cudaStreamSynchronize(st));
-  if (status_h & 2) return DTWJ_ERR_OVERFLOW;
+  // ---- results ----
+  const unsigned long long* d2_h = reinterpret_cast<const unsigned long long*>(result);
+  const unsigned long long* ij_h = d2_h + nslots;
+  const unsigned int* f32_h = reinterpret_cast<const unsigned int*>(ij_h + nslots);
+  const unsigned int* seed_h = f32_h + nslots;
+  const unsigned long long* cnt_h =
+      reinterpret_cast<const unsigned long long*>(result + at_counters);
+  const unsigned int cand_h = *reinterpret_cast<const unsigned int*>(cnt_h + kNumCounters);
+  if (*status_h & 2) return DTWJ_ERR_OVERFLOW;
   if (cand_h > cand_cap) return DTWJ_ERR_OVERFLOW;
   float ms = 0;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
@@ -1020,8 +1170,11 @@ int dtwj_ctx_create(int device, dtwj_ctx** out) {
   }
   cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device);
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess) {
-    delete c;
+      cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->ev_check, cudaEventDisableTiming) != cudaSuccess) {
+    cudaGetLastError();
+    c->bufs.resize(B_COUNT_);
+    dtwj_ctx_destroy(c);
     return DTWJ_ERR_CUDA;
   }
   c->bufs.resize(B_COUNT_);
@@ -1032,13 +1185,15 @@ int dtwj_ctx_create(int device, dtwj_ctx** out) {
 void dtwj_ctx_destroy(dtwj_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
-  cudaStreamSynchronize(c->stream);
+  if (c->stream) cudaStreamSynchronize(c->stream);
   for (auto& b : c->bufs)
     if (b.p) cudaFree(b.p);
   if (c->sweep_exec) cudaGraphExecDestroy(c->sweep_exec);
   for (auto e : c->pool) cudaEventDestroy(e);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
+  if (c->ev_check) cudaEventDestroy(c->ev_check);
+  if (c->pin) cudaFreeHost(c->pin);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -1109,7 +1264,8 @@ int dtwj_time_band(int device, int32_t m, int32_t w, int32_t C, int32_t G, int32
     double* dev = nullptr;
     if ((rc = upload(ctx, x.data(), n, &dev))) break;
     DevSeries S;
-    if ((rc = prepare(ctx, dev, n, m, we, false, false, nullptr, 1, &S))) break;
+    PrepScratch P;
+    if ((rc = plan_and_prepare(ctx, dev, n, m, we, false, kPrepStats, &S, &P))) break;
     std::vector<int2> pr((size_t)pairs);
     const int64_t s = n - m + 1;
     for (int q = 0; q < pairs; ++q) {
@@ -1345,8 +1501,9 @@ int dtwj_matrix_profile(const double* x, int64_t n, int32_t m, double* mp, int64
       break;
     }
     DevSeries S, R;
-    if ((rc = prepare(ctx, dev, n, m, 0, false, false, nullptr, 1, &S))) break;
-    if ((rc = prepare(rev, rdev, n, m, 0, false, false, nullptr, 1, &R))) break;
+    PrepScratch P;
+    if ((rc = plan_and_prepare(ctx, dev, n, m, 0, false, kPrepProfile, &S, &P))) break;
+    if ((rc = plan_and_prepare(rev, rdev, n, m, 0, false, kPrepProfile, &R, &P))) break;
     build_lb_tiles(ctx, n, m, nullptr, 1);
     const int nlb = (int)ctx->lbtiles_host.size();
     if ((rc = ensure(ctx, B_LBTILES, (size_t)nlb * sizeof(Tile), &p))) break;
@@ -1436,7 +1593,8 @@ int dtwj_global_mask(const double* x, int64_t n, int32_t m, int32_t w, float* ma
     double* dev = nullptr;
     if ((rc = upload(ctx, x, n, &dev))) break;
     DevSeries S;
-    if ((rc = prepare(ctx, dev, n, m, we, true, false, nullptr, 1, &S))) break;
+    PrepScratch P;
+    if ((rc = plan_and_prepare(ctx, dev, n, m, we, true, kPrepSweep, &S, &P))) break;
     if (cudaMemcpyAsync(mask, S.mask, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream) !=
             cudaSuccess ||
         cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
@@ -1446,9 +1604,7 @@ int dtwj_global_mask(const double* x, int64_t n, int32_t m, int32_t w, float* ma
     if (table_len) {
       // the table length the mask used: 200 floor(max |z|), at least 600
       float zmax = 0.0f;
-      void* p = nullptr;
-      if ((rc = ensure(ctx, B_ZMAX, 4, &p))) break;
-      if (cudaMemcpy(&zmax, p, 4, cudaMemcpyDeviceToHost) != cudaSuccess) {
+      if (cudaMemcpy(&zmax, P.zmax, 4, cudaMemcpyDeviceToHost) != cudaSuccess) {
         rc = DTWJ_ERR_CUDA;
         break;
       }
@@ -1482,7 +1638,8 @@ int dtwj_pair_dtw(const double* x, int64_t n, int32_t m, int32_t w, const int64_
     double* dev = nullptr;
     if ((rc = upload(ctx, x, n, &dev))) break;
     DevSeries S;
-    if ((rc = prepare(ctx, dev, n, m, we, false, false, nullptr, 1, &S))) break;
+    PrepScratch P;
+    if ((rc = plan_and_prepare(ctx, dev, n, m, we, false, kPrepStats, &S, &P))) break;
     void* p;
     if ((rc = ensure(ctx, B_PAIRS, (size_t)count * sizeof(int2), &p))) break;
     int2* dp = (int2*)p;
@@ -1525,7 +1682,8 @@ int dtwj_pair_lb_petitjean(const double* x, int64_t n, int32_t m, int32_t w, con
     double* dev = nullptr;
     if ((rc = upload(ctx, x, n, &dev))) break;
     DevSeries S;
-    if ((rc = prepare(ctx, dev, n, m, we, false, false, nullptr, 1, &S))) break;
+    PrepScratch P;
+    if ((rc = plan_and_prepare(ctx, dev, n, m, we, false, kPrepSweep, &S, &P))) break;
     void* p;
     if ((rc = ensure(ctx, B_PAIRS, (size_t)count * sizeof(int2), &p))) break;
     int2* dp = (int2*)p;

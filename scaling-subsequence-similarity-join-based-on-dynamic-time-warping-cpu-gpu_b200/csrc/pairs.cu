@@ -765,9 +765,7 @@ void launch_verify(const DevSeries& S, const DevSearch& Q, BandShape band, doubl
   DTWJ_BAND_CASES(X)
 #undef X
   const int ns = S.nseries;
-  cudaMemsetAsync(best_d2, 0xff, (size_t)ns * 8, st);
-  cudaMemsetAsync(best_ij, 0xff, (size_t)ns * 8, st);
-  cudaMemsetAsync(best_f32, 0xff, (size_t)ns * 4, st);
+  cudaMemsetAsync(best_d2, 0xff, (size_t)ns * 20, st);
   const int cap = (int)Q.cand_cap;
   k_best_d2<<<256, 256, 0, st>>>(Q.cand, Q.cand_count, cap, out_d2, best_d2);
   k_best_ij<<<256, 256, 0, st>>>(Q.cand, Q.cand_count, cap, out_d2, best_d2, best_ij);

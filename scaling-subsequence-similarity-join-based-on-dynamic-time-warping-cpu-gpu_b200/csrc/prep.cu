@@ -150,14 +150,16 @@ __global__ void k_diffs(DevSeries S) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= S.s) return;
   if (i == S.s - 1) {
-    S.dfa[i] = S.dga[i] = S.dfE[i] = S.dgE[i] = 0.0;
+    S.dfa[i] = S.dga[i] = 0.0;
+    if (S.E) S.dfE[i] = S.dgE[i] = 0.0;
     return;
   }
   const int m = S.m;
   const double a0 = S.a[i], a1 = S.a[i + m];
-  const double e0 = S.E[i], e1 = S.E[i + m];
   S.dfa[i] = 0.5 * (a1 - a0);
   S.dga[i] = (a1 - S.mu[i + 1]) + (a0 - S.mu[i]);
+  if (!S.E) return;
+  const double e0 = S.E[i], e1 = S.E[i + m];
   S.dfE[i] = 0.5 * (e1 - e0);
   S.dgE[i] = (e1 - S.nu[i + 1]) + (e0 - S.nu[i]);
 }
@@ -343,6 +345,11 @@ void launch_prep(const DevSeries& S, cudaStream_t st) {
 
 void launch_stats(const DevSeries& S, cudaStream_t st) {
   k_stats<<<grid_for(S.s), kThreads, 0, st>>>(S);
+}
+
+int launch_diffs(const DevSeries& S, cudaStream_t st) {
+  k_diffs<<<grid_for(S.s), kThreads, 0, st>>>(S);
+  return 1;
 }
 
 int mask_table_max(int m) {
