@@ -136,7 +136,7 @@ struct Next {
 };
 
 __device__ __forceinline__ Next fetch(const DevSeries& S, const DevSearch& Q, const int2* pairs,
-                                      unsigned int total, int lane) {
+                                      unsigned int total, bool table, int lane) {
   Next nx;
   unsigned int idx = 0;
   if (lane == 0) idx = atomicAdd(Q.queue_next, 1u);
@@ -150,10 +150,12 @@ __device__ __forceinline__ Next fetch(const DevSeries& S, const DevSearch& Q, co
     nx.j = p.y;
     if (p.x >= 0) {  // else taken out of the queue by LB_Petitjean
       nx.sr = Q.qser ? Q.qser[idx] : series_of(S, p.x);
-      nx.mi = S.mu[p.x];
-      nx.si = S.isg[p.x];
-      nx.mj = S.mu[p.y];
-      nx.sj = S.isg[p.y];
+      if (!table) {
+        nx.mi = S.mu[p.x];
+        nx.si = S.isg[p.x];
+        nx.mj = S.mu[p.y];
+        nx.sj = S.isg[p.y];
+      }
     }
   }
   return nx;
@@ -182,25 +184,27 @@ __device__ __forceinline__ float prepare_pair(const DevSeries& S, const Next& nx
         const float4 b = *reinterpret_cast<const float4*>(zj + k);
         const float4 u = *reinterpret_cast<const float4*>(uj + k);
         const float4 l = *reinterpret_cast<const float4*>(lj + k);
-        const float d0 = max3f(a.x - u.x, l.x - a.x, 0.0f), d1 = max3f(a.y - u.y, l.y - a.y, 0.0f);
-        const float d2 = max3f(a.z - u.z, l.z - a.z, 0.0f), d3 = max3f(a.w - u.w, l.w - a.w, 0.0f);
-        if (k >= kBias && k + 4 <= m - kBias) {
+        if (k + 4 <= m) {
           *reinterpret_cast<float4*>(q + k) = a;
           *reinterpret_cast<float4*>(t + k) = b;
-          sum = d0 * d0 + d1 * d1 + (d2 * d2 + d3 * d3);
-        } else {
-          // the window's ends: no terms there, and nothing past the last sample
-          const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-          const float dv[4] = {d0, d1, d2, d3};
+        } else {  // nothing past the last sample
+          const float av[3] = {a.x, a.y, a.z}, bv[3] = {b.x, b.y, b.z};
 #pragma unroll
-          for (int x = 0; x < 4; ++x) {
+          for (int x = 0; x < 3; ++x)
             if (k + x < m) {
               q[k + x] = av[x];
               t[k + x] = bv[x];
             }
-            if (k + x >= kBias && k + x < m - kBias) sum += dv[x] * dv[x];
-          }
         }
+        // no terms at the window's ends: kBias = 3 samples there
+        const int e = m - kBias - k;
+        float d0 = max3f(a.x - u.x, l.x - a.x, 0.0f), d1 = max3f(a.y - u.y, l.y - a.y, 0.0f);
+        float d2 = max3f(a.z - u.z, l.z - a.z, 0.0f), d3 = max3f(a.w - u.w, l.w - a.w, 0.0f);
+        d0 = k > 0 && e > 0 ? d0 : 0.0f;
+        d1 = k > 0 && e > 1 ? d1 : 0.0f;
+        d2 = k > 0 && e > 2 ? d2 : 0.0f;
+        d3 = e > 3 ? d3 : 0.0f;
+        sum = fmaf(d0, d0, fmaf(d1, d1, fmaf(d2, d2, d3 * d3)));
       }
       sum += __shfl_xor_sync(0xffffffffu, sum, 1);
       if ((lane & 1) == 0 && k < m) cbc[k >> 3] = sum;
@@ -277,7 +281,8 @@ __global__ void __launch_bounds__(256, slot_blocks(C, G)) k_dtw_slots(DevSeries 
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int NS = 32 / G;
   constexpr unsigned int kGroup = 0xffffffffu >> (32 - G);  // a slot's lanes
-  constexpr int kIters = (16 + 2 * C - 1) / (2 * C);  // iterations between abandon checks
+  // iterations between abandon checks: every 10 to 18 steps
+  constexpr int kIters = C >= 5 ? 1 : (C == 4 ? 2 : (C == 3 ? 3 : 4));
   const int m = S.m, w = S.w;
   const int lane = threadIdx.x & 31, slot = lane / G, g = lane & (G - 1);
   const float INF = __int_as_float(0x7f800000);
@@ -310,7 +315,7 @@ __global__ void __launch_bounds__(256, slot_blocks(C, G)) k_dtw_slots(DevSeries 
   const unsigned int total = *npairs < Q.queue_cap ? *npairs : Q.queue_cap;
   const bool table = S.zt && *S.zready != 0u;
   unsigned int ncalls = 0, nabandoned = 0, nkeogh = 0;
-  unsigned long long ncells = 0;
+  unsigned long long cells = 0;  // of this lane
   // the slot's pair
   bool active = false;
   int pi = 0, pj = 0, sr = 0, tau = 0, iter = 0;
@@ -318,14 +323,14 @@ __global__ void __launch_bounds__(256, slot_blocks(C, G)) k_dtw_slots(DevSeries 
   const float* tb = t;
   const float* qb = past_q;
   const int qstep = past ? 0 : 2 * C;
-  Next nx = fetch(S, Q, pairs, total, lane);
+  unsigned int idle = 0xffffffffu;  // lanes of the slots without a pair
+  Next nx = fetch(S, Q, pairs, total, table, lane);
   for (;;) {
-    unsigned int idle = __ballot_sync(0xffffffffu, !active);
     while (idle && nx.have) {
       const int s = (__ffs(idle) - 1) / G;
       float* sb = warp_base + (size_t)s * lay.total;
       const Next cur = nx;
-      nx = fetch(S, Q, pairs, total, lane);
+      nx = fetch(S, Q, pairs, total, table, lane);
       if (cur.i < 0) continue;
       const float now =
           __shfl_sync(0xffffffffu, prune_threshold_now(Q.bsf2 + cur.sr, m), 0);
@@ -377,7 +382,7 @@ __global__ void __launch_bounds__(256, slot_blocks(C, G)) k_dtw_slots(DevSeries 
     }
     const bool done = active && tau > tau_end;
     bool over = false;
-    if (++iter == kIters) {  // about every 16 steps
+    if (kIters == 1 || ++iter == kIters) {
       iter = 0;
       thr = fminf(thr, prune_threshold(bsf, m));
       float fm = A[0];
@@ -389,26 +394,27 @@ __global__ void __launch_bounds__(256, slot_blocks(C, G)) k_dtw_slots(DevSeries 
     }
     const unsigned int ob = __ballot_sync(0xffffffffu, over) >> (slot * G);
     const bool ab = active && !done && (ob & kGroup) == kGroup;
-    if (__any_sync(0xffffffffu, done || ab)) {
+    const unsigned int ended = __ballot_sync(0xffffffffu, done || ab);
+    if (ended) {
       float d2 = INF;
+      if (__any_sync(0xffffffffu, done)) {
 #pragma unroll
-      for (int c = 0; c < C; ++c)
-        if (c == c0) d2 = A[c];
-      d2 = __shfl_sync(0xffffffffu, d2, g0, G);
-      // cells swept: rows [0, rows) of each diagonal the lane owns
-      const int rows = tau - g < 0 ? 0 : (tau - g > m ? m : tau - g);
-      unsigned int cnt = 0;
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        const int d = d_lo + c;
-        const int lo = d < 0 ? -d : 0, hi = rows < m - d ? rows : m - d;
-        if (d <= w && hi > lo) cnt += (unsigned int)(hi - lo);
+        for (int c = 0; c < C; ++c)
+          if (c == c0) d2 = A[c];
+        d2 = __shfl_sync(0xffffffffu, d2, g0, G);
       }
+      if (done || ab) {
+        // cells swept: rows [0, rows) of each diagonal the lane owns
+        const int rows = tau - g < 0 ? 0 : (tau - g > m ? m : tau - g);
 #pragma unroll
-      for (int o = G / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+        for (int c = 0; c < C; ++c) {
+          const int d = d_lo + c;
+          const int lo = d < 0 ? -d : 0, hi = rows < m - d ? rows : m - d;
+          if (d <= w && hi > lo) cells += (unsigned int)(hi - lo);
+        }
+      }
       if ((done || ab) && g == 0) {
         ++ncalls;
-        ncells += cnt;
         if (ab) {
           ++nabandoned;
         } else if (d2 <= prune_threshold_now(Q.bsf2 + sr, m)) {
@@ -430,6 +436,7 @@ __global__ void __launch_bounds__(256, slot_blocks(C, G)) k_dtw_slots(DevSeries 
         tb = t;
         qb = past_q;
       }
+      idle |= ended;
     }
   }
   unsigned long long nc = ncalls, na = nabandoned, nk = nkeogh;
@@ -437,13 +444,13 @@ __global__ void __launch_bounds__(256, slot_blocks(C, G)) k_dtw_slots(DevSeries 
     nc += __shfl_xor_sync(0xffffffffu, nc, o);
     na += __shfl_xor_sync(0xffffffffu, na, o);
     nk += __shfl_xor_sync(0xffffffffu, nk, o);
-    ncells += __shfl_xor_sync(0xffffffffu, ncells, o);
+    cells += __shfl_xor_sync(0xffffffffu, cells, o);
   }
   if (lane == 0) {
     if (nc) atomicAdd(&Q.counters[kDtwCalls], nc);
     if (na) atomicAdd(&Q.counters[kDtwAbandoned], na);
     if (nk) atomicAdd(&Q.counters[kPrunedKeogh], nk);
-    if (ncells) atomicAdd(&Q.counters[kDtwCells], ncells);
+    if (cells) atomicAdd(&Q.counters[kDtwCells], cells);
   }
 }
 
