@@ -113,12 +113,18 @@ __device__ __forceinline__ unsigned int append_slot(bool on, int lane, unsigned 
 }
 
 // First level, super-groups of kGrpFan g windows: one warp takes kSupRows
-// consecutive row groups I; lane l takes the column group J = I + L0 / G1 + l
-// (+ 32 w), the groups that hold lags of the tile.  The records of a slot are
-// consecutive in memory: the J loads are coalesced and overlap from row to
-// row, the I loads are broadcasts.  The slots are in an order that spreads
-// the first ones over the window; the warp votes every four.
-constexpr int kSupRows = 4;
+// consecutive row groups against kSupCols column groups, which hold the
+// groups with lags of the tile; a lane takes 2 rows and every eighth column.
+// The slots are in an order that spreads the first ones over the window; the
+// warp votes every four.
+//
+// A record is 16 bytes per lane, and a load returns 128 bytes per clock to an
+// SM's registers whatever the lanes share, so a lane's 2 x 5 group pairs take
+// 28 clocks of loads for 20 of arithmetic, where one row per load and lane
+// took 32 for 8: 139 -> 80 us per chunk of 1776 tiles at m = 1024.
+constexpr int kSupRows = 8;
+constexpr int kSupLaneCols = 5;
+constexpr int kSupCols = 8 * kSupLaneCols;
 template <bool ED>
 __global__ void __launch_bounds__(kThreads) k_group_super(DevSeries S, DevSearch Q, GroupFilter F,
                                                           const Tile* tiles, unsigned int total) {
@@ -129,87 +135,125 @@ __global__ void __launch_bounds__(kThreads) k_group_super(DevSeries S, DevSearch
   const unsigned int tk = item / per, rem = item - tk * per;
   const Tile T = tiles[tk];
   const int g = kGrpFan * S.grp_g;
-  const int row0 = (int)(rem / (unsigned)F.nw) * kSupRows;   // relative to the tile's first
-  const int col = (int)(rem % (unsigned)F.nw) * 32 + lane;   // relative to I + L0 / g
-  const int I0 = T.i0 / g + row0;
-  const int last_row = T.i0 + T.rows - 1;
-  if ((int64_t)I0 * g > last_row) return;
-  const int J0 = I0 + T.L0 / g + col;
+  const int row0 = (int)(rem / (unsigned)F.nw) * kSupRows + 2 * (lane >> 3);  // of this lane
+  const int Ia = T.i0 / g, last_row = T.i0 + T.rows - 1;
+  if ((Ia + (int)(rem / (unsigned)F.nw) * kSupRows) * (int64_t)g > last_row) return;
+  const int I = Ia + row0;
+  const int J = I - 2 * (lane >> 3) + T.L0 / g + (int)(rem % (unsigned)F.nw) * kSupCols + (lane & 7);
+  // the pairs that hold pairs of the tile (group_pair_in_tile, the rows' part once)
   unsigned int alive = 0;
 #pragma unroll
-  for (int r = 0; r < kSupRows; ++r)
-    if (group_pair_in_tile(T, g, I0 + r, J0 + r)) alive |= 1u << r;
+  for (int r = 0; r < 2; ++r) {
+    const int ia = (I + r) * g;
+    const int lo = ia > T.i0 ? ia : T.i0, hi = ia + g - 1 < last_row ? ia + g - 1 : last_row;
+#pragma unroll
+    for (int q = 0; q < kSupLaneCols; ++q) {
+      const int ja = (J + 8 * q) * g;
+      if (lo <= hi && ja < T.send && ja + g - 1 - lo >= T.L0 && ja - hi < T.L0 + kLbLags)
+        alive |= 1u << (r * kSupLaneCols + q);
+    }
+  }
   if (!__any_sync(0xffffffffu, alive != 0u)) return;
   const float thr = ED ? *F.cut : prune_threshold_now(Q.bsf2 + T.series, S.m);
   const float fb = (float)S.grp_b;
   const int64_t n = S.sup_n;
   // addresses past the last record repeat it (those group pairs are not
-  // alive); the records run past the last row group by more than kSupRows
-  const float4* pi = S.sup + I0;
-  const float4* pj[kSupRows];
-  float a1[kSupRows], a2[kSupRows];
+  // alive); the records run past the last row group by kSupRows and more
+  const float4* pi = S.sup + I;
+  const float4* pj[kSupLaneCols];
+  float a1[2][kSupLaneCols], a2[2][kSupLaneCols];
 #pragma unroll
-  for (int r = 0; r < kSupRows; ++r) {
-    pj[r] = S.sup + (J0 + r < n ? J0 + r : n - 1);
-    a1[r] = a2[r] = 0.0f;
+  for (int q = 0; q < kSupLaneCols; ++q) {
+    pj[q] = S.sup + (J + 8 * q < n ? J + 8 * q : n - 1);
+    a1[0][q] = a1[1][q] = a2[0][q] = a2[1][q] = 0.0f;
   }
 #pragma unroll 1
   for (int s0 = 0; s0 < S.grp_d; s0 += 4) {
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
+      const float4 i0 = pi[0], i1 = pi[1];
+      pi += n;
 #pragma unroll
-      for (int r = 0; r < kSupRows; ++r) group_terms<ED>(pi[u * n + r], pj[r][u * n], a1[r], a2[r]);
+      for (int q = 0; q < kSupLaneCols; ++q) {
+        const float4 j = *pj[q];
+        pj[q] += n;
+        group_terms<ED>(i0, j, a1[0][q], a2[0][q]);
+        group_terms<ED>(i1, j, a1[1][q], a2[1][q]);
+      }
     }
-    pi += 4 * n;
 #pragma unroll
-    for (int r = 0; r < kSupRows; ++r) {
-      pj[r] += 4 * n;
-      if (fb * fmaxf(a1[r], a2[r]) > thr) alive &= ~(1u << r);
-    }
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int q = 0; q < kSupLaneCols; ++q)
+        if (fb * fmaxf(a1[r][q], a2[r][q]) > thr) alive &= ~(1u << (r * kSupLaneCols + q));
     if (!__any_sync(0xffffffffu, alive != 0u)) return;
   }
 #pragma unroll
-  for (int r = 0; r < kSupRows; ++r) {
-    const bool on = (alive >> r) & 1u;
-    const unsigned int slot = append_slot(on, lane, F.nsup);
-    if (on && slot < F.sup_cap) F.sup[slot] = group_code(tk, row0 + r, col);
-  }
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int q = 0; q < kSupLaneCols; ++q) {
+      const bool on = (alive >> (r * kSupLaneCols + q)) & 1u;
+      const unsigned int slot = append_slot(on, lane, F.nsup);
+      if (on && slot < F.sup_cap)
+        F.sup[slot] = group_code(tk, row0 + r, J + 8 * q - (I + r) - T.L0 / g);
+    }
 }
 
-// Second level: half a warp per surviving super-group pair, one lane per
-// pair of its kGrpFan x kGrpFan groups.
+// Second level: four lanes per surviving super-group pair, each 2 x 2 of its
+// kGrpFan x kGrpFan group pairs (four records for four pairs; one pair per
+// lane took two for one).
 template <bool ED>
 __global__ void __launch_bounds__(kThreads) k_group(DevSeries S, DevSearch Q, GroupFilter F,
                                                     const Tile* tiles) {
-  static_assert(kGrpFan == 4, "16 group pairs, half a warp");
-  const int lane = threadIdx.x & 31, h = lane & 15;
+  static_assert(kGrpFan == 4, "16 group pairs, four lanes");
+  const int lane = threadIdx.x & 31, ha = (lane >> 1) & 1, hb = lane & 1;
   const unsigned int total = *F.nsup < F.sup_cap ? *F.nsup : F.sup_cap;
   const int g = S.grp_g, G = kGrpFan * g;
   const float fb = (float)S.grp_b;
   const int64_t n = S.grp_n;
-  for (unsigned int e0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 2; e0 < total;
-       e0 += ((gridDim.x * blockDim.x) >> 5) * 2) {
-    const unsigned int e = e0 + (lane >> 4);
+  for (unsigned int e0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 8; e0 < total;
+       e0 += ((gridDim.x * blockDim.x) >> 5) * 8) {
+    const unsigned int e = e0 + (lane >> 2);
     const unsigned int code = F.sup[e < total ? e : total - 1];
     const unsigned int tk = group_code_tile(code);
     const Tile T = tiles[tk];
     const GroupPair p = group_code_pair(code, T, G);
-    const int I = p.I * kGrpFan + (h >> 2), J = p.J * kGrpFan + (h & 3);
-    bool alive = e < total && group_pair_in_tile(T, g, I, J);
-    const float thr = ED ? *F.cut : prune_threshold_now(Q.bsf2 + T.series, S.m);
-    const float4* pi = S.grp + (I < n ? I : n - 1);
-    const float4* pj = S.grp + (J < n ? J : n - 1);
-    float a1 = 0.0f, a2 = 0.0f;
-#pragma unroll 1
-    for (int s0 = 0; s0 < S.grp_d && __any_sync(0xffffffffu, alive); s0 += 4) {
+    const int I = p.I * kGrpFan + 2 * ha, J = p.J * kGrpFan + 2 * hb;
+    unsigned int alive = 0;  // bit 2 r + q: groups I + r, J + q
+    if (e < total) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) group_terms<ED>(pi[u * n], pj[u * n], a1, a2);
-      pi += 4 * n;
-      pj += 4 * n;
-      alive = alive && !(fb * fmaxf(a1, a2) > thr);
+      for (int x = 0; x < 4; ++x)
+        if (group_pair_in_tile(T, g, I + (x >> 1), J + (x & 1))) alive |= 1u << x;
     }
-    const unsigned int mask = (__ballot_sync(0xffffffffu, alive) >> (lane & 16)) & 0xffffu;
-    const bool on = h == 0 && mask != 0u;
+    const float thr = ED ? *F.cut : prune_threshold_now(Q.bsf2 + T.series, S.m);
+    // the records run past the last group by more than a super-group
+    const float4* pi = S.grp + (I < n - 1 ? I : n - 2);
+    const float4* pj = S.grp + (J < n - 1 ? J : n - 2);
+    float a1[4], a2[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) a1[x] = a2[x] = 0.0f;
+#pragma unroll 1
+    for (int s0 = 0; s0 < S.grp_d && __any_sync(0xffffffffu, alive != 0u); s0 += 4) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 i0 = pi[0], i1 = pi[1], j0 = pj[0], j1 = pj[1];
+        pi += n;
+        pj += n;
+        group_terms<ED>(i0, j0, a1[0], a2[0]);
+        group_terms<ED>(i0, j1, a1[1], a2[1]);
+        group_terms<ED>(i1, j0, a1[2], a2[2]);
+        group_terms<ED>(i1, j1, a1[3], a2[3]);
+      }
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        if (fb * fmaxf(a1[x], a2[x]) > thr) alive &= ~(1u << x);
+    }
+    // the 16 pairs of the super-group pair: row 2 ha + r, column 2 hb + q
+    unsigned int mask = ((alive & 3u) << (8 * ha + 2 * hb)) |
+                        ((alive >> 2 & 3u) << (8 * ha + 4 + 2 * hb));
+    mask |= __shfl_xor_sync(0xffffffffu, mask, 1);
+    mask |= __shfl_xor_sync(0xffffffffu, mask, 2);
+    const bool on = (lane & 3) == 0 && mask != 0u;
     const unsigned int slot = append_slot(on, lane, F.nlist);
     if (on && slot < F.list_cap) F.list[slot] = make_uint2(code, mask);
     if (on) atomicAdd(ED ? F.tcount : F.tcount + tk, (unsigned int)__popc(mask));
@@ -303,7 +347,7 @@ size_t group_items(int g, GroupFilter* F) {
   // one row group at most (kLbLags + G - 2) / G + 2 column groups
   const int G = kGrpFan * g, rows = kLbRows / G + 1, cols = (kLbLags + G - 2) / G + 2;
   F->nib = (rows + kSupRows - 1) / kSupRows;
-  F->nw = (cols + 31) / 32;
+  F->nw = (cols + kSupRows - 1 + kSupCols - 1) / kSupCols;
   return (size_t)rows * cols;
 }
 
