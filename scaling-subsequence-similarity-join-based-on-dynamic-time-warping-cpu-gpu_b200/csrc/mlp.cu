@@ -125,15 +125,34 @@ __device__ __forceinline__ void tc_load32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// Stages 128 (or N) rows x kTcK columns of op(r, k) into a K-major tile.
-template <typename Get>
-__device__ __forceinline__ void tc_stage(unsigned char* tile, int rows, int tid, const Get& get) {
+// Stages 128 (or N) rows x kTcK columns of op(r, k) = X[r * sr + k * sk] (zero
+// from row r_end and column k_end on) into a K-major tile; X points at (0, k0).
+// Rows contiguous in k take one 16-byte load per 8 elements; otherwise (the
+// transposed operands of the weight gradients) consecutive threads take
+// consecutive rows, so that the loads of a warp are contiguous.  A training
+// step's five GEMMs took 294 us with two-byte loads along k throughout.
+__device__ __forceinline__ void tc_stage(unsigned char* tile, int rows, int tid, const bf16* X,
+                                         int64_t sr, int64_t sk, int r_end, int k_end) {
+  const bf16 z = __float2bfloat16(0.0f);
+  if (sk == 1 && sr % 8 == 0 && k_end >= kTcK && (reinterpret_cast<uintptr_t>(X) & 15) == 0) {
+    for (int it = tid; it < rows * (kTcK / 8); it += 128) {
+      const int r = it / (kTcK / 8), kg = it % (kTcK / 8);
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (r < r_end) v = *reinterpret_cast<const uint4*>(X + r * sr + kg * 8);
+      *reinterpret_cast<uint4*>(tile + tc_offset(r, kg * 8)) = v;
+    }
+    return;
+  }
   for (int it = tid; it < rows * (kTcK / 8); it += 128) {
-    const int r = it / (kTcK / 8), kg = it % (kTcK / 8);
-    uint32_t v[4];
+    const int r = it % rows, kg = it / rows;
+    bf16 e[8];
 #pragma unroll
-    for (int h = 0; h < 4; ++h) v[h] = pack2(get(r, kg * 8 + 2 * h), get(r, kg * 8 + 2 * h + 1));
-    *reinterpret_cast<uint4*>(tile + tc_offset(r, kg * 8)) = make_uint4(v[0], v[1], v[2], v[3]);
+    for (int h = 0; h < 8; ++h) {
+      const int k = kg * 8 + h;
+      e[h] = r < r_end && k < k_end ? X[r * sr + k * sk] : z;
+    }
+    *reinterpret_cast<uint4*>(tile + tc_offset(r, kg * 8)) =
+        make_uint4(pack2(e[0], e[1]), pack2(e[2], e[3]), pack2(e[4], e[5]), pack2(e[6], e[7]));
   }
 }
 
@@ -166,18 +185,12 @@ __global__ void __launch_bounds__(128) k_gemm_tc(int M, int N, int K, const bf16
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = sh.tmem;
   const uint32_t idesc = tc_idesc(kTcRows, N);
-  const bf16 z = __float2bfloat16(0.0f);
   uint32_t phase = 0;
   bool ok = true;
   for (int k0 = k_beg; k0 < k_end && ok; k0 += kTcK) {
-    tc_stage(reinterpret_cast<unsigned char*>(sh.a), kTcRows, tid, [&](int r, int k) {
-      const int m = m0 + r, kk = k0 + k;
-      return (m < M && kk < k_end) ? A[m * sam + kk * sak] : z;
-    });
-    tc_stage(reinterpret_cast<unsigned char*>(sh.b), N, tid, [&](int n, int k) {
-      const int kk = k0 + k;
-      return kk < k_end ? B[kk * sbk + n * sbn] : z;
-    });
+    tc_stage(reinterpret_cast<unsigned char*>(sh.a), kTcRows, tid, A + m0 * sam + k0 * sak, sam,
+             sak, M - m0, k_end - k0);
+    tc_stage(reinterpret_cast<unsigned char*>(sh.b), N, tid, B + k0 * sbk, sbn, sbk, N, k_end - k0);
     // the tiles written by ordinary stores become visible to the tensor cores
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
@@ -206,12 +219,23 @@ __global__ void __launch_bounds__(128) k_gemm_tc(int M, int N, int K, const bf16
     uint32_t v[32];
     if (ok) tc_load32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
     if (row < M) {
+      // four columns a time (a thread holds one row: single columns would
+      // touch a sector each); the MLP's C are 16-byte aligned, ldc a multiple of 4
       float* c = C + row * ldc + c0;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const float x = ok ? __uint_as_float(v[j]) : __int_as_float(0x7fc00000);
-        if (gridDim.y > 1) atomicAdd(c + j, x);  // split K: C was cleared or holds the sum
-        else c[j] = accumulate ? c[j] + x : x;
+      for (int j = 0; j < 32; j += 4) {
+        float4 x = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
+                               __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+        if (!ok) x.x = x.y = x.z = x.w = __int_as_float(0x7fc00000);
+        float4* c4 = reinterpret_cast<float4*>(c + j);
+        if (gridDim.y > 1) {
+          atomicAdd(c4, x);  // split K: C was cleared or holds the sum
+        } else if (accumulate) {
+          const float4 o = *c4;
+          *c4 = make_float4(o.x + x.x, o.y + x.y, o.z + x.z, o.w + x.w);
+        } else {
+          *c4 = x;
+        }
       }
     }
   }
@@ -244,12 +268,15 @@ __global__ void k_to_bf16(const float* __restrict__ x, bf16* __restrict__ y, int
     y[i] = __float2bfloat16(x[i]);
 }
 
-// H[r][c] = relu(H[r][c] + b[c]) over rows x cols.
+// H[r][c] = relu(H[r][c] + b[c]) over rows x cols; with Hb also its BF16 copy.
 __global__ void k_bias_relu(float* __restrict__ H, const float* __restrict__ b, int rows,
-                            int cols) {
+                            int cols, bf16* __restrict__ Hb) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)rows * cols;
-       i += (int64_t)gridDim.x * blockDim.x)
-    H[i] = fmaxf(H[i] + b[i % cols], 0.0f);
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const float h = fmaxf(H[i] + b[i % cols], 0.0f);
+    H[i] = h;
+    if (Hb) Hb[i] = __float2bfloat16(h);
+  }
 }
 
 // y[r] = H2[r] . w3 + b3; with targets: dy = 2 (y - t) / rows, loss += (y - t)^2 / rows.
@@ -273,46 +300,114 @@ __global__ void k_head(const float* __restrict__ H2, const float* __restrict__ w
   }
 }
 
-// dH2[r][c] = dy[r] w3[c] [H2[r][c] > 0]
-__global__ void k_dh2(const float* __restrict__ dy, const float* __restrict__ w3,
-                      const float* __restrict__ H2, float* __restrict__ dH2, int rows) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)rows * kHid;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = i / kHid;
-    const int c = (int)(i % kHid);
-    dH2[i] = H2[i] > 0.0f ? dy[r] * w3[c] : 0.0f;
-  }
-}
-
-// D[r][c] *= [H[r][c] > 0]
-__global__ void k_relu_grad(float* __restrict__ D, const float* __restrict__ H, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    if (!(H[i] > 0.0f)) D[i] = 0.0f;
-}
-
-// out[c] = sum_r X[r][c] * (v ? v[r] : 1), one thread per column.
-__global__ void k_colsum(const float* __restrict__ X, const float* __restrict__ v, int rows,
-                         int cols, float* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  double acc = 0.0;
-  for (int r = 0; r < rows; ++r) acc += (double)X[(int64_t)r * cols + c] * (v ? v[r] : 1.0f);
-  out[c] = (float)acc;
-}
-
-__global__ void k_sum(const float* __restrict__ v, int n, float* __restrict__ out) {
-  __shared__ float red[32];
-  float acc = 0.f;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) acc += v[i];
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+// Column sums over the batch in FP64, in two stages: a block (kSumLanes
+// threads per hidden unit) adds kSumRows rows, the last block to finish adds
+// the blocks' sums and writes them out, both in a fixed order, so the result
+// does not depend on the order the blocks run in.  One block per matrix walking
+// all 8,192 rows took 740 us, three times per training step.
+constexpr int kSumRows = 64, kSumLanes = 4;
+constexpr int kSumBlocks = kMaxBatch / kSumRows;
+struct ColSums {
+  double* part;          // [kSumBlocks][sets][kHid]
+  unsigned int* ticket;  // zero between launches
+};
+template <int SETS>
+__device__ void finish_sums(const ColSums& cs, const double (&acc)[SETS], float* const (&out)[SETS],
+                            const int (&count)[SETS]) {
+  const int c = threadIdx.x, l = threadIdx.y;
+  __shared__ double red[SETS][kSumLanes][kHid];
+  __shared__ bool last;
+#pragma unroll
+  for (int q = 0; q < SETS; ++q) red[q][l][c] = acc[q];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.f;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-    *out = t;
+  if (l == 0) {
+#pragma unroll
+    for (int q = 0; q < SETS; ++q)
+      cs.part[((size_t)blockIdx.x * SETS + q) * kHid + c] =
+          (red[q][0][c] + red[q][1][c]) + (red[q][2][c] + red[q][3][c]);
+    __threadfence();
   }
+  __syncthreads();
+  if (c == 0 && l == 0) last = atomicAdd(cs.ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+#pragma unroll
+  for (int q = 0; q < SETS; ++q) {
+    double t = 0.0;
+#pragma unroll 8
+    for (unsigned int k = l; k < gridDim.x; k += kSumLanes)
+      t += __ldcg(&cs.part[((size_t)k * SETS + q) * kHid + c]);
+    red[q][l][c] = t;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < SETS; ++q)
+    if (l == 0 && c < count[q])
+      out[q][c] = (float)((red[q][0][c] + red[q][1][c]) + (red[q][2][c] + red[q][3][c]));
+  if (c == 0 && l == 0) *cs.ticket = 0u;
+}
+
+// dH2[r][c] = dy[r] w3[c] [H2[r][c] > 0], as FP32 (dH2) or BF16 (dH2b), and the
+// gradients that are column sums: dw3 = H2^T dy, db2 = sum dH2, db3 = sum dy.
+__global__ void __launch_bounds__(kHid* kSumLanes) k_dh2(
+    const float* __restrict__ dy, const float* __restrict__ w3, const float* __restrict__ H2,
+    float* __restrict__ dH2, bf16* __restrict__ dH2b, int rows, ColSums cs, float* dw3, float* db2,
+    float* db3) {
+  const int c = threadIdx.x;
+  const float w = w3[c];
+  const int r0 = blockIdx.x * kSumRows + threadIdx.y;
+  double acc[3] = {0.0, 0.0, 0.0};
+  float h[kSumRows / kSumLanes], y[kSumRows / kSumLanes];
+#pragma unroll
+  for (int k = 0; k < kSumRows / kSumLanes; ++k) {
+    const int r = r0 + k * kSumLanes;
+    h[k] = r < rows ? H2[(int64_t)r * kHid + c] : 0.0f;
+    y[k] = r < rows ? dy[r] : 0.0f;
+  }
+#pragma unroll
+  for (int k = 0; k < kSumRows / kSumLanes; ++k) {
+    const int r = r0 + k * kSumLanes;
+    const float d = h[k] > 0.0f ? y[k] * w : 0.0f;
+    if (r < rows) {
+      if (dH2b) dH2b[(int64_t)r * kHid + c] = __float2bfloat16(d);
+      else dH2[(int64_t)r * kHid + c] = d;
+    }
+    acc[0] += (double)h[k] * y[k];
+    acc[1] += d;
+    acc[2] += y[k];
+  }
+  float* const out[3] = {dw3, db2, db3};
+  const int count[3] = {kHid, kHid, 1};
+  finish_sums<3>(cs, acc, out, count);
+}
+
+// dH1[r][c] = D[r][c] [H1[r][c] > 0], in place as FP32 or as BF16 (Db), and
+// db1 = sum dH1.
+__global__ void __launch_bounds__(kHid* kSumLanes) k_relu_grad(float* D, const float* __restrict__ H,
+                                                               bf16* __restrict__ Db, int rows,
+                                                               ColSums cs, float* db1) {
+  const int c = threadIdx.x;
+  const int r0 = blockIdx.x * kSumRows + threadIdx.y;
+  double acc[1] = {0.0};
+  float d[kSumRows / kSumLanes];
+#pragma unroll
+  for (int k = 0; k < kSumRows / kSumLanes; ++k) {
+    const int64_t i = (int64_t)(r0 + k * kSumLanes) * kHid + c;
+    d[k] = r0 + k * kSumLanes < rows && H[i] > 0.0f ? D[i] : 0.0f;
+  }
+#pragma unroll
+  for (int k = 0; k < kSumRows / kSumLanes; ++k) {
+    const int r = r0 + k * kSumLanes;
+    if (r < rows) {
+      if (Db) Db[(int64_t)r * kHid + c] = __float2bfloat16(d[k]);
+      else D[(int64_t)r * kHid + c] = d[k];
+    }
+    acc[0] += d[k];
+  }
+  float* const out[1] = {db1};
+  const int count[1] = {kHid};
+  finish_sums<1>(cs, acc, out, count);
 }
 
 // Adam (bias-corrected), then the BF16 copies of W1 and W2.
@@ -350,6 +445,8 @@ struct dtwj_mlp {
   float *X = nullptr, *T = nullptr, *H1 = nullptr, *H2 = nullptr, *Y = nullptr, *DY = nullptr,
         *DH1 = nullptr, *DH2 = nullptr, *loss = nullptr;
   bf16 *Xb = nullptr, *H1b = nullptr, *DH1b = nullptr, *DH2b = nullptr;
+  double* sums = nullptr;         // column sums of the blocks of a batch
+  unsigned int* ticket = nullptr;
   int* tc_status = nullptr;  // set when a tensor-core GEMM gave up waiting on its mbarrier
 };
 
@@ -375,7 +472,7 @@ void gemm(bool precise, int M, int N, int K, const void* A, int64_t sam, int64_t
     // their products into C, cleared first unless accumulating
     const int mblocks = (M + kTcRows - 1) / kTcRows;
     int ksplit = 1;
-    if (mblocks == 1 && K >= 1024) ksplit = K / 512 < 64 ? K / 512 : 64;
+    if (mblocks == 1 && K >= 1024) ksplit = K / 256 < 64 ? K / 256 : 64;
     if (ksplit > 1 && !acc) cudaMemsetAsync(C, 0, (size_t)M * ldc * sizeof(float), st);
     k_gemm_tc<<<dim3((unsigned)mblocks, (unsigned)ksplit), 128, kTcSmemBytes, st>>>(
         M, N, K, (const bf16*)A, sam, sak, (const bf16*)B, sbk, sbn, C, ldc, acc, status);
@@ -393,36 +490,35 @@ void pass(dtwj_mlp* net, int rows, bool train, bool precise) {
   if (!precise) k_to_bf16<<<grid_for((int64_t)rows * kIn), kThreads, 0, st>>>(net->X, net->Xb, (int64_t)rows * kIn);
   gemm(precise, rows, kHid, kIn, precise ? (const void*)net->X : net->Xb, kIn, 1,
        precise ? (const void*)(P + kOffW1) : net->W1b, 1, kIn, net->H1, kHid, false, net->tc_status, st);
-  k_bias_relu<<<gr, kThreads, 0, st>>>(net->H1, P + kOffB1, rows, kHid);
+  k_bias_relu<<<gr, kThreads, 0, st>>>(net->H1, P + kOffB1, rows, kHid,
+                                       precise ? nullptr : net->H1b);
   // H2 = relu(H1 W2^T + b2)
-  if (!precise) k_to_bf16<<<gr, kThreads, 0, st>>>(net->H1, net->H1b, (int64_t)rows * kHid);
   gemm(precise, rows, kHid, kHid, precise ? (const void*)net->H1 : net->H1b, kHid, 1,
        precise ? (const void*)(P + kOffW2) : net->W2b, 1, kHid, net->H2, kHid, false, net->tc_status, st);
-  k_bias_relu<<<gr, kThreads, 0, st>>>(net->H2, P + kOffB2, rows, kHid);
+  k_bias_relu<<<gr, kThreads, 0, st>>>(net->H2, P + kOffB2, rows, kHid, nullptr);
   if (train) cudaMemsetAsync(net->loss, 0, 4, st);
   k_head<<<grid_for((int64_t)rows * 32), kThreads, 0, st>>>(net->H2, P + kOffW3, P + kOffB3, rows,
                                                            net->Y, train ? net->T : nullptr,
                                                            net->DY, net->loss);
   if (!train) return;
   float* G = net->G;
-  // head: dw3 = H2^T dy, db3 = sum dy
-  k_colsum<<<1, kHid, 0, st>>>(net->H2, net->DY, rows, kHid, G + kOffW3);
-  k_sum<<<1, 256, 0, st>>>(net->DY, rows, G + kOffB3);
-  // dH2, dW2 = dH2^T H1 [128][128] (K = rows), db2
-  k_dh2<<<gr, kThreads, 0, st>>>(net->DY, P + kOffW3, net->H2, net->DH2, rows);
-  if (!precise) k_to_bf16<<<gr, kThreads, 0, st>>>(net->DH2, net->DH2b, (int64_t)rows * kHid);
+  const ColSums cs = {net->sums, net->ticket};
+  const unsigned nsum = (unsigned)((rows + kSumRows - 1) / kSumRows);
+  const dim3 sum_block(kHid, kSumLanes);
+  // dH2, and dw3 = H2^T dy, db2, db3 = sum dy; dW2 = dH2^T H1 [128][128] (K = rows)
+  k_dh2<<<nsum, sum_block, 0, st>>>(net->DY, P + kOffW3, net->H2, net->DH2,
+                               precise ? nullptr : net->DH2b, rows, cs, G + kOffW3, G + kOffB2,
+                               G + kOffB3);
   gemm(precise, kHid, kHid, rows, precise ? (const void*)net->DH2 : net->DH2b, 1, kHid,
        precise ? (const void*)net->H1 : net->H1b, kHid, 1, G + kOffW2, kHid, false, net->tc_status, st);
-  k_colsum<<<1, kHid, 0, st>>>(net->DH2, nullptr, rows, kHid, G + kOffB2);
   // dH1 = dH2 W2 . [H1 > 0]: A = dH2 [rows][128], B(k, n) = W2[k][n]
   gemm(precise, rows, kHid, kHid, precise ? (const void*)net->DH2 : net->DH2b, kHid, 1,
        precise ? (const void*)(P + kOffW2) : net->W2b, kHid, 1, net->DH1, kHid, false, net->tc_status, st);
-  k_relu_grad<<<gr, kThreads, 0, st>>>(net->DH1, net->H1, (int64_t)rows * kHid);
-  // dW1 = dH1^T X [128][64] (K = rows), db1
-  if (!precise) k_to_bf16<<<gr, kThreads, 0, st>>>(net->DH1, net->DH1b, (int64_t)rows * kHid);
+  // and db1; dW1 = dH1^T X [128][64] (K = rows)
+  k_relu_grad<<<nsum, sum_block, 0, st>>>(net->DH1, net->H1, precise ? nullptr : net->DH1b, rows, cs,
+                                     G + kOffB1);
   gemm(precise, kHid, kIn, rows, precise ? (const void*)net->DH1 : net->DH1b, 1, kHid,
        precise ? (const void*)net->X : net->Xb, kIn, 1, G + kOffW1, kIn, false, net->tc_status, st);
-  k_colsum<<<1, kHid, 0, st>>>(net->DH1, nullptr, rows, kHid, G + kOffB1);
 }
 
 // After the stream is synchronised: DTWJ_ERR_CUDA if a tensor-core GEMM gave
@@ -479,6 +575,8 @@ int dtwj_mlp_create(int device, uint64_t seed, dtwj_mlp** out) {
             dalloc(&net->DH1, B * kHid) && dalloc(&net->DH2, B * kHid) &&
             dalloc(&net->loss, 1) && dalloc(&net->Xb, B * kIn) && dalloc(&net->H1b, B * kHid) &&
             dalloc(&net->DH1b, B * kHid) && dalloc(&net->DH2b, B * kHid) &&
+            dalloc(&net->sums, (int64_t)kSumBlocks * 3 * kHid) && dalloc(&net->ticket, 1) &&
+            cudaMemset(net->ticket, 0, 4) == cudaSuccess &&
             dalloc(&net->tc_status, 1) && cudaMemset(net->tc_status, 0, 4) == cudaSuccess;
   if (!ok) {
     dtwj_mlp_destroy(net);
@@ -501,7 +599,7 @@ void dtwj_mlp_destroy(dtwj_mlp* net) {
   if (net->stream) cudaStreamSynchronize(net->stream);
   void* bufs[] = {net->P,  net->G,  net->M1, net->M2,  net->W1b, net->W2b, net->X,
                   net->T,  net->H1, net->H2, net->Y,   net->DY,  net->DH1, net->DH2,
-                  net->loss, net->Xb, net->H1b, net->DH1b, net->DH2b, net->tc_status};
+                  net->loss, net->Xb, net->H1b, net->DH1b, net->DH2b, net->sums, net->ticket, net->tc_status};
   for (void* b : bufs)
     if (b) cudaFree(b);
   if (net->stream) cudaStreamDestroy(net->stream);
