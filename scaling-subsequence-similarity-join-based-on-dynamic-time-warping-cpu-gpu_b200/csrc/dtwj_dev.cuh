@@ -375,23 +375,17 @@ void launch_mp(const DevSeries& S, const Tile* tiles, int ntiles, unsigned long 
 // bsf2[t] = an upper bound on tile t's smallest squared DTW (its ED^2 minimum).
 void launch_tile_bound(const unsigned int* tile_best, int ntiles, unsigned int* bsf2,
                        cudaStream_t st);
-// Full profile: lo = row minima of the reversed series (nullptr: upper only).
-void launch_mp_finalize(const DevSeries& S, const unsigned long long* up,
-                        const unsigned long long* lo, double* mp, int64_t* mpi,
-                        cudaStream_t st);
-void launch_reverse(const double* a, int64_t n, double* out, cudaStream_t st);
-// Exact profile: want / wrev = the smaller first-pass key of each row (by
-// series row / by reversed row); the collect pass lists every pair whose high
-// word is near its row's key; the exact pass computes their FP64 distance
-// (pick = false: row minima of the bits, true: lowest partner at the minimum;
-// reversed: the candidates are rows of the reversed series).
-void launch_mp_want(int64_t s, const unsigned long long* up, const unsigned long long* lo,
-                    unsigned long long* want, unsigned long long* wrev, cudaStream_t st);
-void launch_mp_collect(const DevSeries& S, const Tile* tiles, int ntiles,
-                       const unsigned long long* want, int2* cand, unsigned int* count,
-                       unsigned int cap, cudaStream_t st);
+// Matrix profile: best[i] = the smallest high word of ED^2 over window i's
+// partners on both sides (collect = false; best starts at 0xffffffff); then
+// (collect = true) the pairs near it, as (row, later partner) in up and (row,
+// earlier partner) in lo, count[2] how many there are.  The exact pass computes
+// the FP64 distance of such a list (pick = false: row minima of the bits, true:
+// lowest partner at the minimum).
+void launch_profile(const DevSeries& S, const Tile* tiles, int ntiles, bool collect,
+                    unsigned int* best, int2* up, int2* lo, unsigned int* count, unsigned int cap,
+                    cudaStream_t st);
 void launch_mp_exact(const DevSeries& S, const int2* cand, const unsigned int* count,
-                     unsigned int cap, bool reversed, bool pick, unsigned long long* rowmin,
+                     unsigned int cap, bool pick, unsigned long long* rowmin,
                      unsigned long long* rowidx, cudaStream_t st);
 void launch_mp_exact_out(int64_t s, const unsigned long long* rowmin,
                          const unsigned long long* rowidx, double* mp, int64_t* mpi,

@@ -185,8 +185,7 @@ struct dtwj_ctx {
 namespace {
 
 enum BufId {
-  B_A = 0, B_WORK, B_KEYS_UP, B_RESULT, B_PAIRS, B_OUT, B_MP, B_MPI, B_LBTILES, B_TILEBEST, B_FEAT, B_SCORE, B_MPX_WANT, B_MPX_WREV, B_MPX_MIN, B_MPX_IDX, B_MPX_CAND,
-  B_MPX_CNT, B_NOTES2, B_SORT, B_SORT_TEMP, B_LBTILES2,
+  B_A = 0, B_WORK, B_KEYS_UP, B_RESULT, B_PAIRS, B_OUT, B_LBTILES, B_TILEBEST, B_FEAT, B_SCORE, B_NOTES2, B_SORT, B_SORT_TEMP, B_LBTILES2,
   B_COUNT_
 };
 
@@ -1477,85 +1476,54 @@ int dtwj_matrix_profile(const double* x, int64_t n, int32_t m, double* mp, int64
   if (!mp || !mpi) return DTWJ_ERR_ARG;
   int rc = check_args(x, n, m, 0);
   if (rc) return rc;
-  // Row minima over partners j >= i + m come from the series, those over
-  // j <= i - m from the reversed series: reversing both windows keeps their
-  // z-normalised distance, and window i becomes window s-1-i.
   dtwj_ctx* ctx = nullptr;
-  dtwj_ctx* rev = nullptr;
   rc = dtwj_ctx_create(0, &ctx);
   if (rc) return rc;
-  rc = dtwj_ctx_create(0, &rev);
-  if (rc) {
-    dtwj_ctx_destroy(ctx);
-    return rc;
-  }
   do {
     double* dev = nullptr;
     if ((rc = upload(ctx, x, n, &dev))) break;
-    void* p;
-    if ((rc = ensure(rev, B_A, n * 8, &p))) break;
-    double* rdev = (double*)p;
-    launch_reverse(dev, n, rdev, ctx->stream);
-    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
-      rc = DTWJ_ERR_CUDA;
-      break;
-    }
-    DevSeries S, R;
-    PrepScratch P;
-    if ((rc = plan_and_prepare(ctx, dev, n, m, 0, false, kPrepProfile, &S, &P))) break;
-    if ((rc = plan_and_prepare(rev, rdev, n, m, 0, false, kPrepProfile, &R, &P))) break;
     build_lb_tiles(ctx, n, m, nullptr, 1);
     const int nlb = (int)ctx->lbtiles_host.size();
-    if ((rc = ensure(ctx, B_LBTILES, (size_t)nlb * sizeof(Tile), &p))) break;
-    Tile* tiles = (Tile*)p;
-    cudaMemcpy(tiles, ctx->lbtiles_host.data(), (size_t)nlb * sizeof(Tile), cudaMemcpyHostToDevice);
     const int64_t s = n - m + 1;
-    if ((rc = ensure(ctx, B_KEYS_UP, s * 8, &p))) break;
-    unsigned long long* up = (unsigned long long*)p;
-    if ((rc = ensure(rev, B_KEYS_UP, s * 8, &p))) break;
-    unsigned long long* lo = (unsigned long long*)p;
-    launch_mp(S, tiles, nlb, up, ctx->stream);
-    launch_mp(R, tiles, nlb, lo, rev->stream);
-    if (cudaStreamSynchronize(rev->stream) != cudaSuccess) {
-      rc = DTWJ_ERR_CUDA;
-      break;
-    }
-    if ((rc = ensure(ctx, B_MP, s * 8, &p))) break;
-    double* dmp = (double*)p;
-    if ((rc = ensure(ctx, B_MPI, s * 8, &p))) break;
-    int64_t* dmpi = (int64_t*)p;
-    // Exact pass.  The first pass keeps about 17 mantissa bits of ED^2 per
-    // row; every pair whose key lies within ten 20-bit units of its row's
-    // smallest key (either direction) is a candidate, its FP64 distance is
-    // computed directly, and the row takes the smallest, lowest partner on
-    // ties.
-    unsigned long long *want, *wrev, *rowmin, *rowidx;
-    if ((rc = ensure(ctx, B_MPX_WANT, s * 8, &p))) break;
-    want = (unsigned long long*)p;
-    if ((rc = ensure(ctx, B_MPX_WREV, s * 8, &p))) break;
-    wrev = (unsigned long long*)p;
-    if ((rc = ensure(ctx, B_MPX_MIN, s * 8, &p))) break;
-    rowmin = (unsigned long long*)p;
-    if ((rc = ensure(ctx, B_MPX_IDX, s * 8, &p))) break;
-    rowidx = (unsigned long long*)p;
     const unsigned int cap =
         (unsigned int)(s * 16 + 4096 < (1ll << 31) ? s * 16 + 4096 : (1ll << 31));
-    if ((rc = ensure(ctx, B_MPX_CAND, (size_t)cap * sizeof(int2), &p))) break;
-    int2* cand_up = (int2*)p;
-    if ((rc = ensure(rev, B_MPX_CAND, (size_t)cap * sizeof(int2), &p))) break;
-    int2* cand_lo = (int2*)p;
-    if ((rc = ensure(ctx, B_MPX_CNT, 8, &p))) break;
-    unsigned int* cnt = (unsigned int*)p;
+    DevSeries S;
+    PrepScratch P;
+    Tile* tiles;
+    double* dmp;
+    int64_t* dmpi;
+    unsigned long long *rowmin, *rowidx;
+    unsigned int *best, *cnt;
+    int2 *cand_up, *cand_lo;
+    Arena A;
+    plan_series(A, dev, n, m, 0, false, kPrepProfile, nullptr, 1, &S, &P);
+    A.add(&tiles, (size_t)nlb * sizeof(Tile));
+    A.add(&dmp, s * 8);
+    A.add(&dmpi, s * 8);
+    A.add(&rowmin, s * 8);
+    A.add(&rowidx, s * 8);
+    A.add(&best, s * 4);
+    A.add(&cnt, 8);
+    A.add(&cand_up, (size_t)cap * sizeof(int2));
+    A.add(&cand_lo, (size_t)cap * sizeof(int2));
+    if ((rc = A.place(ctx, B_WORK))) break;
+    if ((rc = prepare(ctx, S, P))) break;
     cudaStream_t st = ctx->stream;
-    launch_mp_want(s, up, lo, want, wrev, st);
+    cudaMemcpyAsync(tiles, ctx->lbtiles_host.data(), (size_t)nlb * sizeof(Tile),
+                    cudaMemcpyHostToDevice, st);
+    cudaMemsetAsync(best, 0xff, s * 4, st);
     cudaMemsetAsync(cnt, 0, 8, st);
     cudaMemsetAsync(rowmin, 0xff, s * 8, st);
     cudaMemsetAsync(rowidx, 0xff, s * 8, st);
-    launch_mp_collect(S, tiles, nlb, want, cand_up, cnt, cap, st);
-    launch_mp_collect(R, tiles, nlb, wrev, cand_lo, cnt + 1, cap, st);
+    // The first walk keeps the high word of ED^2 per window; every pair within
+    // ten units of it for either of its windows is a candidate, its FP64
+    // distance is computed directly, and the row takes the smallest, lowest
+    // partner on ties.
+    launch_profile(S, tiles, nlb, false, best, nullptr, nullptr, nullptr, 0, st);
+    launch_profile(S, tiles, nlb, true, best, cand_up, cand_lo, cnt, cap, st);
     for (int pick = 0; pick < 2; ++pick) {
-      launch_mp_exact(S, cand_up, cnt, cap, false, pick != 0, rowmin, rowidx, st);
-      launch_mp_exact(S, cand_lo, cnt + 1, cap, true, pick != 0, rowmin, rowidx, st);
+      launch_mp_exact(S, cand_up, cnt, cap, pick != 0, rowmin, rowidx, st);
+      launch_mp_exact(S, cand_lo, cnt + 1, cap, pick != 0, rowmin, rowidx, st);
     }
     launch_mp_exact_out(s, rowmin, rowidx, dmp, dmpi, st);
     unsigned int cnt_h[2] = {0, 0};
@@ -1568,14 +1536,13 @@ int dtwj_matrix_profile(const double* x, int64_t n, int32_t m, double* mp, int64
       rc = DTWJ_ERR_OVERFLOW;
       break;
     }
-    if (cudaMemcpyAsync(mp, dmp, s * 8, cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
-        cudaMemcpyAsync(mpi, dmpi, s * 8, cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
-        cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+    if (cudaMemcpyAsync(mp, dmp, s * 8, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaMemcpyAsync(mpi, dmpi, s * 8, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess) {
       rc = DTWJ_ERR_CUDA;
       break;
     }
   } while (0);
-  dtwj_ctx_destroy(rev);
   dtwj_ctx_destroy(ctx);
   return rc;
 }

@@ -13,8 +13,8 @@
 // monotone for non-negative doubles; the lowest 3 bits give way to the lag
 // inside a thread's minimum) above the partner index, so a 64-bit atomicMin
 // keeps the nearest neighbour at that resolution.  That is all the seeds
-// need; the matrix profile (dtwj_matrix_profile) then decides every row at
-// FP64 among the partners whose key is near the row's (launch_mp_collect).
+// need; the matrix profile (dtwj_matrix_profile, k_profile below) decides every
+// row at FP64 among the partners whose key is near the row's.
 //
 // The seeds are the kSeeds smallest row minima, as in
 // CPU_version1/new_dtw_motifGUI.cpp:53-74 (min_v_k + exact DTW per seed).
@@ -44,24 +44,12 @@ static_assert(kLbPerThread <= 8, "the lag fits the key's 3 low bits");
 struct MpShared {
   double p1[kCols], p2[kCols], is[kCols], c2[kCols];
   double r1[kStage], r2[kStage], ci[kStage];
-  unsigned int lim[kStage];
   unsigned long long rowbest[kStage];  // row minima of the current stage
 };
 
-// Candidate list of the exact profile (COLLECT): every pair whose high word
-// is within ten units of its row's smallest key.
-struct MpCollect {
-  const unsigned long long* want;  // per row: the smallest key of the first pass
-  int2* cand;
-  unsigned int* count;
-  unsigned int cap;
-};
-
-template <bool COLLECT>
 __global__ void __launch_bounds__(kLbThreads, 4) k_mp(DevSeries S, const Tile* tiles,
                                                       unsigned long long* keys,
-                                                      unsigned int* tile_best, int tile_base,
-                                                      MpCollect col) {
+                                                      unsigned int* tile_best, int tile_base) {
   extern __shared__ __align__(16) unsigned char smraw[];
   MpShared& sh = *reinterpret_cast<MpShared*>(smraw);
   const Tile T = tiles[blockIdx.x];
@@ -99,8 +87,7 @@ __global__ void __launch_bounds__(kLbThreads, 4) k_mp(DevSeries S, const Tile* t
   for (int st = 0; st < T.rows; st += kStage) {
     const int64_t r0 = i0 + st, c0 = r0 + L0;
     __syncthreads();
-    if (!COLLECT)
-      for (int x = t; x < kStage; x += kLbThreads) sh.rowbest[x] = ULLONG_MAX;
+    for (int x = t; x < kStage; x += kLbThreads) sh.rowbest[x] = ULLONG_MAX;
     for (int x = t; x < kCols; x += kLbThreads) {
       const int64_t j = c0 + x;
       const bool in = j >= 0 && j < s, up = j >= 1 && j < s;  // update terms exist for j >= 1
@@ -115,12 +102,6 @@ __global__ void __launch_bounds__(kLbThreads, 4) k_mp(DevSeries S, const Tile* t
       sh.r1[x] = up ? S.dfa[i - 1] : 0.0;
       sh.r2[x] = up ? S.dga[i - 1] : 0.0;
       sh.ci[x] = (in && !S.flat[i]) ? -2.0 * S.isg[i] : 0.0;
-      if (COLLECT) {
-        // the first pass's key is the row's smallest high word with its 3
-        // low bits cleared: its partners lie within 8 units, plus 2 of margin
-        const unsigned long long k = in ? col.want[i] : ULLONG_MAX;
-        sh.lim[x] = k == ULLONG_MAX ? 0u : (unsigned int)(k >> 32) + 10u;
-      }
     }
     __syncthreads();
     const int cb = t * kLbPerThread;
@@ -138,7 +119,6 @@ __global__ void __launch_bounds__(kLbThreads, 4) k_mp(DevSeries S, const Tile* t
         const int64_t i = r0 + r;
         const bool first = (st == 0 && r == 0);
         const double q1 = sh.r1[r], q2 = sh.r2[r], qc = sh.ci[r];
-        const unsigned int lim = COLLECT ? sh.lim[r] : 0u;
         // rows of the tile with a non-flat window (warp-uniform); a column past
         // the series or flat has weight 0 and offset 1e300, so its key is far
         // above any real one and it never needs a test of its own
@@ -153,23 +133,16 @@ __global__ void __launch_bounds__(kLbThreads, 4) k_mp(DevSeries S, const Tile* t
           }
           const double e2 = fmax(fma(C[l] * qc, wi[sl], wc[sl]), 0.0);
           const unsigned int hi = (unsigned int)__double2hiint(e2);
-          if (COLLECT) {
-            if (row_ok && hi <= lim) {
-              const unsigned int slot = atomicAdd(col.count, 1u);
-              if (slot < col.cap) col.cand[slot] = make_int2((int)i, (int)(i + Lt + l));
-            }
-          } else {
-            // the high word with its lowest 3 bits replaced by the lag: one
-            // minimum keeps the nearest lag (17 mantissa bits of ED^2)
-            best = min(best, (hi & ~7u) | (unsigned int)l);
-          }
+          // the high word with its lowest 3 bits replaced by the lag: one
+          // minimum keeps the nearest lag (17 mantissa bits of ED^2)
+          best = min(best, (hi & ~7u) | (unsigned int)l);
         }
         const int nx = cb + r + kLbPerThread;
         w1[u] = sh.p1[nx];
         w2[u] = sh.p2[nx];
         wi[u] = sh.is[nx];
         wc[u] = sh.c2[nx];
-        if (!COLLECT && row_ok) {  // flat rows have no neighbour
+        if (row_ok) {  // flat rows have no neighbour
           const unsigned int wbest = __reduce_min_sync(0xffffffffu, best);
           if (wbest < kKeyReal) {
             const unsigned int ballot = __ballot_sync(0xffffffffu, best == wbest);
@@ -183,20 +156,17 @@ __global__ void __launch_bounds__(kLbThreads, 4) k_mp(DevSeries S, const Tile* t
         }
       }
     }
-    if (!COLLECT) {
-      // the stage's row minima into the series' keys (each row once per tile)
-      __syncthreads();
-      const int nrow = T.rows - st < kStage ? T.rows - st : kStage;
-      for (int x = t; x < nrow; x += kLbThreads) {
-        const unsigned long long v = sh.rowbest[x];
-        if (v != ULLONG_MAX) {
-          atomicMin(&keys[r0 + x], v);
-          tmin = min(tmin, (unsigned int)(v >> 32));
-        }
+    // the stage's row minima into the series' keys (each row once per tile)
+    __syncthreads();
+    const int nrow = T.rows - st < kStage ? T.rows - st : kStage;
+    for (int x = t; x < nrow; x += kLbThreads) {
+      const unsigned long long v = sh.rowbest[x];
+      if (v != ULLONG_MAX) {
+        atomicMin(&keys[r0 + x], v);
+        tmin = min(tmin, (unsigned int)(v >> 32));
       }
     }
   }
-  if (COLLECT) return;
   if (tile_best) {
     for (int o = 16; o > 0; o >>= 1) tmin = min(tmin, __shfl_xor_sync(0xffffffffu, tmin, o));
     if (lane == 0 && tmin != 0xffffffffu) atomicMin(&tile_best[tile_base + blockIdx.x], tmin);
@@ -416,52 +386,18 @@ __global__ void k_fill_u64(unsigned long long* p, int64_t n, unsigned long long 
     p[i] = v;
 }
 
-// Exact FP64 distance of each row's nearest neighbour.
-__global__ void k_mp_finalize(DevSeries S, const unsigned long long* up,
-                              const unsigned long long* lo, double* mp, int64_t* mpi) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= S.s) return;
-  unsigned long long k = up[i];
-  if (lo) {
-    // lo holds the row minima of the reversed series: row s-1-i, partner s-1-j
-    unsigned long long k2 = lo[S.s - 1 - i];
-    if (k2 != ULLONG_MAX)
-      k2 = (k2 & 0xffffffff00000000ull) |
-           (unsigned long long)(unsigned int)(S.s - 1 - (int64_t)(k2 & 0xffffffffu));
-    // tie on the distance key: lowest partner index
-    if ((k2 >> 32) < (k >> 32) || ((k2 >> 32) == (k >> 32) && (k2 & 0xffffffffu) < (k & 0xffffffffu)))
-      k = k2;
-  }
-  if (k == ULLONG_MAX) {
-    mp[i] = __longlong_as_double(0x7ff0000000000000LL);
-    mpi[i] = -1;
-    return;
-  }
-  const int64_t j = (int64_t)(k & 0xffffffffu);
-  const double mi = S.mu[i], mj = S.mu[j], si = S.isg[i], sj = S.isg[j];
-  double d2 = 0.0;
-  for (int q = 0; q < S.m; ++q) {
-    const double d = (S.a[i + q] - mi) * si - (S.a[j + q] - mj) * sj;
-    d2 = fma(d, d, d2);
-  }
-  mp[i] = sqrt(d2);
-  mpi[i] = j;
-}
-
-// Exact squared distance of candidate pairs, one warp per pair (the same
-// arithmetic as k_mp_finalize).  A candidate (i, j) of the reversed series is
-// the pair (s-1-i, s-1-j) of the series.  pick == false: rowmin[i] = the
+// Exact squared distance of candidate pairs (row, partner), one warp per pair.
+// pick == false: rowmin[i] = the
 // smallest FP64 bits over the row's candidates (non-negative doubles order as
 // their bits); pick == true: rowidx[i] = the lowest partner reaching it.
 __global__ void k_mp_exact(DevSeries S, const int2* cand, const unsigned int* count,
-                           unsigned int cap, bool reversed, bool pick,
-                           unsigned long long* rowmin, unsigned long long* rowidx) {
+                           unsigned int cap, bool pick, unsigned long long* rowmin, unsigned long long* rowidx) {
   const int lane = threadIdx.x & 31;
   const unsigned int total = *count < cap ? *count : cap;
   for (unsigned int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < total;
        c += (gridDim.x * blockDim.x) >> 5) {
     const int2 p = cand[c];
-    const int64_t i = reversed ? S.s - 1 - p.x : p.x, j = reversed ? S.s - 1 - p.y : p.y;
+    const int64_t i = p.x, j = p.y;
     const double mi = S.mu[i], mj = S.mu[j], si = S.isg[i], sj = S.isg[j];
     double d2 = 0.0;
     for (int q = lane; q < S.m; q += 32) {
@@ -491,19 +427,187 @@ __global__ void k_mp_exact_out(int64_t s, const unsigned long long* rowmin,
   mpi[i] = (int64_t)rowidx[i];
 }
 
-// want[i] = the smaller of row i's keys over j > i (up) and over j < i (lo,
-// rows of the reversed series); wrev is the same indexed by reversed rows.
-__global__ void k_mp_want(int64_t s, const unsigned long long* up, const unsigned long long* lo,
-                          unsigned long long* want, unsigned long long* wrev) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= s) return;
-  const unsigned long long a = up[i], b = lo[s - 1 - i];
-  const unsigned long long ha = a == ULLONG_MAX ? ULLONG_MAX : (a >> 32);
-  const unsigned long long hb = b == ULLONG_MAX ? ULLONG_MAX : (b >> 32);
-  const unsigned long long h = ha < hb ? ha : hb;
-  const unsigned long long k = h == ULLONG_MAX ? ULLONG_MAX : (h << 32);
-  want[i] = k;
-  wrev[s - 1 - i] = k;
+// The ED matrix profile (dtwj_matrix_profile): one walk over the upper triangle
+// keeps every window's smallest ED^2 as row and as column, a second one lists
+// the pairs near either window's smallest.  Walking only rows needed both
+// walks on the reversed series as well: 18.3 ms at 100,003 samples and m = 256.
+//
+// Tile, staging and recurrence are k_mp's.  A column passes through a thread's
+// kLbPerThread ring registers from its last lag to its first over as many
+// rows, so its minimum costs one integer minimum per pair and one shared
+// atomic per row and thread; the keys are the high words of ED^2.
+struct ProfShared {
+  double p1[kCols], p2[kCols], is[kCols], c2[kCols];
+  double r1[kStage], r2[kStage], ci[kStage];
+  unsigned int row[kStage], col[kCols];  // minima of the stage, or limits (COLLECT)
+};
+constexpr int kProfCtasPerSm = 4;  // launch bounds of k_profile
+struct ProfOut {
+  unsigned int* best;  // per window: smallest high word (also what COLLECT reads)
+  int2* up;            // (row, later partner) and (row, earlier partner) near the row's best
+  int2* lo;
+  unsigned int* count;  // [2]
+  unsigned int cap;
+};
+
+template <bool COLLECT>
+__global__ void __launch_bounds__(kLbThreads, kProfCtasPerSm) k_profile(DevSeries S,
+                                                                      const Tile* tiles, int part,
+                                                                      ProfOut out) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  ProfShared& sh = *reinterpret_cast<ProfShared*>(smraw);
+  Tile T = tiles[blockIdx.x];
+  {  // this block's stages of the tile
+    const int first = (int)blockIdx.y * part * kStage;
+    if (first >= T.rows) return;
+    T.i0 += first;
+    T.rows = T.rows - first < part * kStage ? T.rows - first : part * kStage;
+  }
+  const int64_t s = T.send;
+  const int m = S.m;
+  const int t = threadIdx.x, lane = t & 31;
+  const int64_t L0 = T.L0, i0 = T.i0;
+  const int64_t Lt = L0 + (int64_t)t * kLbPerThread;
+  const int cb = t * kLbPerThread;
+  // exact anchors C(i0, i0 + L) for the thread's lags, the samples staged
+  // kStage at a time
+  double C[kLbPerThread];
+  {
+    double mj[kLbPerThread];
+#pragma unroll
+    for (int l = 0; l < kLbPerThread; ++l) {
+      C[l] = 0.0;
+      mj[l] = S.mu[i0 + Lt + l < s ? i0 + Lt + l : s - 1];
+    }
+    const double mi = S.mu[i0];
+    for (int k0 = 0; k0 < m; k0 += kStage) {
+      const int cnt = m - k0 < kStage ? m - k0 : kStage;
+      __syncthreads();
+      for (int x = t; x < kCols; x += kLbThreads) {
+        const int64_t q = i0 + L0 + k0 + x;
+        sh.p1[x] = S.a[q < S.n ? q : S.n - 1];
+      }
+      for (int x = t; x < cnt; x += kLbThreads) sh.r1[x] = S.a[i0 + k0 + x] - mi;
+      __syncthreads();
+#pragma unroll 2
+      for (int k = 0; k < cnt; ++k) {
+        const double ai = sh.r1[k];
+#pragma unroll
+        for (int l = 0; l < kLbPerThread; ++l) C[l] = fma(ai, sh.p1[cb + k + l] - mj[l], C[l]);
+      }
+    }
+  }
+  double w1[kLbPerThread], w2[kLbPerThread], wi[kLbPerThread], wc[kLbPerThread];
+  unsigned int wm[kLbPerThread];  // the ring columns' minima, or limits
+  const double two_m = 2.0 * m;
+  for (int st = 0; st < T.rows; st += kStage) {
+    const int64_t r0 = i0 + st, c0 = r0 + L0;
+    __syncthreads();
+    for (int x = t; x < kCols; x += kLbThreads) {
+      const int64_t j = c0 + x;
+      const bool in = j < s, up = j >= 1 && in;  // update terms exist for j >= 1
+      sh.p1[x] = up ? S.dfa[j - 1] : 0.0;
+      sh.p2[x] = up ? S.dga[j - 1] : 0.0;
+      sh.is[x] = in ? S.isg[j] : 0.0;
+      // a column past the series or flat: no weight, an offset no pair reaches
+      sh.c2[x] = (in && !S.flat[j]) ? two_m : 1e300;
+      const unsigned int b = COLLECT && in ? out.best[j] : UINT_MAX;
+      // two high words are within two units of each other when their ED^2 are
+      // within 2^-19; ten units leave room for the recurrence's rounding
+      sh.col[x] = COLLECT ? (b == UINT_MAX ? 0u : b + 10u) : UINT_MAX;
+    }
+    for (int x = t; x < kStage; x += kLbThreads) {
+      const int64_t i = r0 + x;
+      const bool in = i < s, up = i >= 1 && in;
+      sh.r1[x] = up ? S.dfa[i - 1] : 0.0;
+      sh.r2[x] = up ? S.dga[i - 1] : 0.0;
+      sh.ci[x] = (in && !S.flat[i]) ? -2.0 * S.isg[i] : 0.0;
+      const unsigned int b = COLLECT && in ? out.best[i] : UINT_MAX;
+      sh.row[x] = COLLECT ? (b == UINT_MAX ? 0u : b + 10u) : UINT_MAX;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int l = 0; l < kLbPerThread; ++l) {
+      w1[l] = sh.p1[cb + l];
+      w2[l] = sh.p2[cb + l];
+      wi[l] = sh.is[cb + l];
+      wc[l] = sh.c2[cb + l];
+      wm[l] = COLLECT ? sh.col[cb + l] : UINT_MAX;
+    }
+    for (int qq = 0; qq < kStage / kLbPerThread; ++qq) {
+#pragma unroll
+      for (int u = 0; u < kLbPerThread; ++u) {
+        const int r = qq * kLbPerThread + u;
+        const int64_t i = r0 + r;
+        const double q1 = sh.r1[r], q2 = sh.r2[r], qc = sh.ci[r];
+        // rows of the tile with a non-flat window (warp-uniform)
+        const bool row_ok = (st + r < T.rows) && qc != 0.0;
+        if (st > 0 || r > 0) {
+#pragma unroll
+          for (int l = 0; l < kLbPerThread; ++l) {
+            const int sl = (u + l) % kLbPerThread;
+            C[l] = fma(q1, w2[sl], C[l]);
+            C[l] = fma(w1[sl], q2, C[l]);
+          }
+        }
+        if (row_ok) {
+          const unsigned int lim = COLLECT ? sh.row[r] : 0u;
+          unsigned int best = UINT_MAX, hs[kLbPerThread];
+          bool hit = false;  // one branch per row: candidates are rare
+#pragma unroll
+          for (int l = 0; l < kLbPerThread; ++l) {
+            const int sl = (u + l) % kLbPerThread;
+            // below zero only by rounding
+            const int h = __double2hiint(fma(C[l] * qc, wi[sl], wc[sl]));
+            const unsigned int hi = (unsigned int)max(h, 0);
+            if (COLLECT) {
+              hs[l] = hi;
+              hit = hit || hi <= max(lim, wm[sl]);
+            } else {
+              best = min(best, hi);
+              wm[sl] = min(wm[sl], hi);
+            }
+          }
+          if (COLLECT && hit) {
+#pragma unroll
+            for (int l = 0; l < kLbPerThread; ++l) {
+              const int j = (int)(i + Lt + l);
+              if (hs[l] <= lim) {
+                const unsigned int slot = atomicAdd(out.count, 1u);
+                if (slot < out.cap) out.up[slot] = make_int2((int)i, j);
+              }
+              if (hs[l] <= wm[(u + l) % kLbPerThread]) {
+                const unsigned int slot = atomicAdd(out.count + 1, 1u);
+                if (slot < out.cap) out.lo[slot] = make_int2(j, (int)i);
+              }
+            }
+          }
+          if (!COLLECT) {
+            best = __reduce_min_sync(0xffffffffu, best);
+            if (lane == 0) atomicMin(&sh.row[r], best);
+          }
+        }
+        // lag 0's column leaves the thread (a stage's last ones below)
+        const int nx = cb + r + kLbPerThread;
+        if (!COLLECT) atomicMin(&sh.col[nx - kLbPerThread], wm[u]);
+        w1[u] = sh.p1[nx];
+        w2[u] = sh.p2[nx];
+        wi[u] = sh.is[nx];
+        wc[u] = sh.c2[nx];
+        wm[u] = COLLECT ? sh.col[nx] : UINT_MAX;
+      }
+    }
+    if (!COLLECT) {
+      // ring slot l holds column kStage + l (kStage rows are whole turns)
+#pragma unroll
+      for (int l = 0; l < kLbPerThread; ++l) atomicMin(&sh.col[cb + kStage + l], wm[l]);
+      __syncthreads();
+      for (int x = t; x < kStage; x += kLbThreads)
+        if (sh.row[x] < kKeyReal) atomicMin(&out.best[r0 + x], sh.row[x]);
+      for (int x = t; x < kCols; x += kLbThreads)
+        if (sh.col[x] < kKeyReal) atomicMin(&out.best[c0 + x], sh.col[x]);
+    }
+  }
 }
 
 constexpr int kSelThreads = 1024;
@@ -611,17 +715,27 @@ __global__ void __launch_bounds__(kSelThreads) k_seed_select(DevSeries S,
   if (t == 0) nseeds[b] = taken;
 }
 
-__global__ void k_reverse(const double* a, int64_t n, double* out) {
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
-       p += (int64_t)gridDim.x * blockDim.x)
-    out[p] = a[n - 1 - p];
-}
-
 }  // namespace
 
-void launch_reverse(const double* a, int64_t n, double* out, cudaStream_t st) {
-  k_reverse<<<1024, 256, 0, st>>>(a, n, out);
+namespace {
+constexpr int kStages = kLbRows / kStage;
+// Stages of a tile per block: by the rounds of resident blocks and the work of
+// one, its anchors (m rows of 7 FP64 multiply-adds) and `part` stages of kStage
+// rows, a row costing row_cost anchor rows.
+int tile_part(int64_t ntiles, int m, int64_t resident, double row_cost) {
+  int part = kStages;
+  double best = 0.0;
+  for (int p = kStages; p >= 1; --p) {
+    const int64_t units = ntiles * ((kStages + p - 1) / p);
+    // fewer blocks than the GPU holds run faster, up to one per scheduler
+    const double rounds = units >= resident ? (double)((units + resident - 1) / resident)
+                                            : (units * 4 >= resident ? (double)units / resident : 0.25);
+    const double cost = rounds * ((double)m + row_cost * kStage * p);
+    if (p == kStages || cost < 0.95 * best) best = cost, part = p;
+  }
+  return part;
 }
+}  // namespace
 
 void launch_tile_bound(const unsigned int* tile_best, int ntiles, unsigned int* bsf2,
                        cudaStream_t st) {
@@ -632,13 +746,12 @@ void launch_mp(const DevSeries& S, const Tile* tiles, int ntiles, unsigned long 
                cudaStream_t st, unsigned int* tile_best) {
   k_fill_u64<<<1024, 256, 0, st>>>(keys, S.s, ULLONG_MAX);
   if (ntiles <= 0) return;
-  cudaFuncSetAttribute(k_mp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaFuncSetAttribute(k_mp, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(MpShared));
   const int slab = 1 << 20;
   for (int b = 0; b < ntiles; b += slab) {
     const int cnt = ntiles - b < slab ? ntiles - b : slab;
-    k_mp<false><<<cnt, kLbThreads, sizeof(MpShared), st>>>(S, tiles + b, keys, tile_best, b,
-                                                           MpCollect{});
+    k_mp<<<cnt, kLbThreads, sizeof(MpShared), st>>>(S, tiles + b, keys, tile_best, b);
   }
 }
 
@@ -648,21 +761,8 @@ void launch_mp_seed(const DevSeries& S, const Tile* tiles, int ntiles, unsigned 
   if (ntiles <= 0) return;
   cudaFuncSetAttribute(k_mp_seed, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(MpSeedShared));
-  // parts per tile by the rounds of resident blocks and the work of one:
-  // anchors (m rows of 7 FP64 multiply-adds) against `part` stages (kStage
-  // rows of 14 FP32 ones at twice the rate, and the keyed rows)
-  constexpr int kStages = kLbRows / kStage;
-  const int64_t resident = (int64_t)kSeedCtasPerSm * num_sms;
-  int part = kStages;
-  double best = 0.0;
-  for (int p = kStages; p >= 1; --p) {
-    const int64_t units = (int64_t)ntiles * ((kStages + p - 1) / p);
-    // fewer blocks than the GPU holds run faster, up to one per scheduler
-    const double rounds = units >= resident ? (double)((units + resident - 1) / resident)
-                                            : (units * 4 >= resident ? (double)units / resident : 0.25);
-    const double cost = rounds * ((double)S.m + 1.5 * kStage * p);
-    if (p == kStages || cost < 0.95 * best) best = cost, part = p;
-  }
+  // (FP32 stages: half the FP64 rate's cost per multiply-add, and the keyed rows)
+  const int part = tile_part(ntiles, S.m, kSeedCtasPerSm * num_sms, 1.5);
   const int parts = (kStages + part - 1) / part;
   const int slab = 1 << 20;
   for (int b = 0; b < ntiles; b += slab) {
@@ -672,41 +772,32 @@ void launch_mp_seed(const DevSeries& S, const Tile* tiles, int ntiles, unsigned 
   }
 }
 
-void launch_mp_collect(const DevSeries& S, const Tile* tiles, int ntiles,
-                       const unsigned long long* want, int2* cand, unsigned int* count,
-                       unsigned int cap, cudaStream_t st) {
-  if (ntiles <= 0) return;
-  cudaFuncSetAttribute(k_mp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(MpShared));
+void launch_profile(const DevSeries& S, const Tile* tiles, int ntiles, bool collect,
+                    unsigned int* best, int2* up, int2* lo, unsigned int* count, unsigned int cap,
+                    cudaStream_t st) {
+  auto kern = collect ? k_profile<true> : k_profile<false>;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ProfShared));
+  const ProfOut out = {best, up, lo, count, cap};
+  const int part = tile_part(ntiles, S.m, kProfCtasPerSm * 148, 4.0);
+  const unsigned parts = (unsigned)((kStages + part - 1) / part);
   const int slab = 1 << 20;
   for (int b = 0; b < ntiles; b += slab) {
     const int cnt = ntiles - b < slab ? ntiles - b : slab;
-    k_mp<true><<<cnt, kLbThreads, sizeof(MpShared), st>>>(S, tiles + b, nullptr, nullptr, b,
-                                                          MpCollect{want, cand, count, cap});
+    kern<<<dim3((unsigned)cnt, parts), kLbThreads, sizeof(ProfShared), st>>>(S, tiles + b, part,
+                                                                             out);
   }
 }
 
-void launch_mp_want(int64_t s, const unsigned long long* up, const unsigned long long* lo,
-                    unsigned long long* want, unsigned long long* wrev, cudaStream_t st) {
-  k_mp_want<<<(unsigned)((s + 255) / 256), 256, 0, st>>>(s, up, lo, want, wrev);
-}
-
 void launch_mp_exact(const DevSeries& S, const int2* cand, const unsigned int* count,
-                     unsigned int cap, bool reversed, bool pick, unsigned long long* rowmin,
+                     unsigned int cap, bool pick, unsigned long long* rowmin,
                      unsigned long long* rowidx, cudaStream_t st) {
-  k_mp_exact<<<148 * 8, 256, 0, st>>>(S, cand, count, cap, reversed, pick, rowmin, rowidx);
+  k_mp_exact<<<148 * 8, 256, 0, st>>>(S, cand, count, cap, pick, rowmin, rowidx);
 }
 
 void launch_mp_exact_out(int64_t s, const unsigned long long* rowmin,
                          const unsigned long long* rowidx, double* mp, int64_t* mpi,
                          cudaStream_t st) {
   k_mp_exact_out<<<(unsigned)((s + 255) / 256), 256, 0, st>>>(s, rowmin, rowidx, mp, mpi);
-}
-
-void launch_mp_finalize(const DevSeries& S, const unsigned long long* up,
-                        const unsigned long long* lo, double* mp, int64_t* mpi,
-                        cudaStream_t st) {
-  k_mp_finalize<<<(unsigned)((S.s + 255) / 256), 256, 0, st>>>(S, up, lo, mp, mpi);
 }
 
 void launch_seed_select(const DevSeries& S, const unsigned long long* keys, int2* seeds,
