@@ -385,7 +385,7 @@ void launch_tile_bound(const unsigned int* tile_best, int ntiles, unsigned int* 
 // lowest partner at the minimum).
 void launch_profile(const DevSeries& S, const Tile* tiles, int ntiles, bool collect,
                     unsigned int* best, int2* up, int2* lo, unsigned int* count, unsigned int cap,
-                    cudaStream_t st);
+                    int num_sms, cudaStream_t st);
 void launch_mp_exact(const DevSeries& S, const int2* cand, const unsigned int* count,
                      unsigned int cap, bool pick, unsigned long long* rowmin,
                      unsigned long long* rowidx, cudaStream_t st);

@@ -1519,8 +1519,10 @@ int dtwj_matrix_profile(const double* x, int64_t n, int32_t m, double* mp, int64
     // ten units of it for either of its windows is a candidate, its FP64
     // distance is computed directly, and the row takes the smallest, lowest
     // partner on ties.
-    launch_profile(S, tiles, nlb, false, best, nullptr, nullptr, nullptr, 0, st);
-    launch_profile(S, tiles, nlb, true, best, cand_up, cand_lo, cnt, cap, st);
+    launch_profile(S, tiles, nlb, false, best, nullptr, nullptr, nullptr, 0, ctx->num_sms,
+                   st);
+    launch_profile(S, tiles, nlb, true, best, cand_up, cand_lo, cnt, cap, ctx->num_sms,
+                   st);
     for (int pick = 0; pick < 2; ++pick) {
       launch_mp_exact(S, cand_up, cnt, cap, pick != 0, rowmin, rowidx, st);
       launch_mp_exact(S, cand_lo, cnt + 1, cap, pick != 0, rowmin, rowidx, st);

@@ -202,9 +202,9 @@ struct MpSeedShared {
 
 // A block takes `part` stages of a tile (blockIdx.x: tile, blockIdx.y: part of
 // it), all 18 when the tiles alone fill the GPU.  Each part starts from its
-// own exact anchors, so a tile is cut only as far as that pays: a series of
-// 20,000 samples has 74 tiles, and one block per tile walked 4,032 rows one
-// after another on half of the SMs (0.26 ms).
+// own exact anchors, so a tile is cut only as far as that pays (tile_part): a
+// series of 20,000 samples has 66 tiles, and one block per tile walks 4,032
+// rows one after another on half of the SMs (0.25 ms).
 __global__ void __launch_bounds__(kLbThreads, kSeedCtasPerSm) k_mp_seed(DevSeries S,
                                                                       const Tile* tiles, int part,
                                                                       unsigned long long* keys,
@@ -719,19 +719,25 @@ __global__ void __launch_bounds__(kSelThreads) k_seed_select(DevSeries S,
 
 namespace {
 constexpr int kStages = kLbRows / kStage;
-// Stages of a tile per block: by the rounds of resident blocks and the work of
-// one, its anchors (m rows of 7 FP64 multiply-adds) and `part` stages of kStage
-// rows, a row costing row_cost anchor rows.
-int tile_part(int64_t ntiles, int m, int64_t resident, double row_cost) {
+// Stages of a tile per block.  A block's time alone is its anchors (m rows) and
+// `part` stages of kStage rows, a row costing kRowCost anchor rows: 12 us per
+// stage and 8 us of anchors at m = 256, nearly all of it latency.  Blocks that
+// share an SM hide each other's, so r blocks per SM take 0.75 + r / 3 times
+// that (fits r = 1 .. 29 within 15 % for k_mp_seed, and k_profile's best parts
+// within 9 %).  Walks of k_mp_seed, against a rule that counted an SM as full
+// with four warps: 20,000 samples at m = 256 (66 tiles) 6 -> 2 stages, 110 ->
+// 70 us; 30,000 at m = 64 9 -> 1, 153 -> 107 us; 40,000 at m = 400 18 -> 3,
+// 298 -> 205 us.  dtwj_matrix_profile of 50,000 at m = 512 18 -> 6, 3.79 ->
+// 3.35 ms.
+constexpr double kRowCost = 1.75;
+int tile_part(int64_t ntiles, int m, int num_sms) {
   int part = kStages;
   double best = 0.0;
   for (int p = kStages; p >= 1; --p) {
-    const int64_t units = ntiles * ((kStages + p - 1) / p);
-    // fewer blocks than the GPU holds run faster, up to one per scheduler
-    const double rounds = units >= resident ? (double)((units + resident - 1) / resident)
-                                            : (units * 4 >= resident ? (double)units / resident : 0.25);
-    const double cost = rounds * ((double)m + row_cost * kStage * p);
-    if (p == kStages || cost < 0.95 * best) best = cost, part = p;
+    const double r = (double)(ntiles * ((kStages + p - 1) / p)) / num_sms;
+    const double load = 0.75 + r / 3.0;
+    const double cost = (load > 1.0 ? load : 1.0) * ((double)m + kRowCost * kStage * p);
+    if (p == kStages || cost < best) best = cost, part = p;
   }
   return part;
 }
@@ -761,8 +767,7 @@ void launch_mp_seed(const DevSeries& S, const Tile* tiles, int ntiles, unsigned 
   if (ntiles <= 0) return;
   cudaFuncSetAttribute(k_mp_seed, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(MpSeedShared));
-  // (FP32 stages: half the FP64 rate's cost per multiply-add, and the keyed rows)
-  const int part = tile_part(ntiles, S.m, kSeedCtasPerSm * num_sms, 1.5);
+  const int part = tile_part(ntiles, S.m, num_sms);
   const int parts = (kStages + part - 1) / part;
   const int slab = 1 << 20;
   for (int b = 0; b < ntiles; b += slab) {
@@ -774,11 +779,11 @@ void launch_mp_seed(const DevSeries& S, const Tile* tiles, int ntiles, unsigned 
 
 void launch_profile(const DevSeries& S, const Tile* tiles, int ntiles, bool collect,
                     unsigned int* best, int2* up, int2* lo, unsigned int* count, unsigned int cap,
-                    cudaStream_t st) {
+                    int num_sms, cudaStream_t st) {
   auto kern = collect ? k_profile<true> : k_profile<false>;
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ProfShared));
   const ProfOut out = {best, up, lo, count, cap};
-  const int part = tile_part(ntiles, S.m, kProfCtasPerSm * 148, 4.0);
+  const int part = tile_part(ntiles, S.m, num_sms);
   const unsigned parts = (unsigned)((kStages + part - 1) / part);
   const int slab = 1 << 20;
   for (int b = 0; b < ntiles; b += slab) {
