@@ -706,7 +706,8 @@ __global__ void __launch_bounds__(kSelThreads) k_seed_select(DevSeries S,
       // the pair and its diagonal neighbours that lie in the series
       for (int d = 0; d < kSeedSpread; ++d) {
         const int off = d - kSeedSpread / 2;
-        const bool ok = lo + off >= wb && hi + off < we;
+        // (a flat window has no z-normalisation: no pair of the join holds one)
+        const bool ok = lo + off >= wb && hi + off < we && !S.flat[lo + off] && !S.flat[hi + off];
         seeds[slot * kSeedSpread + d] = ok ? make_int2(lo + off, hi + off) : make_int2(-1, -1);
       }
     }
