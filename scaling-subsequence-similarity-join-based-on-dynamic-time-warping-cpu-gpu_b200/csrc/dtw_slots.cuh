@@ -388,7 +388,11 @@ __global__ void __launch_bounds__(256, slot_blocks(C, G)) k_dtw_slots(DevSeries 
       float fm = A[0];
 #pragma unroll
       for (int c = 1; c < C; ++c) fm = fminf(fm, A[c]);
-      int idx = tau - g + w;  // the row after this lane's latest, plus w
+      // The bound's terms belong to rows, and a path's last cell on the lanes'
+      // frontier lies on the latest row of its lane: rows fall by at most one
+      // per lane, so the path can only leave from there.  Every later row is
+      // still ahead, also those within w of it.
+      int idx = tau - g;
       idx = idx < 0 ? 0 : (idx + 7) >> 3;
       over = fm + cbc[idx < lay.nc ? idx : lay.nc] > thr;
     }

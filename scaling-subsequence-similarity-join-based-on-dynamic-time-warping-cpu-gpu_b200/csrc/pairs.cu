@@ -228,7 +228,7 @@ __device__ T dtw_band(const T* __restrict__ q, const T* __restrict__ t, int m, i
       T fm = A[0];
 #pragma unroll
       for (int c = 1; c < C; ++c) fm = fmin_(fm, A[c]);
-      int idx = r + w + 1;
+      int idx = r + 1;  // (the path leaves the lanes' frontier from its lane's latest row)
       idx = idx < 0 ? 0 : (idx + 7) >> 3;
       const float cbv = cbc[idx < nc ? idx : nc];
       thr = fminf(thr, prune_threshold_now(bsf2, m));
