@@ -418,23 +418,25 @@ def run_ours(args):
     e2e_wall = _max_over_ranks(time.perf_counter() - t1, dist, local)
 
     hbm_peak, peak_kind, sm_max = _peaks()
-    # Algorithmic DRAM bytes of the three sweep kernels over one join (the
-    # data each must move at least once; averaged per launch below):
-    #   k_lb    reads the six per-index FP64 operands of its rows and columns
-    #           ((2 rows + 896 lags) x 48 B per tile) and writes the survivor
-    #           bits (896 lags x 126 words x 4 B per tile)
-    #   k_paa   reads those bits and the 16-byte block means of the windows a
-    #           tile covers (rows + 896 lags + m samples per tile), and writes
-    #           one 16-byte LB_Keogh candidate per pair that passes the
-    #           block-mean and endpoint bounds (k_runs, the masked cascade's
-    #           filter, in its place under F_MASKED_CASCADE)
-    #   k_keogh reads the candidates and writes an 8-byte DTW entry per survivor
+    # Algorithmic DRAM bytes of the three sweep stages over one join (the data
+    # each must move at least once; averaged per launch below):
+    #   diag   the group bound (k_group_super, k_group) reads the records of a
+    #          tile's row and column groups (32 segments x 16 B per g windows,
+    #          g = 8 from m = 512 on, else 4 - see group.cu); tiles it leaves
+    #          dense go through k_lb, which reads six FP64 operands per row and
+    #          column (48 B each) and writes survivor bits.  Counted: the records
+    #   runs   k_paa_groups reads the 16-byte block means of the windows a tile
+    #          covers (rows + 896 lags + m samples) and writes one 16-byte
+    #          LB_Keogh candidate per pair that passes the block-mean and
+    #          endpoint bounds (k_paa_lags, k_paa on dense tiles; k_runs under
+    #          F_MASKED_CASCADE)
+    #   keogh  k_keogh reads the candidates and writes an 8-byte DTW entry per
+    #          survivor
     ntiles, rows_sum = sweep_tiles(n, m)
-    bits_bytes = ntiles * 896 * 126 * 4
     kq_entries = r0.pruned_keogh + r0.dtw_calls  # pairs that reached LB_Keogh (seeds aside)
     alg = {
-        "diag": ("k_lb", (2 * rows_sum + ntiles * 896) * 48 + bits_bytes),
-        "runs": ("k_paa", bits_bytes + 16 * (rows_sum + ntiles * (896 + m)) + 16 * kq_entries),
+        "diag": ("k_group", (2 * rows_sum + ntiles * 896) * 32 * 16 // (8 if m >= 512 else 4)),
+        "runs": ("k_paa_groups", 16 * (rows_sum + ntiles * (896 + m)) + 16 * kq_entries),
         "keogh": ("k_keogh", 16 * kq_entries + 8 * r0.dtw_calls),
     }
     sweep_phases = [p for p in ("runs", "keogh", "diag") if phases.get(p, 0) > 0]
@@ -444,11 +446,9 @@ def run_ours(args):
     per_launch_s = phases[roof_phase] / nl
     achieved_gbs = alg_bytes / max(phases[roof_phase], 1e-12) / 1e9
     traffic = None
-    if args.workload == "rw1m_motif" and kname in ("k_lb", "k_paa"):
+    if args.workload == "rw1m_motif" and kname in ("k_lb", "k_paa"):  # (what was captured)
         traffic = launch_traffic(os.path.join(ROOT, "profiles", "ncu_traffic_rw1m_motif.json"),
                                  kname, ntiles / nl)
-    fp64_flops = pairs_total * 12.0  # k_lb: 2 recurrences x 2 DFMA + 2 DFMA tests per pair
-    fp64_peak = 148 * 64 * 2 * sm_max * 1e6 / 1e12
     cells_per_s = r0.dtw_cells / max(phases.get("pairs", 1e-12) + phases.get("seeds", 0), 1e-12)
 
     cpu = None
@@ -503,11 +503,6 @@ def run_ours(args):
                      "peak_kind": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)",
                      "per_launch_ms": 1000 * per_launch_s,
                      "note": "issue-bound, not HBM-bound: see profiles/"},
-        "issue_roofline": {"pipe": "fp64", "kernel": "k_lb",
-                           "achieved": fp64_flops / max(phases["diag"], 1e-12) / 1e12,
-                           "peak": fp64_peak, "unit": "TFLOP/s",
-                           "frac": fp64_flops / max(phases["diag"], 1e-12) / 1e12 / fp64_peak,
-                           "peak_kind": "nominal 148 SM x 64 DFMA/clk x max clock"},
         "dominant_phase": dominant,
         "learned_order": learned,
         "cpu_baseline": cpu,

@@ -292,10 +292,11 @@ int dtwj_time_band(int device, int32_t m, int32_t w, int32_t C, int32_t G, int32
                    double* cells_per_s);
 int dtwj_ctx_set_band(dtwj_ctx* ctx, int32_t w, int32_t C, int32_t G);
 /* Further tunables of a context's joins (no counterpart in the reference):
- * the CTA size of the DTW kernel in warps (1, 2, 4 or 8; each warp is one
- * pair in the default layout) and the tiles per chunk of the diagonal sweep
- * (16 to 4096; a chunk's survivors share the queues).  0 restores a default
- * (4 warps, 1024 tiles).  The result never depends on them. */
+ * the CTA size of the DTW kernel in warps (1, 2, 4 or 8; a warp holds one pair
+ * or, for narrow bands, several) and the tiles per chunk of the sweep (16 to
+ * 4096; a chunk's survivors share the queues).  0 restores a default (2 warps,
+ * 4 where a pair takes a warp of the general kernel; 12 tiles per SM).  The
+ * result never depends on them. */
 int dtwj_ctx_set_tuning(dtwj_ctx* ctx, int32_t dtw_warps, int32_t chunk_tiles);
 
 /* Series files in the formats of the reference's loaders

@@ -185,7 +185,8 @@ struct dtwj_ctx {
 namespace {
 
 enum BufId {
-  B_A = 0, B_WORK, B_KEYS_UP, B_RESULT, B_PAIRS, B_OUT, B_LBTILES, B_TILEBEST, B_FEAT, B_SCORE, B_NOTES2, B_SORT, B_SORT_TEMP, B_LBTILES2,
+  B_A = 0, B_WORK, B_RESULT, B_PAIRS, B_OUT, B_LBTILES, B_TILEBEST, B_FEAT, B_SCORE, B_NOTES2,
+  B_SORT, B_SORT_TEMP, B_LBTILES2,
   B_COUNT_
 };
 
