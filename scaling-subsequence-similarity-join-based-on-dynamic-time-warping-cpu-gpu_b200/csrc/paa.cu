@@ -170,7 +170,10 @@ __global__ void k_window_scale(DevSeries S) {
 // Window records for pq2: the block offset (x_c - mu_i) isg_i of the copy
 // block holding window i (center x_c), FP64; isg_i as FP32; and the error
 // scale isg_i (cmax2 + |x_c - mu_i|) of the values the block-mean bound forms
-// for it (the rw of pq2).
+// for it (the rw of pq2).  A zero isg marks a flat window (k_paa_groups drops
+// its pairs), so the isg of a window whose deviation is past 2^149, which FP32
+// cannot hold, is the smallest FP32 value instead; its copies are infinite, its
+// error scale too, and no FP32 bound judges it.
 __global__ void k_window_rec(DevSeries S) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= S.s) return;
@@ -179,8 +182,9 @@ __global__ void k_window_rec(DevSeries S) {
   const double x = copy_center(S, c, b), mu = S.mu[i], is = S.isg[i];
   const double off = (x - mu) * is;
   const double r = ((double)S.cmax2[c * kCopyBlocks(S.n) + b] + fabs(x - mu)) * is * (1.0 + 1e-6);
+  const float fis = S.flat[i] ? 0.0f : fmaxf((float)is, __int_as_float(1));
   S.wrec[i] = make_float4(__int_as_float(__double2loint(off)), __int_as_float(__double2hiint(off)),
-                          (float)is, (float)r);
+                          fis, (float)r);
 }
 
 // Scaled block offset of window x at 1024-sample block b, FP64.
