@@ -155,6 +155,16 @@ __global__ void k_block_max2(DevSeries S) {
   if (threadIdx.x == 0) S.cmax2[blockIdx.x] = t;
 }
 
+// The error scale r of a window's FP32 bounds as FP32, infinite (no FP32 bound
+// judges the window) where the scale of its samples leaves FP32: below a
+// deviation of 2^-100 the copies lose bits to FP32's smallest exponent and the
+// reciprocal may overflow, which at a deviation of 2^-140 pruned pairs by
+// infinite differences; above 2^100 the same the other way round.
+__device__ __forceinline__ float error_scale(double r, double is) {
+  const bool held = is >= 0x1p-100 && is <= 0x1p100;
+  return held ? (float)r : __int_as_float(0x7f800000);
+}
+
 // rw[i] = isg_i * max over the blocks window i covers of (cmax[b] +
 // |cb[b] - mu_i|): bounds every z-like value the FP32 bounds form for it.
 __global__ void k_window_scale(DevSeries S) {
@@ -164,7 +174,7 @@ __global__ void k_window_scale(DevSeries S) {
   const int64_t b0 = i >> kBlkShift, b1 = (i + S.m - 1) >> kBlkShift;
   double r = 0.0;
   for (int64_t b = b0; b <= b1; ++b) r = fmax(r, (double)S.cmax[b] + fabs(S.cb[b] - mu));
-  S.rw[i] = (float)(r * S.isg[i] * (1.0 + 1e-6));
+  S.rw[i] = error_scale(r * S.isg[i] * (1.0 + 1e-6), S.isg[i]);
 }
 
 // Window records for pq2: the block offset (x_c - mu_i) isg_i of the copy
@@ -172,8 +182,7 @@ __global__ void k_window_scale(DevSeries S) {
 // scale isg_i (cmax2 + |x_c - mu_i|) of the values the block-mean bound forms
 // for it (the rw of pq2).  A zero isg marks a flat window (k_paa_groups drops
 // its pairs), so the isg of a window whose deviation is past 2^149, which FP32
-// cannot hold, is the smallest FP32 value instead; its copies are infinite, its
-// error scale too, and no FP32 bound judges it.
+// cannot hold, is the smallest FP32 value instead (its error scale is infinite).
 __global__ void k_window_rec(DevSeries S) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= S.s) return;
@@ -184,7 +193,7 @@ __global__ void k_window_rec(DevSeries S) {
   const double r = ((double)S.cmax2[c * kCopyBlocks(S.n) + b] + fabs(x - mu)) * is * (1.0 + 1e-6);
   const float fis = S.flat[i] ? 0.0f : fmaxf((float)is, __int_as_float(1));
   S.wrec[i] = make_float4(__int_as_float(__double2loint(off)), __int_as_float(__double2hiint(off)),
-                          fis, (float)r);
+                          fis, error_scale(r, is));
 }
 
 // Scaled block offset of window x at 1024-sample block b, FP64.

@@ -1,9 +1,10 @@
 """Joins do not depend on the units of the series: z-normalisation cancels a
 scale, and a power of two cancels exactly in FP64.  The FP32 copies and
 reciprocal deviations of the bounds do not hold every scale (2^149 and beyond:
-1 / deviation rounds to zero), so at both ends the join must still be
-the unscaled series' by the oracle: indices exact, distance within 1e-5
-relative (the tolerance of the join tests)."""
+1 / deviation rounds to zero; 2^-127 and below: the samples lose bits, then
+1 / deviation overflows), so at both ends the join must still be the unscaled
+series' by the oracle: indices exact, distance within 1e-5 relative (the
+tolerance of the join tests)."""
 import numpy as np
 import pytest
 
@@ -26,5 +27,19 @@ def test_join_of_large_values(gpu_dtwj, walk, scale):
     with gpu_dtwj.Context() as ctx:
         for fl in (0, gpu_dtwj.F_NO_SEED, gpu_dtwj.F_MASKED_CASCADE):
             r = ctx.join(x * scale, M, W, fl)
+            assert (r.i, r.j) == (ref.i, ref.j), fl
+            assert abs(r.dist - ref.dist) <= 1e-5 * ref.dist, fl
+
+
+# the smallest normal FP32 value is 2^-126, the smallest 2^-149
+@pytest.mark.parametrize("e", [-100, -126, -128, -140, -145, -150, -480])
+@pytest.mark.parametrize("m,w", [(256, 25), (1100, 20)])  # both copies of the block means
+def test_join_of_small_values(gpu_dtwj, oracle, walk, e, m, w):
+    x, ref = walk
+    if m != M:
+        ref = oracle.join(x, m, w)
+    with gpu_dtwj.Context() as ctx:
+        for fl in (0, gpu_dtwj.F_NO_SEED):
+            r = ctx.join(x * 2.0 ** e, m, w, fl)
             assert (r.i, r.j) == (ref.i, ref.j), fl
             assert abs(r.dist - ref.dist) <= 1e-5 * ref.dist, fl
