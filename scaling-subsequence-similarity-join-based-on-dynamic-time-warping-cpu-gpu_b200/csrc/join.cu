@@ -1516,8 +1516,8 @@ int dtwj_matrix_profile(const double* x, int64_t n, int32_t m, double* mp, int64
     cudaMemsetAsync(cnt, 0, 8, st);
     cudaMemsetAsync(rowmin, 0xff, s * 8, st);
     cudaMemsetAsync(rowidx, 0xff, s * 8, st);
-    // The first walk keeps the high word of ED^2 per window; every pair within
-    // ten units of it for either of its windows is a candidate, its FP64
+    // The first walk keeps the high word of ED^2 per window; every pair near it
+    // (near_limit, mp.cu) for either of its windows is a candidate, its FP64
     // distance is computed directly, and the row takes the smallest, lowest
     // partner on ties.
     launch_profile(S, tiles, nlb, false, best, nullptr, nullptr, nullptr, 0, ctx->num_sms,
@@ -1536,8 +1536,27 @@ int dtwj_matrix_profile(const double* x, int64_t n, int32_t m, double* mp, int64
       break;
     }
     if (cnt_h[0] > cap || cnt_h[1] > cap) {
-      rc = DTWJ_ERR_OVERFLOW;
-      break;
+      // more ties than the lists hold (a periodic series): again, a few tiles at
+      // a time, with lists that hold every pair of them
+      constexpr int kSlab = 8;
+      constexpr size_t kSlabPairs = (size_t)kSlab * kLbLags * kLbRows;
+      void* p;
+      if ((rc = ensure(ctx, B_OUT, 2 * kSlabPairs * sizeof(int2), &p))) break;
+      cand_up = static_cast<int2*>(p);
+      cand_lo = cand_up + kSlabPairs;
+      cudaMemsetAsync(rowmin, 0xff, s * 8, st);
+      cudaMemsetAsync(rowidx, 0xff, s * 8, st);
+      for (int pick = 0; pick < 2; ++pick)
+        for (int t = 0; t < nlb; t += kSlab) {
+          const int k = nlb - t < kSlab ? nlb - t : kSlab;
+          cudaMemsetAsync(cnt, 0, 8, st);
+          launch_profile(S, tiles + t, k, true, best, cand_up, cand_lo, cnt,
+                         (unsigned int)kSlabPairs, ctx->num_sms, st);
+          launch_mp_exact(S, cand_up, cnt, (unsigned int)kSlabPairs, pick != 0, rowmin, rowidx, st);
+          launch_mp_exact(S, cand_lo, cnt + 1, (unsigned int)kSlabPairs, pick != 0, rowmin, rowidx,
+                          st);
+        }
+      launch_mp_exact_out(s, rowmin, rowidx, dmp, dmpi, st);
     }
     if (cudaMemcpyAsync(mp, dmp, s * 8, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaMemcpyAsync(mpi, dmpi, s * 8, cudaMemcpyDeviceToHost, st) != cudaSuccess ||

@@ -450,6 +450,21 @@ struct ProfOut {
   unsigned int cap;
 };
 
+// The largest high word of ED^2 at which a pair is listed for a window whose
+// smallest is `best` (UINT_MAX: none).  Two words are within two units of each
+// other when their ED^2 are within 2^-19; ten units leave room for the
+// recurrence's relative rounding.  Near zero, where ED^2 is a difference of
+// equal terms, its absolute rounding counts: each of up to kLbRows rows rounds
+// twice by 2^-53 of a covariance of at most m sig_i sig_j, the anchor's m terms
+// once, so two pairs of equal distance are within 2 m (2^-39 + m 2^-52).  The
+// row and the column minimum of a window come from different places of their
+// tiles and round differently, also for bitwise equal partners.
+__device__ __forceinline__ unsigned int near_limit(unsigned int best, int m) {
+  if (best == UINT_MAX) return 0u;
+  const double e2 = __hiloint2double((int)best, 0) + m * (0x1p-38 + m * 0x1p-51);
+  return (unsigned int)__double2hiint(e2) + 10u;
+}
+
 template <bool COLLECT>
 __global__ void __launch_bounds__(kLbThreads, kProfCtasPerSm) k_profile(DevSeries S,
                                                                       const Tile* tiles, int part,
@@ -511,10 +526,7 @@ __global__ void __launch_bounds__(kLbThreads, kProfCtasPerSm) k_profile(DevSerie
       sh.is[x] = in ? S.isg[j] : 0.0;
       // a column past the series or flat: no weight, an offset no pair reaches
       sh.c2[x] = (in && !S.flat[j]) ? two_m : 1e300;
-      const unsigned int b = COLLECT && in ? out.best[j] : UINT_MAX;
-      // two high words are within two units of each other when their ED^2 are
-      // within 2^-19; ten units leave room for the recurrence's rounding
-      sh.col[x] = COLLECT ? (b == UINT_MAX ? 0u : b + 10u) : UINT_MAX;
+      sh.col[x] = COLLECT ? near_limit(in ? out.best[j] : UINT_MAX, m) : UINT_MAX;
     }
     for (int x = t; x < kStage; x += kLbThreads) {
       const int64_t i = r0 + x;
@@ -522,8 +534,7 @@ __global__ void __launch_bounds__(kLbThreads, kProfCtasPerSm) k_profile(DevSerie
       sh.r1[x] = up ? S.dfa[i - 1] : 0.0;
       sh.r2[x] = up ? S.dga[i - 1] : 0.0;
       sh.ci[x] = (in && !S.flat[i]) ? -2.0 * S.isg[i] : 0.0;
-      const unsigned int b = COLLECT && in ? out.best[i] : UINT_MAX;
-      sh.row[x] = COLLECT ? (b == UINT_MAX ? 0u : b + 10u) : UINT_MAX;
+      sh.row[x] = COLLECT ? near_limit(in ? out.best[i] : UINT_MAX, m) : UINT_MAX;
     }
     __syncthreads();
 #pragma unroll
