@@ -50,8 +50,11 @@ extern "C" {
 #define DTWJ_ERR_NOMODEL (-10)  /* learned ordering requested, no model loaded */
 #define DTWJ_ERR_SCRATCH (-11)  /* size exceeds the fixed scratch of dtwj_pair_dtw_noalloc */
 
-/* longest subsequence the joins accept (62 blocks of 1024 samples); longer m
- * returns DTWJ_ERR_ARG */
+/* longest subsequence any entry point accepts (62 blocks of 1024 samples);
+ * longer m returns DTWJ_ERR_ARG.  DTW holds both windows of a pair in shared
+ * memory, so joins, tile minima and FP64 pair lists end at 12,665 (w <= 31) to
+ * 12,217 samples (w = 255) and FP32 pair lists at about twice that: longer m
+ * returns DTWJ_ERR_ARG there too. */
 #define DTWJ_MAX_M 63488
 
 /* flags */

@@ -348,7 +348,10 @@ bool choose_band_join(int m, int w, BandShape* out);
 // Exact DTW lists (no early abandoning): G in {4, 8, 16, 32} and C in
 // [2, 16] covering 2w+1 diagonals with the least waste.
 bool choose_band_list(int w, BandShape* out);
-// The layout of a list of `count` pairs.
+// Whether a list of pairs in this layout runs: the windows of a warp's pairs
+// lie in shared memory.
+bool pair_list_fits(int m, BandShape band, bool precise);
+// The layout of a list of `count` pairs; false: w > 255 or none fits.
 bool choose_band_pairs(int m, int w, int64_t count, bool precise, BandShape* out);
 // (C, G) has a kernel instantiation and covers band w.
 bool band_shape_ok(int w, int C, int G);

@@ -559,6 +559,8 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   // the seeds and the verification: few pairs, each as fast as one can go
   BandShape wide;
   choose_band(w, &wide);
+  // windows too long for the FP64 verification (features need none)
+  if (!(tq && !tq->min_dist) && !pair_list_fits(m, wide, true)) return DTWJ_ERR_ARG;
   const bool learned = (flags & DTWJ_F_LEARNED) && !tq;
   if (learned && !ctx->model) return DTWJ_ERR_NOMODEL;
   if (learned && mlp_device(ctx->model) != ctx->device) return DTWJ_ERR_ARG;
@@ -901,6 +903,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     ph.begin();
     launch_verify(S, Q, wide, vd2, best_d2, best_ij, best_f32, st);
     ph.end(DTWJ_PHASE_VERIFY, 4);
+    CUDA_OK(cudaGetLastError());
     CUDA_OK(cudaEventRecord(ctx->ev1, st));
     CUDA_OK(cudaMemcpyAsync(result, result_dev, result_bytes, cudaMemcpyDeviceToHost, st));
     CUDA_OK(cudaStreamSynchronize(st));
@@ -1619,7 +1622,8 @@ int dtwj_pair_dtw(const double* x, int64_t n, int32_t m, int32_t w, const int64_
   if (count == 0) return DTWJ_OK;
   const int we = effective_band(m, w);
   BandShape band;
-  if (!choose_band_pairs(m, we, count, precise != 0, &band)) return DTWJ_ERR_BAND;
+  if (!choose_band(we, &band)) return DTWJ_ERR_BAND;
+  if (!choose_band_pairs(m, we, count, precise != 0, &band)) return DTWJ_ERR_ARG;
   dtwj_ctx* ctx = nullptr;
   rc = dtwj_ctx_create(0, &ctx);
   if (rc) return rc;
@@ -1637,7 +1641,8 @@ int dtwj_pair_dtw(const double* x, int64_t n, int32_t m, int32_t w, const int64_
     cudaMemcpyAsync(dp, pairs.data(), (size_t)count * sizeof(int2), cudaMemcpyHostToDevice,
                     ctx->stream);
     launch_pair_dtw(S, dp, (int)count, precise != 0, band, dout, ctx->stream);
-    if (cudaMemcpyAsync(dist, dout, (size_t)count * 8, cudaMemcpyDeviceToHost, ctx->stream) !=
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaMemcpyAsync(dist, dout, (size_t)count * 8, cudaMemcpyDeviceToHost, ctx->stream) !=
             cudaSuccess ||
         cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
       rc = DTWJ_ERR_CUDA;

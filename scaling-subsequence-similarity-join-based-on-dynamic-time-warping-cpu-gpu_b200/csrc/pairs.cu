@@ -606,13 +606,19 @@ void run_pairs(const DevSeries& S, const DevSearch& Q, const int2* pairs,
                                                               lay.total);
 }
 
+// Elements of T that a pair of a list takes in shared memory.
+int list_elems(int m, int C, int G, size_t elem_bytes) {
+  const int pq = G + 1, pt = G * C + G + 2;
+  const int elems = 2 * pq + 2 * pt + 2 * m;
+  return elems + (elem_bytes == 4 ? ((17 - elems % 32) + 32) % 32 : ((9 - elems % 16) + 16) % 16);
+}
+constexpr size_t kListSmem = 200 * 1024;
+
 template <typename T, int C, int G>
 void run_list(const DevSeries& S, const int2* pairs, const Candidate* cands,
               const unsigned int* count_ptr, int count, const unsigned int* bsf2, double* out,
               cudaStream_t st) {
-  const int pq = G + 1, pt = G * C + G + 2;
-  int elems = 2 * pq + 2 * pt + 2 * S.m;
-  elems += sizeof(T) == 4 ? ((17 - elems % 32) + 32) % 32 : ((9 - elems % 16) + 16) % 16;
+  const int elems = list_elems(S.m, C, G, sizeof(T));
   int threads = 128;
   size_t bytes = (size_t)(threads / G) * elems * sizeof(T);
   while (bytes > 100 * 1024 && threads > G && threads > 32) {
@@ -621,7 +627,7 @@ void run_list(const DevSeries& S, const int2* pairs, const Candidate* cands,
   }
   bytes = (size_t)(threads / G) * elems * sizeof(T);
   cudaFuncSetAttribute(k_dtw_list<T, C, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       200 * 1024);
+                       (int)kListSmem);
   const int groups = threads / G;
   int blocks = (count + groups - 1) / groups;
   if (blocks < 1) blocks = 1;
@@ -702,18 +708,18 @@ bool choose_band_list(int w, BandShape* out) {
   return true;
 }
 
+bool pair_list_fits(int m, BandShape band, bool precise) {
+  const size_t elem = precise ? 8 : 4;
+  return list_elems(m, band.C, band.G, elem) * elem * (32 / band.G) <= kListSmem;
+}
+
 bool choose_band_pairs(int m, int w, int64_t count, bool precise, BandShape* out) {
   // A short FP32 list runs in one wave, one pair per warp: the fewest cells per
   // lane make the shortest row step.
-  auto group_bytes = [&](int C, int G, int elem) {
-    return (double)elem * (2 * m + 2 * (G + 1) + 2 * (G * C + G + 2) + 32);
-  };
-  constexpr double kSmem = 200.0 * 1024;
   if (!precise) {
-    if (count <= 148 * 16) return choose_band(w, out);
-    if (!choose_band_list(w, out)) return false;
-    // windows so long that a warp's pairs do not fit: one pair per warp
-    if (group_bytes(out->C, out->G, 4) * (32 / out->G) > kSmem) return choose_band(w, out);
+    // windows so long that a warp's pairs do not fit also run one pair per warp
+    if (count <= 148 * 16 || !choose_band_list(w, out) || !pair_list_fits(m, *out, false))
+      return choose_band(w, out) && pair_list_fits(m, *out, false);
     return true;
   }
   // FP64 lists are bound by latency: a cell's minimum and multiply-add take
@@ -724,14 +730,13 @@ bool choose_band_pairs(int m, int w, int64_t count, bool precise, BandShape* out
   // operations per cell, 64 lanes).  20,000 pairs at m = 512, w = 52: (7, 16)
   // 1.46 ms, (4, 32) 1.23; at m = 256, w = 13: 0.36 -> 0.21 ms.
   const int cells = 2 * w + 1;
+  const double smem = (double)kListSmem;
   double best = 0.0;
   BandShape pick = {0, 0};
   for (int G = 4; G <= 32; G *= 2)
     for (int C = 2; C <= 16; ++C) {
-      if (C * G < cells || !band_supported(C, G)) continue;
-      const double bytes = group_bytes(C, G, 8);
-      if (G < 32 && bytes * (32 / G) > kSmem) continue;
-      double pairs = kSmem / bytes;
+      if (C * G < cells || !band_supported(C, G) || !pair_list_fits(m, {C, G}, true)) continue;
+      double pairs = smem / (8.0 * list_elems(m, C, G, 8));
       if (pairs > 20.0 * 32 / G) pairs = 20.0 * 32 / G;
       const double by_latency = pairs / (40.0 * C + 60.0), by_units = 16.0 / (C * G);
       const double rate = by_latency < by_units ? by_latency : by_units;
@@ -763,7 +768,7 @@ bool choose_band_join(int m, int w, BandShape* out) {
 void launch_pairs(const DevSeries& S, const DevSearch& Q, const int2* pairs,
                   const unsigned int* npairs, bool bounds, BandShape band, int num_sms,
                   cudaStream_t st) {
-  if (bounds && band.C <= 8 && slot_bytes(S.m, S.w, band.C, band.G) <= 200 * 1024) {
+  if (bounds && band.C <= 8 && 64 + slot_bytes(S.m, S.w, band.C, band.G) <= 200 * 1024) {
     auto go = band.G == 4    ? launch_dtw_slots4
               : band.G == 8  ? launch_dtw_slots8
               : band.G == 16 ? launch_dtw_slots16
@@ -882,9 +887,7 @@ __global__ void __launch_bounds__(128) k_dtw_pairs64(DevSeries S, const int64_t*
 template <typename T, int C, int G>
 void run_pairs64(const DevSeries& S, const int64_t* pi, const int64_t* pj, int64_t count,
                  double* out, cudaStream_t st) {
-  const int pq = G + 1, pt = G * C + G + 2;
-  int elems = 2 * pq + 2 * pt + 2 * S.m;
-  elems += sizeof(T) == 4 ? ((17 - elems % 32) + 32) % 32 : ((9 - elems % 16) + 16) % 16;
+  const int elems = list_elems(S.m, C, G, sizeof(T));
   int threads = 128;
   size_t bytes = (size_t)(threads / G) * elems * sizeof(T);
   while (bytes > 100 * 1024 && threads > G && threads > 32) {
@@ -893,7 +896,7 @@ void run_pairs64(const DevSeries& S, const int64_t* pi, const int64_t* pj, int64
   }
   bytes = (size_t)(threads / G) * elems * sizeof(T);
   cudaFuncSetAttribute(k_dtw_pairs64<T, C, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       200 * 1024);
+                       (int)kListSmem);
   const int groups = threads / G;
   int64_t blocks = (count + groups - 1) / groups;
   if (blocks < 1) blocks = 1;
