@@ -22,9 +22,12 @@
 // block-mean bound of single pairs (k_paa_groups).
 //
 // Records are FP32, rounded outward from FP64 (qmin, Lmin down, qmax, Umax
-// up), so only the evaluation rounds: each term is off by 2^-24 relative and
-// the sum by (terms + 2) 2^-24 < 3e-6, inside the 1/512 the threshold keeps
-// above the best-so-far.
+// up).  The FP64 means are of samples relative to the segment's first one, so
+// they round by 2^-53 of the window's own range, whatever its level (of samples
+// as they are, they were off by a thousandth of a deviation of 1e-12 of the
+// level, and pruned pairs).  What is left is the evaluation: each term is off
+// by 2^-24 relative and the sum by (terms + 2) 2^-24 < 3e-6, inside the 1/512
+// the threshold keeps above the best-so-far.
 #include "dtwj_dev.cuh"
 
 #include <cfloat>
@@ -41,15 +44,16 @@ struct SegOrder {
   unsigned char seg[kGrpSlots];  // segment of slot x; 255: a padding slot
 };
 
-// Means of the series and its envelope over [p, p + B), FP64: [3][n].
+// Means of the series and its envelope over [p, p + B) less sample p, FP64: [3][n].
 __global__ void k_seg_means(DevSeries S, int B, double* gm) {
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (p + B > S.n) return;
+  const double c = S.a[p];
   double sa = 0.0, su = 0.0, sl = 0.0;
   for (int k = 0; k < B; ++k) {
-    sa += S.a[p + k];
-    su += S.U[p + k];
-    sl += S.L[p + k];
+    sa += S.a[p + k] - c;
+    su += S.U[p + k] - c;
+    sl += S.L[p + k] - c;
   }
   const double ib = 1.0 / (double)B;
   gm[p] = sa * ib;
@@ -73,11 +77,11 @@ __global__ void k_group_rec(DevSeries S, const double* gm, SegOrder ord) {
       if (i >= S.s || S.flat[i]) continue;
       const double mu = S.mu[i], is = S.isg[i];
       const int64_t p = i + (int64_t)seg * S.grp_b;
-      const double q = (gm[p] - mu) * is;
+      const double c = S.a[p] - mu, q = (gm[p] + c) * is;
       qlo = fmin(qlo, q);
       qhi = fmax(qhi, q);
-      up = fmax(up, (gm[S.n + p] - mu) * is);
-      lo = fmin(lo, (gm[2 * S.n + p] - mu) * is);
+      up = fmax(up, (gm[S.n + p] + c) * is);
+      lo = fmin(lo, (gm[2 * S.n + p] + c) * is);
     }
     if (qlo <= qhi)
       rec = make_float4(__double2float_rd(qlo), __double2float_ru(qhi), __double2float_ru(up),

@@ -63,8 +63,9 @@ __device__ __forceinline__ double copy_center(const DevSeries& S, int copy, int6
 // Sliding block means over [p, p + B) of a, U and L, centered: on the
 // 1024-sample block of p (pq, windows longer than 1024 samples), or on the
 // block of p in each of the two copies (pq2), there also over [p, p + B / 4)
-// (fq, ful).  Entries whose block runs past the series are zero (never read: a
-// window's blocks end inside it).
+// (fq, ful).  The sums are of samples less sample p, so that they round by the
+// samples' spread, not by their level.  Entries whose block runs past the series
+// are zero (never read: a window's blocks end inside it).
 __global__ void k_slide_means(DevSeries S, int B) {
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (p >= S.n) return;
@@ -72,10 +73,11 @@ __global__ void k_slide_means(DevSeries S, int B) {
   const int F = B / 4;
   double sa = 0.0, su = 0.0, sl = 0.0, fa = 0.0, fu = 0.0, fl = 0.0;
   const int cnt = p + B <= S.n ? B : (p + F <= S.n ? F : 0);
+  const double first = S.a[p];
   for (int k = 0; k < cnt; ++k) {
-    sa += S.a[p + k];
-    su += S.U[p + k];
-    sl += S.L[p + k];
+    sa += S.a[p + k] - first;
+    su += S.U[p + k] - first;
+    sl += S.L[p + k] - first;
     if (k == F - 1) {
       fa = sa;
       fu = su;
@@ -87,18 +89,18 @@ __global__ void k_slide_means(DevSeries S, int B) {
     const double jf = 1.0 / (double)F;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-      const double x = copy_center(S, c, copy_block(c, p));
-      S.pq2[c * S.n + p] = cnt < B ? z : make_float4((float)(sa * ib - x), (float)(su * ib - x),
-                                                     (float)(sl * ib - x), 0.0f);
+      const double x = first - copy_center(S, c, copy_block(c, p));
+      S.pq2[c * S.n + p] = cnt < B ? z : make_float4((float)(sa * ib + x), (float)(su * ib + x),
+                                                     (float)(sl * ib + x), 0.0f);
       const int64_t at = fine_at(S, c, p);
-      S.fq[at] = cnt < F ? 0.0f : (float)(fa * jf - x);
+      S.fq[at] = cnt < F ? 0.0f : (float)(fa * jf + x);
       S.ful[at] = cnt < F ? make_float2(0.0f, 0.0f)
-                          : make_float2((float)(fu * jf - x), (float)(fl * jf - x));
+                          : make_float2((float)(fu * jf + x), (float)(fl * jf + x));
     }
   } else {
-    const double x = S.cb[p >> kBlkShift];
-    S.pq[p] = cnt < B ? z : make_float4((float)(sa * ib - x), (float)(su * ib - x),
-                                        (float)(sl * ib - x), 0.0f);
+    const double x = first - S.cb[p >> kBlkShift];
+    S.pq[p] = cnt < B ? z : make_float4((float)(sa * ib + x), (float)(su * ib + x),
+                                        (float)(sl * ib + x), 0.0f);
   }
 }
 
