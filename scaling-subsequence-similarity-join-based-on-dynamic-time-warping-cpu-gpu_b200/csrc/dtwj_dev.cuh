@@ -233,6 +233,8 @@ struct DevSearch {
   unsigned int* kq_count;
   unsigned int* kq_next;
   unsigned int kq_cap;
+  unsigned long long* low;      // [2] of this join: pairs well below the threshold that LB_Keogh
+                                //   tried all the same, those of them it pruned
 };
 
 __device__ __forceinline__ float max3f(float a, float b, float c) {

@@ -125,7 +125,7 @@ __global__ void k_chunk_note(int* status, const unsigned long long* counters, Ch
 // counters, candidates and the seeds' work counter zero.
 __global__ void k_init_search(unsigned int* bsf2, int nslots, unsigned long long* counters,
                               unsigned int* cand_count, unsigned int* nseeds, int nseries,
-                              int seed_slots, unsigned int* zready) {
+                              int seed_slots, unsigned int* zready, unsigned long long* low) {
   for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < nslots; x += gridDim.x * blockDim.x)
     bsf2[x] = 0x7f800000u;
   if (blockIdx.x == 0) {
@@ -135,6 +135,7 @@ __global__ void k_init_search(unsigned int* bsf2, int nslots, unsigned long long
       nseeds[nseries] = (unsigned int)seed_slots;
       nseeds[nseries + 1] = 0u;
       zready[0] = zready[1] = 0u;  // the window table: not filled
+      low[0] = low[1] = 0ull;
     }
   }
 }
@@ -662,6 +663,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
       A.add(&F.dense, (size_t)chunk_max * 4);
       A.add(&Q.bsf2, (size_t)nslots * 4);
       A.add(&S.zready, 8);
+      A.add(&Q.low, 16);
       A.add(&seeds, (size_t)nseries * kSeedSlots * sizeof(int2));
       A.add(&nseeds, ((size_t)nseries + 2) * 4);
       A.add(&notes, (ranges.size() + 1) * sizeof(ChunkNote));
@@ -721,7 +723,8 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     paa_next = qc + 11;
     if (S.grp) F.tcount = qc + kQcTiles;
     k_init_search<<<(nslots + 255) / 256 < 256 ? (nslots + 255) / 256 : 256, 256, 0, st>>>(
-        Q.bsf2, nslots, Q.counters, Q.cand_count, nseeds, nseries, nseries * kSeedSlots, S.zready);
+        Q.bsf2, nslots, Q.counters, Q.cand_count, nseeds, nseries, nseries * kSeedSlots, S.zready,
+        Q.low);
   }
 
   // ---- ED matrix profile (row minima; per tile for the tile minima) ----

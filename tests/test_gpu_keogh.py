@@ -25,3 +25,16 @@ def test_fine_block_means_match_the_oracle(gpu_dtwj, oracle, synth, kind, n, m, 
             total = (r.pruned_fast + r.pruned_paa + r.pruned_kim + r.pruned_masked +
                      r.pruned_keogh + r.dtw_calls)
             assert 0 <= total - r.pairs <= 700, (fl, total, r.pairs)
+
+
+def test_exact_bound_where_block_means_say_little(gpu_dtwj, oracle, synth):
+    # half a walk, half noise: the fine block means stay far below LB_Keogh, which prunes
+    # 72 of the 81 million pairs that reach it when it is tried on all; a third more DTWs
+    # than that are allowed for the pairs that pass before the rule has seen enough
+    x = synth.random_walk(30007, 7)
+    x[15003:] = x[15003] + np.random.default_rng(7).standard_normal(15004)
+    with gpu_dtwj.Context() as ctx:
+        r = ctx.join(x, 700, 20)
+        assert r.dtw_calls < (r.dtw_calls + r.pruned_keogh) * (1 - 72.0 / 81.0) * 4 / 3
+        plain = ctx.join(x, 700, 20, gpu_dtwj.F_MASKED_CASCADE)
+    assert (r.i, r.j) == (plain.i, plain.j) and abs(r.dist - plain.dist) <= 1e-9
