@@ -262,6 +262,8 @@ struct GroupFilter {
   unsigned int sup_cap, list_cap;
   const float* cut;      // seeds only: the cutoff on ED^2 ...
   unsigned int* walk;    // ... and whether the diagonals must be walked after all
+  unsigned int* off;     // nonzero: the bound settles nothing on this join, every tile is dense
+  unsigned int* probe;   // [3] zeroed words of launch_group_probe
   unsigned int* dense;   // tiles the diagonal sweep ran on
   unsigned int* ndense;
   int nib, nw;           // first-level work items per tile: blocks of row groups x column words
@@ -411,8 +413,8 @@ void launch_mp_seed(const DevSeries& S, const Tile* tiles, int ntiles, unsigned 
                     const unsigned int* walk, int num_sms, cudaStream_t st);
 // The same keys for the rows that can be among the kSeeds smallest, by the
 // group bound (group.cu).  F: lists of sup_cap and list_cap entries, nsup,
-// nlist, tcount (one word: the group pair count) consecutive, cut and walk;
-// samples: kSeedSamples floats.  Single series.
+// nlist, tcount (one word: the group pair count) consecutive, walk and probe
+// consecutive, cut; samples: kSeedSamples floats.  Single series.
 constexpr int kSeedSamples = 2048;
 constexpr int kSeedSlab = 16384;  // tiles per pass
 void launch_seed_groups(const DevSeries& S, GroupFilter F, const Tile* tiles, int ntiles,
@@ -429,6 +431,10 @@ void group_shape(int m, int64_t s, DevSeries* S);
 int launch_group_prep(const DevSeries& S, double* means, cudaStream_t st);
 // and returns the largest number of super-group pairs of one.
 size_t group_items(int g, GroupFilter* F);
+// Samples group pairs of the join's tiles against the best-so-far and sets *F.off
+// if nearly all survive.
+void launch_group_probe(const DevSeries& S, const DevSearch& Q, const GroupFilter& F,
+                        const Tile* tiles, int ntiles, cudaStream_t st);
 // F.nsup, F.nlist and F.tcount are zero at launch.  Two kernels.
 void launch_group(const DevSeries& S, const DevSearch& Q, const GroupFilter& F, const Tile* tiles,
                   int tile_begin, int tile_end, int num_sms, cudaStream_t st);
@@ -466,8 +472,8 @@ void launch_paa(const DevSeries& S, const DevSearch& Q, const GroupFilter& F, co
 // The same over the pairs of the group filter's surviving groups (sparse
 // tiles; next: a zeroed work counter).
 void launch_paa_groups(const DevSeries& S, const DevSearch& Q, const GroupFilter& F,
-                       const Tile* tiles, int tile_begin, unsigned int* next, int num_sms,
-                       cudaStream_t st);
+                       const Tile* tiles, int tile_begin, int tile_end, unsigned int* next,
+                       int num_sms, cudaStream_t st);
 // Block length of the block-mean bound for windows of length m.
 int paa_block(int m);
 // Sliding block means (pq, or pq2 and wrec for windows of at most 1024

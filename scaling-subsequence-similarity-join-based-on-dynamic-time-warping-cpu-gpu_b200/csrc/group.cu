@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kThreads) k_group_super(DevSeries S, DevSearch
                                                           const Tile* tiles, unsigned int total) {
   const int lane = threadIdx.x & 31;
   const unsigned int item = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-  if (item >= total) return;
+  if (item >= total || *(ED ? F.walk : F.off) != 0u) return;
   const unsigned int per = (unsigned int)(F.nib * F.nw);
   const unsigned int tk = item / per, rem = item - tk * per;
   const Tile T = tiles[tk];
@@ -264,6 +264,52 @@ __global__ void __launch_bounds__(kThreads) k_group(DevSeries S, DevSearch Q, Gr
   }
 }
 
+// Whether the bound settles anything.  On white noise it settles nothing, its two
+// levels are extra work (70,000 samples of noise, m = 512, w = 0: 7.6 ms with
+// them, 5.1 without), and the seeds' lists of group pairs overflow (100,003
+// samples, m = 256: 8.7 ms for the seeds, walking the diagonals takes 1.1).  A
+// sample of the pairs of the join's tiles, one per thread and spread over the
+// tiles, decides first: *flag is set if more than num / den of their group pairs
+// survive the threshold.  Pairs without a threshold yet don't count.
+constexpr int kProbeSamples = 8192;
+template <bool ED>
+__global__ void __launch_bounds__(kThreads) k_group_probe(DevSeries S, DevSearch Q, GroupFilter F,
+                                                          const Tile* tiles, int ntiles,
+                                                          unsigned int num, unsigned int den,
+                                                          unsigned int* flag) {
+  const unsigned int x = blockIdx.x * kThreads + threadIdx.x;
+  const Tile T = tiles[(unsigned long long)x * ntiles / kProbeSamples];
+  unsigned int h = x * 0x9e3779b1u;  // a row and a lag of the tile
+  h = (h ^ (h >> 15)) * 0x85ebca77u;
+  h ^= h >> 13;
+  const int row = (int)(h % (unsigned)T.rows), lag = (int)(h / (unsigned)T.rows % kLbLags);
+  const int64_t i = T.i0 + row, j = i + T.L0 + lag;
+  const float thr = ED ? *F.cut : prune_threshold_now(Q.bsf2 + T.series, S.m);
+  const bool counts = j < T.send && thr < __int_as_float(0x7f800000);
+  bool alive = counts;
+  if (counts) {
+    const float4 *pi = S.grp + i / S.grp_g, *pj = S.grp + j / S.grp_g;
+    float a1 = 0.0f, a2 = 0.0f;
+    for (int s0 = 0; s0 < S.grp_d && alive; s0 += 4) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        group_terms<ED>(pi[(s0 + u) * S.grp_n], pj[(s0 + u) * S.grp_n], a1, a2);
+      alive = !((float)S.grp_b * fmaxf(a1, a2) > thr);
+    }
+  }
+  const int all = __syncthreads_count(counts), left = __syncthreads_count(alive);
+  if (threadIdx.x == 0) {
+    atomicAdd(&F.probe[0], (unsigned int)all);
+    atomicAdd(&F.probe[1], (unsigned int)left);
+    __threadfence();
+    if (atomicAdd(&F.probe[2], 1u) == gridDim.x - 1) {
+      __threadfence();
+      const unsigned int total = atomicAdd(&F.probe[0], 0u), kept = atomicAdd(&F.probe[1], 0u);
+      if (kept * den > total * num) *flag = 1u;
+    }
+  }
+}
+
 // The masked cascade reads survivor bits: the pairs of the surviving groups
 // of the sparse tiles, set in the bits the diagonal sweep cleared for them.
 __global__ void k_group_bits(DevSeries S, DevSearch Q, GroupFilter F, const Tile* tiles,
@@ -365,6 +411,13 @@ void run_group(const DevSeries& S, const DevSearch& Q, const GroupFilter& F, con
   k_group<ED><<<num_sms * 8, kThreads, 0, st>>>(S, Q, F, tiles);
 }
 }  // namespace
+
+// 15/16: a tile stays sparse at 7/8 or less, so hardly any would.
+void launch_group_probe(const DevSeries& S, const DevSearch& Q, const GroupFilter& F,
+                        const Tile* tiles, int ntiles, cudaStream_t st) {
+  k_group_probe<false><<<kProbeSamples / kThreads, kThreads, 0, st>>>(S, Q, F, tiles, ntiles, 15u,
+                                                                      16u, F.off);
+}
 
 void launch_group(const DevSeries& S, const DevSearch& Q, const GroupFilter& F, const Tile* tiles,
                   int tile_begin, int tile_end, int num_sms, cudaStream_t st) {
@@ -478,6 +531,7 @@ __global__ void __launch_bounds__(kThreads) k_seed_exact(DevSeries S, GroupFilte
                                                          unsigned long long* keys) {
   const int lane = threadIdx.x & 31;
   const unsigned int total = *F.nlist;
+  if (*F.walk != 0u) return;
   // too many group pairs, or some were dropped: the diagonals are walked instead
   if (total > F.list_cap || *F.nsup > F.sup_cap || *F.tcount > budget) {
     if (blockIdx.x == 0 && threadIdx.x == 0) *F.walk = 1u;
@@ -536,7 +590,7 @@ void launch_seed_groups(const DevSeries& S, GroupFilter F, const Tile* tiles, in
                         int world, float* samples, unsigned long long* keys, int num_sms,
                         cudaStream_t st) {
   cudaMemsetAsync(keys, 0xff, (size_t)S.s * 8, st);
-  cudaMemsetAsync(F.walk, 0, 4, st);
+  cudaMemsetAsync(F.walk, 0, 16, st);  // and the words of the probe
   // one row group in `stride`, at most kSeedSamples; the rank that should
   // leave 4 kSeeds grid rows (of this shard) below the cutoff, at least 4 deep
   const int64_t ng = (S.s + S.grp_g - 1) / S.grp_g, rows = (S.s + kSeedGrid - 1) / kSeedGrid;
@@ -548,6 +602,10 @@ void launch_seed_groups(const DevSeries& S, GroupFilter F, const Tile* tiles, in
   if (rank > count - 1) rank = count - 1;
   k_seed_sample<<<count, kThreads, 0, st>>>(S, stride, samples);
   k_seed_cut<<<1, 1024, 0, st>>>(samples, count, (int)rank, const_cast<float*>(F.cut));
+  // one group pair in 128 (g = 8) or 256 may survive (the budget below); twice that
+  // in a sample is too many
+  k_group_probe<true><<<kProbeSamples / kThreads, kThreads, 0, st>>>(
+      S, DevSearch{}, F, tiles, ntiles, 1u, S.grp_g == 8 ? 64u : 128u, F.walk);
   for (int b = 0; b < ntiles; b += kSeedSlab) {
     const int cnt = ntiles - b < kSeedSlab ? ntiles - b : kSeedSlab;
     cudaMemsetAsync(F.nsup, 0, 12, st);  // nsup, nlist and the group pair count

@@ -52,8 +52,13 @@ constexpr int kLbChunkRounds = 4;
 // queue (2^27 entries) and 55 would not.
 constexpr int kResweepTiles = 32;
 // Tiles from which the seeds come from the group bound instead of a walk over
-// every diagonal.
+// every diagonal: random walks of 100,003 samples (1,421 tiles, m = 256) 0.87 ms
+// against 1.04, of 131,071 (m = 512) 1.02 against 1.74; at 65,536 (590 tiles)
+// 0.62 against 0.56.
 constexpr int kSeedGroupTiles = 1024;
+// Tiles from which a sample decides whether the sweep uses the group bound at all
+// (4 us; the smallest such join takes about 1 ms).
+constexpr int kProbeTiles = 256;
 // Their lists of group pairs, and with the samples and five words the bytes
 // they take.
 constexpr unsigned int kSeedSupCap = 1u << 24, kSeedListCap = 1u << 22;
@@ -125,7 +130,8 @@ __global__ void k_chunk_note(int* status, const unsigned long long* counters, Ch
 // counters, candidates and the seeds' work counter zero.
 __global__ void k_init_search(unsigned int* bsf2, int nslots, unsigned long long* counters,
                               unsigned int* cand_count, unsigned int* nseeds, int nseries,
-                              int seed_slots, unsigned int* zready, unsigned long long* low) {
+                              int seed_slots, unsigned int* zready, unsigned long long* low,
+                              unsigned int* group_off) {
   for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < nslots; x += gridDim.x * blockDim.x)
     bsf2[x] = 0x7f800000u;
   if (blockIdx.x == 0) {
@@ -136,6 +142,7 @@ __global__ void k_init_search(unsigned int* bsf2, int nslots, unsigned long long
       nseeds[nseries + 1] = 0u;
       zready[0] = zready[1] = 0u;  // the window table: not filled
       low[0] = low[1] = 0ull;
+      group_off[0] = group_off[1] = group_off[2] = group_off[3] = 0u;
     }
   }
 }
@@ -664,6 +671,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
       A.add(&Q.bsf2, (size_t)nslots * 4);
       A.add(&S.zready, 8);
       A.add(&Q.low, 16);
+      A.add(&F.off, 16);
       A.add(&seeds, (size_t)nseries * kSeedSlots * sizeof(int2));
       A.add(&nseeds, ((size_t)nseries + 2) * 4);
       A.add(&notes, (ranges.size() + 1) * sizeof(ChunkNote));
@@ -724,7 +732,8 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     if (S.grp) F.tcount = qc + kQcTiles;
     k_init_search<<<(nslots + 255) / 256 < 256 ? (nslots + 255) / 256 : 256, 256, 0, st>>>(
         Q.bsf2, nslots, Q.counters, Q.cand_count, nseeds, nseries, nseries * kSeedSlots, S.zready,
-        Q.low);
+        Q.low, F.off);
+    F.probe = F.off + 1;
   }
 
   // ---- ED matrix profile (row minima; per tile for the tile minima) ----
@@ -756,10 +765,11 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
       E.nlist = word + 1;
       E.tcount = word + 2;
       E.walk = word + 3;
-      E.cut = reinterpret_cast<const float*>(word + 4);
+      E.probe = word + 4;
+      E.cut = reinterpret_cast<const float*>(word + 7);
       launch_seed_groups(S, E, lbtiles, nlb, ctx->shard_world, samples, keys, ctx->num_sms, st);
       launch_mp_seed(S, lbtiles, nlb, keys, E.walk, ctx->num_sms, st);
-      launches = 3 + 3 * ((nlb + kSeedSlab - 1) / kSeedSlab);
+      launches = 4 + 3 * ((nlb + kSeedSlab - 1) / kSeedSlab);
     } else {
       launch_mp_seed(S, lbtiles, nlb, keys, nullptr, ctx->num_sms, st);
       launches = 1;
@@ -817,7 +827,9 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     Qs.queue_next = nseeds + nseries + 1;
     Qs.queue_cap = (unsigned int)(nseries * kSeedSlots);
     launch_pairs(S, Qs, seeds, nseeds + nseries, false, wide, ctx->num_sms, st);
-    ph.end(DTWJ_PHASE_SEEDS, 2);
+    const bool probe = S.grp && nlb >= kProbeTiles;
+    if (probe) launch_group_probe(S, Q, F, lbtiles, nlb, st);
+    ph.end(DTWJ_PHASE_SEEDS, probe ? 3 : 2);
   }
   CUDA_OK(cudaMemcpyAsync(seed_bsf, Q.bsf2, (size_t)nslots * 4, cudaMemcpyDeviceToDevice, st));
 
@@ -829,7 +841,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
       launch_runs(S, Q, lbtiles, t0, t1, bits, masked, !enumerate_all, ctx->num_sms, st);
       ph.end(DTWJ_PHASE_RUNS, 1);
     } else {
-      if (S.grp) launch_paa_groups(S, Q, F, lbtiles, t0, paa_next, ctx->num_sms, st);
+      if (S.grp) launch_paa_groups(S, Q, F, lbtiles, t0, t1, paa_next, ctx->num_sms, st);
       launch_paa(S, Q, F, lbtiles, t0, t1, bits, ctx->num_sms, st);
       ph.end(DTWJ_PHASE_RUNS, S.grp ? 2 : 1);
     }

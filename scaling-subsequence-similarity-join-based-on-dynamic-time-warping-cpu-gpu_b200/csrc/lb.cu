@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kLbThreads, kLbCtasPerSm) k_lb(DevSeries S, De
     if (k >= (unsigned int)ntiles) break;
     const Tile T = tiles[k];
     unsigned int* out = bits + (size_t)k * kLbLags * kLbWords;
-    if (F.tcount && !group_tile_dense(T, S.grp_g, F.tcount[k])) {
+    if (F.tcount && *F.off == 0u && !group_tile_dense(T, S.grp_g, F.tcount[k])) {
       if (threadIdx.x == 0) sparse += (unsigned long long)tile_pairs(T);
       if (clear_sparse)
         for (int x = threadIdx.x; x < kLbLags * kLbWords; x += kLbThreads) out[x] = 0u;

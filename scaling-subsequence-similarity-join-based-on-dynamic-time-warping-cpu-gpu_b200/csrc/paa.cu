@@ -550,7 +550,9 @@ __global__ void __launch_bounds__(kPaaWarps * 32, 3) k_paa_lags(DevSeries S, Dev
 template <int B, int G>
 __global__ void __launch_bounds__(kPaaWarps * 32, 3) k_paa_groups(DevSeries S, DevSearch Q,
                                                                   GroupFilter F, const Tile* tiles,
+                                                                  unsigned int ntiles,
                                                                   unsigned int* next) {
+  if (*F.ndense == ntiles) return;  // (the list then holds pairs of dense tiles only)
   constexpr int R = G == 8 ? 2 : 1;  // pairs per lane
   __shared__ unsigned long long cnt_paa, cnt_kim, cnt_seen;
   if (threadIdx.x == 0) cnt_paa = cnt_kim = cnt_seen = 0;
@@ -720,13 +722,14 @@ void launch_paa(const DevSeries& S, const DevSearch& Q, const GroupFilter& F, co
 }
 
 void launch_paa_groups(const DevSeries& S, const DevSearch& Q, const GroupFilter& F,
-                       const Tile* tiles, int tile_begin, unsigned int* next, int num_sms,
-                       cudaStream_t st) {
+                       const Tile* tiles, int tile_begin, int tile_end, unsigned int* next,
+                       int num_sms, cudaStream_t st) {
   auto go = [&](auto kern) {
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPaaWarps * 32, 0);
     if (per_sm < 1) per_sm = 1;
-    kern<<<num_sms * per_sm, kPaaWarps * 32, 0, st>>>(S, Q, F, tiles + tile_begin, next);
+    kern<<<num_sms * per_sm, kPaaWarps * 32, 0, st>>>(S, Q, F, tiles + tile_begin,
+                                                      (unsigned int)(tile_end - tile_begin), next);
   };
   // group_windows and paa_block change at the same window lengths
   if (S.paa_b == 32) go(k_paa_groups<32, 8>);
