@@ -18,7 +18,8 @@
 // previous step (a shuffle of its last cell) and (r-1, d+1) from the right
 // lane's first cell of this step (a shuffle right after it is computed), so
 // every lane computes a full row of its C cells per step with two shuffles.
-// The join runs one pair per warp (G = 32); pair lists pack several.  q and t
+// The join's queue runs in slots (dtw_slots.cuh) up to w = 127 and one pair per
+// warp here (G = 32) above, as its seeds do; pair lists pack several.  q and t
 // are z-normalised in shared memory with finite sentinels outside [0, m) so
 // out-of-range cells are effectively infinite without branches; a lane keeps
 // the q and t values of C consecutive steps in registers.
@@ -70,15 +71,16 @@ __device__ __forceinline__ V group_sum(V v, unsigned int gm) {
   return v;
 }
 
-// Shared-memory footprint of one group (in elements of T).
-struct GroupLayout {
+// Shared-memory footprint of a warp of k_pairs (in floats).
+struct WarpLayout {
   int pq, pt;     // padding of q and t on each side
   int nc;         // cumulative-bound chunks
   int q_off, t_off, cb_off, total;
 };
 
-__host__ __device__ inline GroupLayout group_layout(int m, int w, int C, int G, bool bounds) {
-  GroupLayout l;
+__host__ __device__ inline WarpLayout warp_layout(int m, int C) {
+  constexpr int G = 32;
+  WarpLayout l;
   l.pq = G + 1;
   l.pt = G * C + G + 2;  // t is read at offsets [-(G + w), m + G + GC)
   l.nc = (m + 7) / 8;
@@ -86,10 +88,6 @@ __host__ __device__ inline GroupLayout group_layout(int m, int w, int C, int G, 
   l.t_off = l.pq + m + l.pq + l.pt;
   l.cb_off = l.t_off + m + l.pt;
   l.total = l.cb_off + l.nc + 2;
-  // groups of a warp read their own q and t at a stride of C - 1 floats per
-  // lane: an odd group stride (17 mod 32) keeps two groups off each other's
-  // shared-memory banks
-  l.total = l.total + ((17 - l.total % 32) + 32) % 32;
   return l;
 }
 
@@ -102,24 +100,20 @@ __host__ __device__ inline GroupLayout group_layout(int m, int w, int C, int G, 
 // q[r] and tw(c) returns t[r + d_lo + c].  With LIVE false the lane keeps its
 // row (a lane that has not reached row 0 yet), and its neighbours read its
 // unchanged cells: for row 0 those are the virtual row -1 (0 on d = 0, +inf
-// elsewhere), exactly what row 0 needs.  HI selects the cells that take the
-// band mask: every cell (HI = -2), none (HI = -1) or cell HI alone (the
-// layouts of dtw_band that keep the lanes past the band huge by their q).
-template <typename T, int C, int G, int HI, typename TW>
+// elsewhere), exactly what row 0 needs.
+template <typename T, int C, int G, typename TW>
 __device__ __forceinline__ void band_step(T qr, const TW& tw, bool live, int g, unsigned int gm,
                                           const T (&pen)[C], T (&A)[C]) {
   // Lane 0's left neighbour and lane G-1's right neighbour wrap around the
   // group, so no lane needs a select: C G is even and 2w + 1 odd, so C G >
   // 2w + 1 and lane G-1's last cell lies past the band; its +inf penalty
-  // (or its huge cost) keeps it huge, which is what lane 0's first cell
-  // (d = -w) needs on its left, and makes whatever comes from the right
-  // irrelevant to it.
+  // keeps it huge, which is what lane 0's first cell (d = -w) needs on its
+  // left, and makes whatever comes from the right irrelevant to it.
   const T left = __shfl_sync(gm, A[C - 1], (g + G - 1) & (G - 1), G);
   {
     const T d = qr - tw(0);
     const T v = fmin3_(A[1], A[0], left);
-    T x = fma(d, d, v);
-    if (HI == -2 || HI == 0) x = fmax_(x, pen[0]);
+    const T x = fmax_(fma(d, d, v), pen[0]);
     A[0] = live ? x : A[0];
   }
   const T right = __shfl_sync(gm, A[0], (g + 1) & (G - 1), G);
@@ -128,8 +122,7 @@ __device__ __forceinline__ void band_step(T qr, const TW& tw, bool live, int g, 
     const T up = (c + 1 < C) ? A[c + 1 < C ? c + 1 : 0] : right;
     const T d = qr - tw(c);
     const T v = fmin3_(up, A[c], A[c - 1]);
-    T x = fma(d, d, v);
-    if (HI == -2 || HI == c) x = fmax_(x, pen[c]);
+    const T x = fmax_(fma(d, d, v), pen[c]);
     A[c] = live ? x : A[c];
   }
 }
@@ -150,18 +143,7 @@ __device__ __forceinline__ void band_step(T qr, const TW& tw, bool live, int g, 
 // every 16 steps whether every lane's latest row, plus the cumulative bound
 // of the rows still ahead, exceeds the threshold; it then returns +inf and
 // reports the cells it swept.
-//
-// Band mask: HI = -2 masks every cell past the band.  Otherwise HI is the
-// cell, (2w + 1) mod C, at which diagonal w + 1 (the first past the band)
-// sits in its lane (-1 when that is the lane's first cell), and only that
-// cell is masked: it walls the band off from the diagonals beyond, and the
-// lanes whose cells all lie past the band (after that lane, or from it when
-// HI = -1) read the q sentinel instead of q, so every cell they compute is at
-// least 1e36 with no mask.  Lane 0's left neighbour is then such a cell, the
-// cells between the wall and those lanes only see huge values, and every cell
-// of the band, the abandoning test and the result are the same as with the
-// full mask.
-template <typename T, int C, int G, bool ABANDON, int HI = -2>
+template <typename T, int C, int G, bool ABANDON>
 __device__ T dtw_band(const T* __restrict__ q, const T* __restrict__ t, int m, int w,
                       const float* __restrict__ cbc, int nc, float thr,
                       const unsigned int* bsf2, unsigned int gm, int g,
@@ -177,9 +159,6 @@ __device__ T dtw_band(const T* __restrict__ q, const T* __restrict__ t, int m, i
   }
   const T* qg = q - g;         // qg[tau] = q[row]
   const T* tg = t - g + d_lo;  // tg[tau + c] = t[row + d_lo + c]
-  const int g_past = (2 * w + 1) / C + (HI == -1 ? 0 : 1);
-  const bool past = HI != -2 && g >= g_past;  // reads the sentinel q[-1 - x]
-  const T PQ = Pad<T>::q();
   const int g0 = w / C, c0 = w % C;
   const int tau_end = m - 1 + g0;  // lane g0 (cell c0 on d = 0) reaches row m - 1
   *abandoned = false;
@@ -188,8 +167,7 @@ __device__ T dtw_band(const T* __restrict__ q, const T* __restrict__ t, int m, i
   int tau = 0;
   for (; tau < warm; ++tau) {
     const T* tp = tg + tau;
-    band_step<T, C, G, HI>(past ? PQ : qg[tau], [tp](int c) { return tp[c]; }, tau - g >= 0, g,
-                           gm, pen, A);
+    band_step<T, C, G>(qg[tau], [tp](int c) { return tp[c]; }, tau - g >= 0, g, gm, pen, A);
   }
   // blocks of C steps with q and t in registers, two per iteration: W is a
   // ring of 2C values of t (offset x from the iteration's first step at
@@ -202,8 +180,7 @@ __device__ T dtw_band(const T* __restrict__ q, const T* __restrict__ t, int m, i
     for (int x = 0; x < C - 1; ++x) W[x] = tg[tau + x];
   }
   const T* tb = tg + tau + C - 1;  // the blocks' new values of t, and of q,
-  const T* qb = past ? q - 2 * C : qg + tau;  // at immediate offsets from two pointers
-  const int qstep = past ? 0 : 2 * C;
+  const T* qb = qg + tau;          // at immediate offsets from two pointers
   while (tau + 2 * C - 1 <= tau_end) {
     T Qv[2 * C];
 #pragma unroll
@@ -212,15 +189,15 @@ __device__ T dtw_band(const T* __restrict__ q, const T* __restrict__ t, int m, i
     for (int x = 0; x < 2 * C; ++x) Qv[x] = qb[x];
 #pragma unroll
     for (int k = 0; k < C; ++k)
-      band_step<T, C, G, HI>(Qv[k], [&W, k](int c) { return W[k + c]; }, true, g, gm, pen, A);
+      band_step<T, C, G>(Qv[k], [&W, k](int c) { return W[k + c]; }, true, g, gm, pen, A);
 #pragma unroll
     for (int x = 0; x < C; ++x) W[(2 * C - 1 + x) % (2 * C)] = tb[C + x];
 #pragma unroll
     for (int k = 0; k < C; ++k)
-      band_step<T, C, G, HI>(Qv[C + k], [&W, k](int c) { return W[(C + k + c) % (2 * C)]; }, true,
-                             g, gm, pen, A);
+      band_step<T, C, G>(Qv[C + k], [&W, k](int c) { return W[(C + k + c) % (2 * C)]; }, true, g,
+                         gm, pen, A);
     tb += 2 * C;
-    qb += qstep;
+    qb += 2 * C;
     tau += 2 * C;
     if (ABANDON && --ab_count == 0 && tau <= tau_end) {
       ab_count = kAbEvery;
@@ -261,14 +238,13 @@ __device__ T dtw_band(const T* __restrict__ q, const T* __restrict__ t, int m, i
     }
 #pragma unroll
     for (int k = 0; k < C; ++k)
-      band_step<T, C, G, HI>(Qv[k], [&W, k](int c) { return W[k + c]; }, true, g, gm, pen, A);
+      band_step<T, C, G>(Qv[k], [&W, k](int c) { return W[k + c]; }, true, g, gm, pen, A);
     tau += C;
   }
   // the last steps (fewer than C)
   for (; tau <= tau_end; ++tau) {
     const T* tp = tg + tau;
-    band_step<T, C, G, HI>(past ? PQ : qg[tau], [tp](int c) { return tp[c]; }, true, g, gm, pen,
-                           A);
+    band_step<T, C, G>(qg[tau], [tp](int c) { return tp[c]; }, true, g, gm, pen, A);
   }
   T result = INF;
 #pragma unroll
@@ -279,12 +255,13 @@ __device__ T dtw_band(const T* __restrict__ q, const T* __restrict__ t, int m, i
   return result;
 }
 
-// The pair consumer: every group takes pairs from the queue until it is
-// drained.  flags bit 0: run the bounds (otherwise DTW only, for seeds).
-template <int C, int G, int HI>
+// The pair consumer, one pair per warp: every warp takes pairs from the queue
+// until it is drained.  flags bit 0: run the bounds (otherwise DTW only, for
+// seeds).
+template <int C>
 __global__ void __launch_bounds__(256) k_pairs(DevSeries S, DevSearch Q, const int2* pairs,
-                                                const unsigned int* npairs, int flags,
-                                                int group_floats) {
+                                                const unsigned int* npairs, int flags) {
+  constexpr int G = 32;
   extern __shared__ __align__(16) unsigned char smraw[];
   float* sm = reinterpret_cast<float*>(smraw);
   __shared__ unsigned long long cnt[kNumCounters];
@@ -292,8 +269,8 @@ __global__ void __launch_bounds__(256) k_pairs(DevSeries S, DevSearch Q, const i
   const int m = S.m, w = S.w;
   const int gib = threadIdx.x / G, g = threadIdx.x % G;
   const unsigned int gm = group_mask<G>();
-  const GroupLayout lay = group_layout(m, w, C, G, bounds);
-  float* base = sm + (size_t)gib * group_floats;
+  const WarpLayout lay = warp_layout(m, C);
+  float* base = sm + (size_t)gib * lay.total;
   float* q = base + lay.q_off;
   float* t = base + lay.t_off;
   float* cbc = base + lay.cb_off;
@@ -341,12 +318,9 @@ __global__ void __launch_bounds__(256) k_pairs(DevSeries S, DevSearch Q, const i
       kr = __shfl_sync(gm, kr, 0, G);
       // ---- cumulative bound for abandoning: LB_Keogh terms of the rows (q)
       // against the envelope of window j, summed over 8-row chunks, then
-      // suffix-summed over the chunks.  The group takes G consecutive rows
+      // suffix-summed over the chunks.  The warp takes 32 consecutive rows
       // at a time (coalesced envelope loads, conflict-free reads of q); the
-      // rows of a chunk sit in min(G, 8) consecutive lanes and are added by
-      // shuffles (two passes of four lanes when G = 4). ----
-      constexpr int kSeg = G < 8 ? G : 8;
-      float hold = 0.0f;
+      // rows of a chunk sit in 8 consecutive lanes and are added by shuffles. ----
       for (int k0 = 0; k0 < m; k0 += G) {
         const int k = k0 + g;
         float term = 0.0f;
@@ -360,17 +334,8 @@ __global__ void __launch_bounds__(256) k_pairs(DevSeries S, DevSearch Q, const i
           }
         }
 #pragma unroll
-        for (int o = 1; o < kSeg; o <<= 1) term += __shfl_xor_sync(gm, term, o, G);
-        if (kSeg == 8) {
-          if ((g & 7) == 0 && k < m) cbc[k >> 3] = term;
-        } else if (g == 0) {
-          if ((k0 & 4) == 0) {
-            hold = term;
-            if (k0 + 4 >= m) cbc[k0 >> 3] = hold;
-          } else {
-            cbc[k0 >> 3] = hold + term;
-          }
-        }
+        for (int o = 1; o < 8; o <<= 1) term += __shfl_xor_sync(gm, term, o, G);
+        if ((g & 7) == 0 && k < m) cbc[k >> 3] = term;
       }
       __syncwarp(gm);
       // lane g owns chunks [g per, g per + per): it suffix-sums its own from
@@ -411,7 +376,7 @@ __global__ void __launch_bounds__(256) k_pairs(DevSeries S, DevSearch Q, const i
     unsigned long long cells = 0;
     bool ab = false;
     const float d2 =
-        dtw_band<float, C, G, true, HI>(q, t, m, w, cbc, lay.nc, thr, bsf2, gm, g, &cells, &ab);
+        dtw_band<float, C, G, true>(q, t, m, w, cbc, lay.nc, thr, bsf2, gm, g, &cells, &ab);
     if (g == 0) {
       atomicAdd(&cnt[kDtwCalls], 1ull);
       atomicAdd(&cnt[kDtwCells], cells);
@@ -581,29 +546,21 @@ __global__ void k_best_f32(const Candidate* cands, const unsigned int* count_ptr
 
 // ---- dispatch ----
 
-template <int C, int G, int HI>
+template <int C>
 void run_pairs(const DevSeries& S, const DevSearch& Q, const int2* pairs,
                const unsigned int* npairs, int flags, int num_sms, cudaStream_t st,
                int warps) {
-  const bool bounds = flags & 1;
-  const GroupLayout lay = group_layout(S.m, S.w, C, G, bounds);
+  const WarpLayout lay = warp_layout(S.m, C);
   int threads = warps > 0 ? 32 * warps : 128;
-  if (threads < G) threads = G;
-  size_t bytes = (size_t)(threads / G) * lay.total * sizeof(float);
   // keep at least two blocks per SM when the series is long
-  while (bytes > 100 * 1024 && threads > G && threads > 32) {
+  while ((size_t)(threads / 32) * lay.total * sizeof(float) > 100 * 1024 && threads > 32)
     threads /= 2;
-    bytes /= 2;
-  }
-  const int gpb = threads / G;
-  bytes = (size_t)gpb * lay.total * sizeof(float);
-  cudaFuncSetAttribute(k_pairs<C, G, HI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       200 * 1024);
+  const size_t bytes = (size_t)(threads / 32) * lay.total * sizeof(float);
+  cudaFuncSetAttribute(k_pairs<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pairs<C, G, HI>, threads, bytes);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pairs<C>, threads, bytes);
   if (per_sm < 1) per_sm = 1;
-  k_pairs<C, G, HI><<<num_sms * per_sm, threads, bytes, st>>>(S, Q, pairs, npairs, flags,
-                                                              lay.total);
+  k_pairs<C><<<num_sms * per_sm, threads, bytes, st>>>(S, Q, pairs, npairs, flags);
 }
 
 // Elements of T that a pair of a list takes in shared memory.
@@ -787,7 +744,7 @@ void launch_pairs(const DevSeries& S, const DevSearch& Q, const int2* pairs,
 #define X(c, g) \
   if constexpr (g == 32) {                                                          \
     if (band.C == c) {                                                              \
-      run_pairs<c, g, -2>(S, Q, pairs, npairs, flags, num_sms, st, band.warps);      \
+      run_pairs<c>(S, Q, pairs, npairs, flags, num_sms, st, band.warps);             \
       return;                                                                       \
     }                                                                               \
   }
