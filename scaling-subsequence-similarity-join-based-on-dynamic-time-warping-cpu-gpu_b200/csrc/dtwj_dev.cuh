@@ -233,8 +233,8 @@ struct DevSearch {
   unsigned int* kq_count;
   unsigned int* kq_next;
   unsigned int kq_cap;
-  unsigned long long* low;      // [2] of this join: pairs well below the threshold that LB_Keogh
-                                //   tried all the same, those of them it pruned
+  unsigned int* low;            // [2] of this join: of the pairs well below the threshold, those
+                                //   LB_Keogh tried and counted, and those of them it pruned
 };
 
 __device__ __forceinline__ float max3f(float a, float b, float c) {
@@ -262,12 +262,22 @@ struct GroupFilter {
   unsigned int sup_cap, list_cap;
   const float* cut;      // seeds only: the cutoff on ED^2 ...
   unsigned int* walk;    // ... and whether the diagonals must be walked after all
-  unsigned int* off;     // nonzero: the bound settles nothing on this join, every tile is dense
-  unsigned int* probe;   // [3] zeroed words of launch_group_probe
+  unsigned int* probe;   // [2] sampled group pairs, those that survive (nullptr: none sampled)
   unsigned int* dense;   // tiles the diagonal sweep ran on
   unsigned int* ndense;
   int nib, nw;           // first-level work items per tile: blocks of row groups x column words
 };
+// Whether the bound settles too little to be worth its time on this join (every
+// tile is dense then): by the sample, more than one in `den` survivors of ED
+// pairs, 15/16 of the sweep's (a tile stays sparse at 7/8 or less, so hardly any
+// would).
+__device__ __forceinline__ bool group_off(const GroupFilter& F, bool ed, unsigned int den) {
+  if (!F.probe) return false;
+  return ed ? F.probe[1] * den > F.probe[0] : F.probe[1] * 16u > F.probe[0] * 15u;
+}
+// One group pair in 128 (g = 8) or 256 may survive a seed's cutoff (k_seed_exact's
+// budget); twice that in a sample is too many.
+__device__ __forceinline__ unsigned int seed_share(int g) { return g == 8 ? 64u : 128u; }
 // A super-group pair of a tile of the chunk: tile, row group relative to the
 // tile's first (at most 252), column group relative to row group + L0 / G (at
 // most 57).
@@ -431,8 +441,8 @@ void group_shape(int m, int64_t s, DevSeries* S);
 int launch_group_prep(const DevSeries& S, double* means, cudaStream_t st);
 // and returns the largest number of super-group pairs of one.
 size_t group_items(int g, GroupFilter* F);
-// Samples group pairs of the join's tiles against the best-so-far and sets *F.off
-// if nearly all survive.
+// Samples group pairs of the join's tiles against the best-so-far into F.probe
+// (zeroed).
 void launch_group_probe(const DevSeries& S, const DevSearch& Q, const GroupFilter& F,
                         const Tile* tiles, int ntiles, cudaStream_t st);
 // F.nsup, F.nlist and F.tcount are zero at launch.  Two kernels.

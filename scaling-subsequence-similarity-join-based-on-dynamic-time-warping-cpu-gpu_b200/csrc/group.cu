@@ -134,7 +134,10 @@ __global__ void __launch_bounds__(kThreads) k_group_super(DevSeries S, DevSearch
                                                           const Tile* tiles, unsigned int total) {
   const int lane = threadIdx.x & 31;
   const unsigned int item = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-  if (item >= total || *(ED ? F.walk : F.off) != 0u) return;
+  if (item >= total) return;
+  const unsigned int walk = ED ? *F.walk : 0u;
+  // (looked at behind the first records: a wait for it here costs 3 % of the pass)
+  const bool skip = group_off(F, ED, seed_share(S.grp_g)) | (walk != 0u);
   const unsigned int per = (unsigned int)(F.nib * F.nw);
   const unsigned int tk = item / per, rem = item - tk * per;
   const Tile T = tiles[tk];
@@ -190,7 +193,7 @@ __global__ void __launch_bounds__(kThreads) k_group_super(DevSeries S, DevSearch
 #pragma unroll
       for (int q = 0; q < kSupLaneCols; ++q)
         if (fb * fmaxf(a1[r][q], a2[r][q]) > thr) alive &= ~(1u << (r * kSupLaneCols + q));
-    if (!__any_sync(0xffffffffu, alive != 0u)) return;
+    if (skip || !__any_sync(0xffffffffu, alive != 0u)) return;
   }
 #pragma unroll
   for (int r = 0; r < 2; ++r)
@@ -268,16 +271,16 @@ __global__ void __launch_bounds__(kThreads) k_group(DevSeries S, DevSearch Q, Gr
 // levels are extra work (70,000 samples of noise, m = 512, w = 0: 7.6 ms with
 // them, 5.1 without), and the seeds' lists of group pairs overflow (100,003
 // samples, m = 256: 8.7 ms for the seeds, walking the diagonals takes 1.1).  A
-// sample of the pairs of the join's tiles, one per thread and spread over the
-// tiles, decides first: *flag is set if more than num / den of their group pairs
-// survive the threshold.  Pairs without a threshold yet don't count.
-constexpr int kProbeSamples = 8192;
+// sample of the pairs of the join's tiles, one per warp (a lane per segment) and
+// spread over the tiles, decides first (group_off).  Pairs without a threshold
+// yet don't count.
+constexpr int kProbeSamples = 1024;
 template <bool ED>
 __global__ void __launch_bounds__(kThreads) k_group_probe(DevSeries S, DevSearch Q, GroupFilter F,
-                                                          const Tile* tiles, int ntiles,
-                                                          unsigned int num, unsigned int den,
-                                                          unsigned int* flag) {
-  const unsigned int x = blockIdx.x * kThreads + threadIdx.x;
+                                                          const Tile* tiles, int ntiles) {
+  static_assert(kGrpSlots == 32, "a lane per slot");
+  const int lane = threadIdx.x & 31;
+  const unsigned int x = (blockIdx.x * kThreads + threadIdx.x) / 32;
   const Tile T = tiles[(unsigned long long)x * ntiles / kProbeSamples];
   unsigned int h = x * 0x9e3779b1u;  // a row and a lag of the tile
   h = (h ^ (h >> 15)) * 0x85ebca77u;
@@ -286,27 +289,20 @@ __global__ void __launch_bounds__(kThreads) k_group_probe(DevSeries S, DevSearch
   const int64_t i = T.i0 + row, j = i + T.L0 + lag;
   const float thr = ED ? *F.cut : prune_threshold_now(Q.bsf2 + T.series, S.m);
   const bool counts = j < T.send && thr < __int_as_float(0x7f800000);
-  bool alive = counts;
-  if (counts) {
-    const float4 *pi = S.grp + i / S.grp_g, *pj = S.grp + j / S.grp_g;
-    float a1 = 0.0f, a2 = 0.0f;
-    for (int s0 = 0; s0 < S.grp_d && alive; s0 += 4) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        group_terms<ED>(pi[(s0 + u) * S.grp_n], pj[(s0 + u) * S.grp_n], a1, a2);
-      alive = !((float)S.grp_b * fmaxf(a1, a2) > thr);
-    }
+  float a1 = 0.0f, a2 = 0.0f;
+  if (counts && lane < S.grp_d)
+    group_terms<ED>(S.grp[lane * S.grp_n + i / S.grp_g], S.grp[lane * S.grp_n + j / S.grp_g], a1,
+                    a2);
+  for (int o = 16; o > 0; o >>= 1) {
+    a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+    a2 += __shfl_xor_sync(0xffffffffu, a2, o);
   }
-  const int all = __syncthreads_count(counts), left = __syncthreads_count(alive);
+  const bool alive = !((float)S.grp_b * fmaxf(a1, a2) > thr);
+  const int all = __syncthreads_count(lane == 0 && counts);
+  const int left = __syncthreads_count(lane == 0 && counts && alive);
   if (threadIdx.x == 0) {
-    atomicAdd(&F.probe[0], (unsigned int)all);
-    atomicAdd(&F.probe[1], (unsigned int)left);
-    __threadfence();
-    if (atomicAdd(&F.probe[2], 1u) == gridDim.x - 1) {
-      __threadfence();
-      const unsigned int total = atomicAdd(&F.probe[0], 0u), kept = atomicAdd(&F.probe[1], 0u);
-      if (kept * den > total * num) *flag = 1u;
-    }
+    if (all) atomicAdd(&F.probe[0], (unsigned int)all);
+    if (left) atomicAdd(&F.probe[1], (unsigned int)left);
   }
 }
 
@@ -412,11 +408,9 @@ void run_group(const DevSeries& S, const DevSearch& Q, const GroupFilter& F, con
 }
 }  // namespace
 
-// 15/16: a tile stays sparse at 7/8 or less, so hardly any would.
 void launch_group_probe(const DevSeries& S, const DevSearch& Q, const GroupFilter& F,
                         const Tile* tiles, int ntiles, cudaStream_t st) {
-  k_group_probe<false><<<kProbeSamples / kThreads, kThreads, 0, st>>>(S, Q, F, tiles, ntiles, 15u,
-                                                                      16u, F.off);
+  k_group_probe<false><<<kProbeSamples / (kThreads / 32), kThreads, 0, st>>>(S, Q, F, tiles, ntiles);
 }
 
 void launch_group(const DevSeries& S, const DevSearch& Q, const GroupFilter& F, const Tile* tiles,
@@ -514,10 +508,14 @@ __global__ void __launch_bounds__(kThreads) k_seed_sample(DevSeries S, int64_t s
 // cut = the rank-th smallest of the count sampled values (lowest index on
 // ties), rounded up past the FP32 error of the bound.
 __global__ void __launch_bounds__(1024) k_seed_cut(const float* v, int count, int rank, float* cut) {
+  __shared__ float all[kSeedSamples];
+  for (int x = threadIdx.x; x < count; x += blockDim.x) all[x] = v[x];
+  __syncthreads();
   for (int x = threadIdx.x; x < count; x += blockDim.x) {
-    const float mine = v[x];
+    const float mine = all[x];
     int below = 0;
-    for (int y = 0; y < count; ++y) below += v[y] < mine || (v[y] == mine && y < x) ? 1 : 0;
+#pragma unroll 8
+    for (int y = 0; y < count; ++y) below += all[y] < mine || (all[y] == mine && y < x) ? 1 : 0;
     if (below == rank) *cut = mine * (1.0f + 1.0f / 4096.0f) + 1e-6f;
   }
 }
@@ -531,9 +529,8 @@ __global__ void __launch_bounds__(kThreads) k_seed_exact(DevSeries S, GroupFilte
                                                          unsigned long long* keys) {
   const int lane = threadIdx.x & 31;
   const unsigned int total = *F.nlist;
-  if (*F.walk != 0u) return;
   // too many group pairs, or some were dropped: the diagonals are walked instead
-  if (total > F.list_cap || *F.nsup > F.sup_cap || *F.tcount > budget) {
+  if (group_off(F, true, seed_share(G)) || total > F.list_cap || *F.nsup > F.sup_cap || *F.tcount > budget) {
     if (blockIdx.x == 0 && threadIdx.x == 0) *F.walk = 1u;
     return;
   }
@@ -590,7 +587,7 @@ void launch_seed_groups(const DevSeries& S, GroupFilter F, const Tile* tiles, in
                         int world, float* samples, unsigned long long* keys, int num_sms,
                         cudaStream_t st) {
   cudaMemsetAsync(keys, 0xff, (size_t)S.s * 8, st);
-  cudaMemsetAsync(F.walk, 0, 16, st);  // and the words of the probe
+  cudaMemsetAsync(F.walk, 0, 12, st);  // and the probe's two words
   // one row group in `stride`, at most kSeedSamples; the rank that should
   // leave 4 kSeeds grid rows (of this shard) below the cutoff, at least 4 deep
   const int64_t ng = (S.s + S.grp_g - 1) / S.grp_g, rows = (S.s + kSeedGrid - 1) / kSeedGrid;
@@ -602,10 +599,8 @@ void launch_seed_groups(const DevSeries& S, GroupFilter F, const Tile* tiles, in
   if (rank > count - 1) rank = count - 1;
   k_seed_sample<<<count, kThreads, 0, st>>>(S, stride, samples);
   k_seed_cut<<<1, 1024, 0, st>>>(samples, count, (int)rank, const_cast<float*>(F.cut));
-  // one group pair in 128 (g = 8) or 256 may survive (the budget below); twice that
-  // in a sample is too many
-  k_group_probe<true><<<kProbeSamples / kThreads, kThreads, 0, st>>>(
-      S, DevSearch{}, F, tiles, ntiles, 1u, S.grp_g == 8 ? 64u : 128u, F.walk);
+  k_group_probe<true><<<kProbeSamples / (kThreads / 32), kThreads, 0, st>>>(S, DevSearch{}, F,
+                                                                            tiles, ntiles);
   for (int b = 0; b < ntiles; b += kSeedSlab) {
     const int cnt = ntiles - b < kSeedSlab ? ntiles - b : kSeedSlab;
     cudaMemsetAsync(F.nsup, 0, 12, st);  // nsup, nlist and the group pair count

@@ -57,7 +57,7 @@ constexpr int kResweepTiles = 32;
 // 0.62 against 0.56.
 constexpr int kSeedGroupTiles = 1024;
 // Tiles from which a sample decides whether the sweep uses the group bound at all
-// (4 us; the smallest such join takes about 1 ms).
+// (9 us; such a join of a random walk takes 1 ms and more).
 constexpr int kProbeTiles = 256;
 // Their lists of group pairs, and with the samples and five words the bytes
 // they take.
@@ -130,8 +130,8 @@ __global__ void k_chunk_note(int* status, const unsigned long long* counters, Ch
 // counters, candidates and the seeds' work counter zero.
 __global__ void k_init_search(unsigned int* bsf2, int nslots, unsigned long long* counters,
                               unsigned int* cand_count, unsigned int* nseeds, int nseries,
-                              int seed_slots, unsigned int* zready, unsigned long long* low,
-                              unsigned int* group_off) {
+                              int seed_slots, unsigned int* zready, unsigned int* low,
+                              unsigned int* probe) {
   for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < nslots; x += gridDim.x * blockDim.x)
     bsf2[x] = 0x7f800000u;
   if (blockIdx.x == 0) {
@@ -141,8 +141,9 @@ __global__ void k_init_search(unsigned int* bsf2, int nslots, unsigned long long
       nseeds[nseries] = (unsigned int)seed_slots;
       nseeds[nseries + 1] = 0u;
       zready[0] = zready[1] = 0u;  // the window table: not filled
-      low[0] = low[1] = 0ull;
-      group_off[0] = group_off[1] = group_off[2] = group_off[3] = 0u;
+      low[0] = 64u;  // 43 pruned before all are tried
+      low[1] = 0u;
+      probe[0] = probe[1] = 0u;
     }
   }
 }
@@ -650,7 +651,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
   const bool want_keys = nlb > 0 && (tile_mode || want_features || !(flags & DTWJ_F_NO_SEED));
   // counters of a chunk, then the group filter's surviving group pairs per tile
   constexpr int kQcTiles = 16;
-  unsigned int *qc, *nseeds, *bits;  // nseeds: [nseries] counts, total slots, work counter
+  unsigned int *qc, *nseeds, *bits, *probe;  // nseeds: [nseries] counts, total slots, work counter
   unsigned long long* keys;          // row minima of the ED profile
   int2* seeds;
   ChunkNote* notes;
@@ -670,8 +671,8 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
       A.add(&F.dense, (size_t)chunk_max * 4);
       A.add(&Q.bsf2, (size_t)nslots * 4);
       A.add(&S.zready, 8);
-      A.add(&Q.low, 16);
-      A.add(&F.off, 16);
+      A.add(&Q.low, 8);
+      A.add(&probe, 8);
       A.add(&seeds, (size_t)nseries * kSeedSlots * sizeof(int2));
       A.add(&nseeds, ((size_t)nseries + 2) * 4);
       A.add(&notes, (ranges.size() + 1) * sizeof(ChunkNote));
@@ -732,8 +733,8 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     if (S.grp) F.tcount = qc + kQcTiles;
     k_init_search<<<(nslots + 255) / 256 < 256 ? (nslots + 255) / 256 : 256, 256, 0, st>>>(
         Q.bsf2, nslots, Q.counters, Q.cand_count, nseeds, nseries, nseries * kSeedSlots, S.zready,
-        Q.low, F.off);
-    F.probe = F.off + 1;
+        Q.low, probe);
+    if (S.grp && nlb >= kProbeTiles) F.probe = probe;
   }
 
   // ---- ED matrix profile (row minima; per tile for the tile minima) ----
@@ -766,7 +767,7 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
       E.tcount = word + 2;
       E.walk = word + 3;
       E.probe = word + 4;
-      E.cut = reinterpret_cast<const float*>(word + 7);
+      E.cut = reinterpret_cast<const float*>(word + 6);
       launch_seed_groups(S, E, lbtiles, nlb, ctx->shard_world, samples, keys, ctx->num_sms, st);
       launch_mp_seed(S, lbtiles, nlb, keys, E.walk, ctx->num_sms, st);
       launches = 4 + 3 * ((nlb + kSeedSlab - 1) / kSeedSlab);
@@ -827,9 +828,8 @@ int run_join(dtwj_ctx* ctx, const double* x_dev, int64_t n, const int64_t* sbeg,
     Qs.queue_next = nseeds + nseries + 1;
     Qs.queue_cap = (unsigned int)(nseries * kSeedSlots);
     launch_pairs(S, Qs, seeds, nseeds + nseries, false, wide, ctx->num_sms, st);
-    const bool probe = S.grp && nlb >= kProbeTiles;
-    if (probe) launch_group_probe(S, Q, F, lbtiles, nlb, st);
-    ph.end(DTWJ_PHASE_SEEDS, probe ? 3 : 2);
+    if (F.probe) launch_group_probe(S, Q, F, lbtiles, nlb, st);
+    ph.end(DTWJ_PHASE_SEEDS, F.probe ? 3 : 2);
   }
   CUDA_OK(cudaMemcpyAsync(seed_bsf, Q.bsf2, (size_t)nslots * 4, cudaMemcpyDeviceToDevice, st));
 

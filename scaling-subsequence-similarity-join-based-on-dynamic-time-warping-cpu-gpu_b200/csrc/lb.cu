@@ -224,6 +224,7 @@ __global__ void __launch_bounds__(kLbThreads, kLbCtasPerSm) k_lb(DevSeries S, De
   const int lane = threadIdx.x & 31;
   unsigned int npairs = 0, nfast = 0;
   unsigned long long sparse = 0;
+  const bool grouped = F.tcount && !group_off(F, false, 0u);
   for (;;) {
     __syncthreads();  // every thread has read tile_idx and left the previous tile's staging
     if (threadIdx.x == 0) tile_idx = atomicAdd(next, 1u);
@@ -232,7 +233,7 @@ __global__ void __launch_bounds__(kLbThreads, kLbCtasPerSm) k_lb(DevSeries S, De
     if (k >= (unsigned int)ntiles) break;
     const Tile T = tiles[k];
     unsigned int* out = bits + (size_t)k * kLbLags * kLbWords;
-    if (F.tcount && *F.off == 0u && !group_tile_dense(T, S.grp_g, F.tcount[k])) {
+    if (grouped && !group_tile_dense(T, S.grp_g, F.tcount[k])) {
       if (threadIdx.x == 0) sparse += (unsigned long long)tile_pairs(T);
       if (clear_sparse)
         for (int x = threadIdx.x; x < kLbLags * kLbWords; x += kLbThreads) out[x] = 0u;

@@ -33,9 +33,9 @@ constexpr int kRunWarps = 4;
 constexpr int kKeoghCheck = 128;  // samples between two best-so-far checks of LB_Keogh
 constexpr int kKeoghWarps = 8;    // warps per block of the LB_Keogh kernel
 constexpr int kKeoghBatch = 8;    // entries a warp prepares at once for the exact bound
-// In a long queue, every kLowEvery-th batch tries the exact bound also on the
-// pairs well below the threshold (k_keogh).
-constexpr unsigned int kLowEvery = 256;
+// In a long queue, every kLowEvery-th batch tries the exact bound also on one of
+// its pairs well below the threshold (k_keogh); a join counts kLowMany of them.
+constexpr unsigned int kLowEvery = 16, kLowMany = 1u << 24;
 
 // Masked bound for env = r, query = c from the raw FP64 sums
 // F1 = sum_T M_r a_c, F2 = sum_T M_r a_c^2, F3 = sum_T M_r E_r a_c.
@@ -398,8 +398,8 @@ __device__ __forceinline__ float warp_sum4(const float (&v)[4], int lane) {
 // On noise the blocks average the difference away and the exact bound prunes
 // what they leave far below: a series that is half a walk, half noise (30,007
 // samples, m = 700, w = 20) sent 18.5 million pairs to DTW instead of 8.8 and took
-// 147 ms instead of 94.  So some of the low pairs are tried all the time, and
-// while more than two thirds of those tried are pruned, all are: 86 ms.  The
+// 147 ms instead of 94.  So in long queues some of the low pairs are tried all the
+// time, and while more than two thirds of those tried are pruned, all are: 86 ms.  The
 // share is 0.86 to 1 on such series, 0.44 where skipping still wins (60,000
 // samples, m = 1024), 0.08 to 0.42 on walks and below 0.14 on ECG-like ones.
 //
@@ -412,6 +412,7 @@ __global__ void __launch_bounds__(kKeoghWarps * 32, 5) k_keogh(DevSeries S, DevS
   __shared__ KeoghSide side[kKeoghWarps][kKeoghBatch][2];
   __shared__ float endsv[kKeoghWarps][kKeoghBatch][2];
   __shared__ float errv[kKeoghWarps][kKeoghBatch];  // FP32 error scale of the pair
+  __shared__ unsigned int lowv[kKeoghWarps];
   __shared__ unsigned long long pruned_block;
   if (threadIdx.x == 0) pruned_block = 0;
   __syncthreads();
@@ -423,25 +424,17 @@ __global__ void __launch_bounds__(kKeoghWarps * 32, 5) k_keogh(DevSeries S, DevS
   const int F = S.paa_b / 4, kb = (kBias + F - 1) / F, ke = (S.m - kBias) / F;
   const float skip = !S.zt ? 0.5f : (S.m >= 192 ? 0.8f : 0.6f);
   unsigned long long pruned = 0;
-  unsigned int tried = 0, hits = 0;  // low pairs tried all the same, those pruned (lane 0)
   for (;;) {
     unsigned int idx = 0;
-    bool always = false;  // the exact bound for low pairs too
-    if (lane == 0) {
-      idx = atomicAdd(Q.kq_next, batch);
-      const volatile unsigned long long* low = Q.low;
-      always = 3ull * low[1] > 2ull * low[0];
-    }
+    if (lane == 0) idx = atomicAdd(Q.kq_next, batch);
     idx = __shfl_sync(0xffffffffu, idx, 0);
     if (idx >= total) break;
-    const bool probe = batch == 32u && idx / 32u % kLowEvery == kLowEvery - 1u;
-    always = __any_sync(0xffffffffu, always) || probe;
     const int cnt = total - idx < batch ? (int)(total - idx) : (int)batch;
     // lane e holds entry e of the batch
     const int4 r = Q.kq[idx + (lane < cnt ? lane : cnt - 1)];
     const float thr_e = prune_threshold_now(Q.bsf2 + r.w, S.m);
     const unsigned int all = cnt == 32 ? 0xffffffffu : (1u << cnt) - 1u;
-    unsigned int alive = all, exact = all, below = 0;  // below: of the low pairs
+    unsigned int alive = all, exact = all;
     if (S.fq) {
       const float4 wx = S.wrec[r.x], wy = S.wrec[r.y];
       const float o_e = (float)(__hiloint2double(__float_as_int(wx.y), __float_as_int(wx.x)) -
@@ -477,10 +470,17 @@ __global__ void __launch_bounds__(kKeoghWarps * 32, 5) k_keogh(DevSeries S, DevS
         dead = (dead & 1u) | (dead >> 7 & 2u) | (dead >> 14 & 4u) | (dead >> 21 & 8u);
         low = (low & 1u) | (low >> 7 & 2u) | (low >> 14 & 4u) | (low >> 21 & 8u);
         alive &= ~(dead << e0);
-        exact &= ~(dead << e0);
-        below |= (low & ~dead) << e0;
+        exact &= ~((dead | low) << e0);
       }
-      if (!always) exact &= ~below;
+      if (batch == 32u) {
+        // the low pairs that are tried all the same: all, one or none
+        unsigned int low = alive & ~exact;
+        const volatile unsigned int* stat = Q.low;
+        if (!(3u * stat[1] > 2u * stat[0]))
+          low = idx / 32u % kLowEvery == 0u ? low & (0u - low) : 0u;
+        exact |= low;
+        if (lane == 0) lowv[warp] = low;
+      }
     }
     while (exact) {
       // the next (up to) eight entries; lane (q, d) owns window d of the q-th
@@ -538,13 +538,12 @@ __global__ void __launch_bounds__(kKeoghWarps * 32, 5) k_keogh(DevSeries S, DevS
       }
     }
     if (lane == 0) pruned += (unsigned long long)(cnt - __popc(alive));
-    if (lane == 0 && always && below) {
-      tried += __popc(below);
-      hits += __popc(below & ~alive);
-      if (tried >= 256u || probe) {
-        atomicAdd(&Q.low[0], (unsigned long long)tried);
-        if (hits) atomicAdd(&Q.low[1], (unsigned long long)hits);
-        tried = hits = 0;
+    if (batch == 32u && idx / 32u % kLowEvery == 0u && lane == 0 && S.fq) {
+      // the first of them counts
+      const unsigned int low = lowv[warp];
+      if (low && Q.low[0] < kLowMany) {
+        atomicAdd(&Q.low[0], 1u);
+        if (low & (0u - low) & ~alive) atomicAdd(&Q.low[1], 1u);
       }
     }
     if (alive) {
