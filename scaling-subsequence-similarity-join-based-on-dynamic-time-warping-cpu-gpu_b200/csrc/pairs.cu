@@ -260,7 +260,8 @@ __device__ T dtw_band(const T* __restrict__ q, const T* __restrict__ t, int m, i
 // seeds).
 template <int C>
 __global__ void __launch_bounds__(256) k_pairs(DevSeries S, DevSearch Q, const int2* pairs,
-                                                const unsigned int* npairs, int flags) {
+                                                const unsigned int* npairs, int flags,
+                                                int warp_floats) {
   constexpr int G = 32;
   extern __shared__ __align__(16) unsigned char smraw[];
   float* sm = reinterpret_cast<float*>(smraw);
@@ -270,7 +271,7 @@ __global__ void __launch_bounds__(256) k_pairs(DevSeries S, DevSearch Q, const i
   const int gib = threadIdx.x / G, g = threadIdx.x % G;
   const unsigned int gm = group_mask<G>();
   const WarpLayout lay = warp_layout(m, C);
-  float* base = sm + (size_t)gib * lay.total;
+  float* base = sm + (size_t)gib * warp_floats;
   float* q = base + lay.q_off;
   float* t = base + lay.t_off;
   float* cbc = base + lay.cb_off;
@@ -560,7 +561,7 @@ void run_pairs(const DevSeries& S, const DevSearch& Q, const int2* pairs,
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pairs<C>, threads, bytes);
   if (per_sm < 1) per_sm = 1;
-  k_pairs<C><<<num_sms * per_sm, threads, bytes, st>>>(S, Q, pairs, npairs, flags);
+  k_pairs<C><<<num_sms * per_sm, threads, bytes, st>>>(S, Q, pairs, npairs, flags, lay.total);
 }
 
 // Elements of T that a pair of a list takes in shared memory.
