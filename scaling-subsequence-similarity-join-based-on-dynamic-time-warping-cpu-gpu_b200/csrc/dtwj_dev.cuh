@@ -163,7 +163,7 @@ struct DevSeries {
   float* MDUL2;     // s, sum_m M (nU - nL)^2
   float* MDUL;      // s
   double* SM;       // s, sum_T M            (T = [kBias, m-1-kBias])
-  double* SME;      // s, sum_T M E
+  double* SME;      // s, sum_T M (E - 2 mu)
   double* cb;       // (n >> kBlkShift) + 2, block centers
   float* af;        // n, a - cb[block]
   float2* ulf;      // n, (U - cb[block], L - cb[block])

@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kThreads) k_rowterms(DevSeries S) {
         if (k >= kBias && k <= m - 1 - kBias) {
           MN += M * (u * u + l * l);
           SM += M;
-          SME += M * (U + L);
+          SME += M * ((U - mu) + (L - mu));
         }
         MD2 += M * (u - l) * (u - l);
       }

@@ -37,14 +37,15 @@ constexpr int kKeoghBatch = 8;    // entries a warp prepares at once for the exa
 // its pairs well below the threshold (k_keogh); a join counts kLowMany of them.
 constexpr unsigned int kLowEvery = 16, kLowMany = 1u << 24;
 
-// Masked bound for env = r, query = c from the raw FP64 sums
-// F1 = sum_T M_r a_c, F2 = sum_T M_r a_c^2, F3 = sum_T M_r E_r a_c.
-__device__ inline double masked_lb(const DevSeries& S, int64_t r, int64_t c, double F1,
-                                   double F2, double F3) {
-  const double mr = S.mu[r], mc = S.mu[c], ir = S.isg[r], ic = S.isg[c];
-  const double SM = S.SM[r];
-  const double mnorm = (F2 - 2.0 * mc * F1 + mc * mc * SM) * ic * ic;
-  const double t = (F3 - 2.0 * mr * F1 - mc * S.SME[r] + 2.0 * mr * mc * SM) * ir * ic;
+// Masked bound for env = r, query = c from the FP64 sums
+// F1 = sum_T M_r a_c, F2 = sum_T M_r a_c^2, F3 = sum_T M_r E_r a_c, with a_c less
+// kc and E_r less 2 kr.  kr and kc are means near the windows': of samples as they
+// are, the sums cancel to nothing on a high level (a walk on 1e9 lost its pair).
+__device__ inline double masked_lb(const DevSeries& S, int64_t r, int64_t c, double kr, double kc,
+                                   double F1, double F2, double F3) {
+  const double mr = S.mu[r] - kr, mc = S.mu[c] - kc, ir = S.isg[r], ic = S.isg[c];
+  const double mnorm = (F2 - 2.0 * mc * F1 + mc * mc * S.SM[r]) * ic * ic;
+  const double t = (F3 - 2.0 * mr * F1 - mc * S.SME[r]) * ir * ic;
   const double dist = 2.0 * mnorm - 2.0 * t + (double)S.MN[r];
   const double d2 = (double)S.MDUL2[r];
   if (dist < d2) return 0.0;
@@ -267,16 +268,17 @@ __global__ void __launch_bounds__(kRunWarps * 32, 8) k_runs(DevSeries S, DevSear
         float thr = prune_threshold_now(bsf2, S.m);
         // ---- masked sums at the run's first pair (exact, FP64) ----
         double F1 = 0, F2 = 0, F3 = 0, R1 = 0, R2 = 0, R3 = 0;
+        const double ki = S.mu[i0], kj = S.mu[j0];
         if (masked) {
           for (int k = lo + lane; k <= hi; k += 32) {
-            const double ai = S.a[i0 + k], aj = S.a[j0 + k];
+            const double ai = S.a[i0 + k] - ki, aj = S.a[j0 + k] - kj;
             const double Mi = S.mask[i0 + k], Mj = S.mask[j0 + k];
             F1 = fma(Mi, aj, F1);
             F2 = fma(Mi * aj, aj, F2);
-            F3 = fma(Mi * S.E[i0 + k], aj, F3);
+            F3 = fma(Mi * (S.E[i0 + k] - 2.0 * ki), aj, F3);
             R1 = fma(Mj, ai, R1);
             R2 = fma(Mj * ai, ai, R2);
-            R3 = fma(Mj * S.E[j0 + k], ai, R3);
+            R3 = fma(Mj * (S.E[j0 + k] - 2.0 * kj), ai, R3);
           }
           F1 = warp_sum(F1);
           F2 = warp_sum(F2);
@@ -297,18 +299,21 @@ __global__ void __launch_bounds__(kRunWarps * 32, 8) k_runs(DevSeries S, DevSear
             if (valid && p > 0) {
               const int64_t io = i - 1 + lo, in = i + hi, jo = j - 1 + lo, jn = j + hi;
               const double Mio = S.mask[io], Min = S.mask[in], Mjo = S.mask[jo], Mjn = S.mask[jn];
-              const double ajo = S.a[jo], ajn = S.a[jn], aio = S.a[io], ain = S.a[in];
+              const double ajo = S.a[jo] - kj, ajn = S.a[jn] - kj;
+              const double aio = S.a[io] - ki, ain = S.a[in] - ki;
               d1 = Min * ajn - Mio * ajo;
               d2 = Min * ajn * ajn - Mio * ajo * ajo;
-              d3 = Min * S.E[in] * ajn - Mio * S.E[io] * ajo;
+              d3 = Min * (S.E[in] - 2.0 * ki) * ajn - Mio * (S.E[io] - 2.0 * ki) * ajo;
               e1 = Mjn * ain - Mjo * aio;
               e2 = Mjn * ain * ain - Mjo * aio * aio;
-              e3 = Mjn * S.E[jn] * ain - Mjo * S.E[jo] * aio;
+              e3 = Mjn * (S.E[jn] - 2.0 * kj) * ain - Mjo * (S.E[jo] - 2.0 * kj) * aio;
             }
             const double f1 = F1 + warp_iscan(d1, lane), f2 = F2 + warp_iscan(d2, lane);
             const double f3 = F3 + warp_iscan(d3, lane), r1 = R1 + warp_iscan(e1, lane);
             const double r2 = R2 + warp_iscan(e2, lane), r3 = R3 + warp_iscan(e3, lane);
-            if (valid) lbm = fmax(masked_lb(S, i, j, f1, f2, f3), masked_lb(S, j, i, r1, r2, r3));
+            if (valid)
+              lbm = fmax(masked_lb(S, i, j, ki, kj, f1, f2, f3),
+                         masked_lb(S, j, i, kj, ki, r1, r2, r3));
             F1 = __shfl_sync(0xffffffffu, f1, 31);
             F2 = __shfl_sync(0xffffffffu, f2, 31);
             F3 = __shfl_sync(0xffffffffu, f3, 31);

@@ -40,3 +40,16 @@ def test_join_of_small_deviations_on_a_high_level(gpu_dtwj, oracle):
                 r = ctx.join(x, M, 0, fl)
                 assert (r.i, r.j) == (ref.i, ref.j), (chunk, fl)
                 assert abs(r.dist - ref.dist) <= 1e-5 * ref.dist, (chunk, fl)
+
+
+@pytest.mark.parametrize("level", [2.0 ** 20, 2.0 ** 30, 2.0 ** 36])
+@pytest.mark.parametrize("n,m,w", [(2504, 200, 0), (3000, 64, 3), (5000, 256, 13)])
+def test_join_does_not_depend_on_the_level(gpu_dtwj, oracle, synth, level, n, m, w):
+    # samples on a grid of 2^-10, so that a level of up to 2^36 is added exactly
+    x = np.round(synth.random_walk(n, n + m) * 1024.0) / 1024.0
+    ref = oracle.join(x, m, w)
+    with gpu_dtwj.Context() as ctx:
+        for fl in (0, gpu_dtwj.F_MASKED_CASCADE, gpu_dtwj.F_MASKED_CASCADE | gpu_dtwj.F_NO_SEED):
+            r = ctx.join(x + level, m, w, fl)
+            assert (r.i, r.j) == (ref.i, ref.j), fl
+            assert abs(r.dist - ref.dist) <= 1e-5 * ref.dist, fl
