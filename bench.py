@@ -131,10 +131,10 @@ def sweep_tiles(n: int, m: int):
 
 
 def launch_traffic(tfile: str, kname: str, tiles_per_launch: float):
-    """DRAM bytes per launch of a sweep kernel: the ncu capture of one launch
-    over a full chunk (profiles/ncu_traffic_rw1m_motif.json, its "tiles"
-    field), scaled to this run's average tiles per launch, since each tile
-    moves the same bytes.  None without a capture."""
+    """DRAM bytes per launch of a sweep stage: the ncu capture of one chunk
+    (profiles/ncu_traffic_rw1m_groups.json: the stage's launches together, and
+    the chunk's "tiles"), scaled to this run's average tiles per launch.
+    None without a capture."""
     if not os.path.exists(tfile):
         return None
     with open(tfile) as f:
@@ -446,8 +446,8 @@ def run_ours(args):
     per_launch_s = phases[roof_phase] / nl
     achieved_gbs = alg_bytes / max(phases[roof_phase], 1e-12) / 1e9
     traffic = None
-    if args.workload == "rw1m_motif" and kname in ("k_lb", "k_paa"):  # (what was captured)
-        traffic = launch_traffic(os.path.join(ROOT, "profiles", "ncu_traffic_rw1m_motif.json"),
+    if args.workload == "rw1m_motif" and not args.petitjean:  # (what was captured)
+        traffic = launch_traffic(os.path.join(ROOT, "profiles", "ncu_traffic_rw1m_groups.json"),
                                  kname, ntiles / nl)
     cells_per_s = r0.dtw_cells / max(phases.get("pairs", 1e-12) + phases.get("seeds", 0), 1e-12)
 

@@ -33,3 +33,13 @@ def test_launch_traffic_scales_the_capture_by_tiles(tmp_path):
     # the bench workload's tiles over its launches: 1M samples, m = 1024
     ntiles, _ = bench.sweep_tiles(1_000_000, 1024)
     assert 1024 * 100 < ntiles < 1776 * 100
+
+
+def test_every_sweep_stage_has_a_capture():
+    path = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "profiles",
+                        "ncu_traffic_rw1m_groups.json")
+    for k in ("k_group", "k_paa_groups", "k_keogh"):
+        whole = bench.launch_traffic(path, k, 1776)
+        assert whole > 0
+        # the group stage's three launches share the chunk's tiles
+        assert abs(3 * bench.launch_traffic(path, k, 1776 / 3) - whole) < 1e-6 * whole
