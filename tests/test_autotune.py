@@ -70,3 +70,38 @@ def test_tune_join_searches_each_knob_and_caches(tmp_path):
     calls.clear()
     assert at.tune_join(None, 256, 13, path, measure=measure, shapes=shapes) == saved[at.join_key(256, 13)]
     assert not calls
+
+
+def test_tune_join_times_a_replayed_join(monkeypatch):
+    at = _autotune()
+    joins = []
+
+    class FakeContext:
+        """Joins as a context does: direct, capturing, replayed."""
+
+        def __init__(self, device):
+            self.n = 0
+
+        def __enter__(self):
+            return self
+
+        def __exit__(self, *exc):
+            joins.append(self.n)
+
+        def set_band(self, w, C, G):
+            self.band = (C, G)
+
+        def set_tuning(self, warps, chunk):
+            pass
+
+        def join(self, series, m, w, flags=0):
+            self.n += 1
+            r = type("R", (), {})()
+            # the capture takes the wider layout longer; replayed, it is the faster one
+            r.seconds_join = 1.0 / self.band[1] if self.n > 2 else float(self.band[1])
+            return r
+
+    monkeypatch.setattr(at, "Context", FakeContext)
+    e = at.tune_join(None, 256, 13, None, shapes=lambda w: [(7, 4), (2, 32)])
+    assert (e["C"], e["G"]) == (2, 32)
+    assert set(joins) == {3}
