@@ -63,12 +63,17 @@ extern "C" {
 #define DTWJ_F_NO_SEED 0x2u     /* no ED-profile seeding of the best-so-far   */
 #define DTWJ_F_NO_DIAG 0x4u     /* skip all diagonal bounds (LB_Keogh + DTW)  */
 #define DTWJ_F_LEARNED 0x8u     /* sweep tiles in the order the context's MLP
-                                   scores them (dtwj_ctx_set_model)           */
+                                   scores them (dtwj_ctx_set_model).  Their
+                                   features need a walk over every diagonal that
+                                   a plain join of 100,000 samples and more does
+                                   without: slower there (1M samples: 0.20 s
+                                   against 0.11)                              */
 #define DTWJ_F_VERBOSE 0x10u    /* phase timings on stderr                    */
 #define DTWJ_F_PROFILE 0x20u    /* per-phase device times (CUDA events)       */
 #define DTWJ_F_NO_GRAPH 0x40u   /* launch the sweep directly, not as a CUDA graph
-                                   (by default a context captures the sweep once and
-                                   replays it while its launches are unchanged) */
+                                   (by default a context captures the sweep on its
+                                   second join of a shape and replays it while its
+                                   launches are unchanged)                    */
 #define DTWJ_F_MASKED_CASCADE 0x80u /* run filter = the reference's masked diagonal
                                    bound and endpoint bound (diag_mask_global,
                                    CPU_version1/diag_mask_global.cpp:11-311) on
@@ -148,10 +153,11 @@ int dtwj_ctx_join_device(dtwj_ctx* ctx, const double* x_dev, int64_t n, int32_t 
  * CPU_version1/mpx_v2.cpp:13): mp[i] = min over |i-j| >= m, mpi[i] its
  * 0-based argmin (lowest index on ties; -1 and +inf when none).  mp, mpi
  * hold s = n - m + 1 entries.  The FP64 recurrence finds each row's minimum
- * to about 2^-17 relative; every partner within about 2^-16 of it is then
- * measured directly in FP64, and the row takes the smallest (lowest partner
- * on ties).  DTWJ_ERR_OVERFLOW if those near-minimal partners average more
- * than 16 per row (a series of many near-identical windows). */
+ * to about 2^-20 relative; every partner within about 2^-17 of it, and near
+ * zero within the recurrence's rounding, is then measured directly in FP64, and
+ * the row takes the smallest (lowest partner on ties).  Where those near-minimal
+ * partners average more than 16 per row (a series of many near-identical
+ * windows) they are collected in pieces, which takes longer. */
 int dtwj_matrix_profile(const double* x, int64_t n, int32_t m, double* mp, int64_t* mpi);
 
 /* The global CDF mask of the masked diagonal bound (compute_shared_data_global

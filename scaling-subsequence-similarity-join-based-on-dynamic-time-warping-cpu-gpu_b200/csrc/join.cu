@@ -38,12 +38,12 @@ namespace {
 constexpr unsigned int kCandCap = 1u << 20;
 constexpr unsigned int kQueueCapMax = 1u << 26;
 // Default tiles per chunk of the sweep: kLbChunkRounds tiles for each of the
-// diagonal sweep's resident CTAs.  Its tiles take about the same time, so a
-// chunk that is not a whole number of rounds leaves CTAs idle in its last
-// round (1024 tiles on 444 CTAs: 2.3 rounds, the last one 31 % busy).  On
-// the 1M-sample bench series 4 rounds (1776 tiles) measured best: 0.973 s
-// per join against 0.998 s at 3 rounds, 0.980 s at 5, 0.985 s at 6 and
-// 1.008 s at 1024 tiles.
+// diagonal sweep's resident CTAs, chosen when that bound ran on every tile (1M
+// bench series: 0.973 s per join at 4 rounds, 0.998 at 3, 0.980 at 5).  Tiles
+// that the group bound leaves sparse skip it, and each stage's tail is then what
+// a chunk costs: 157 ms at 444 tiles, 136 at 888, 119 at 1332, 112 at 1776, 103
+// at 2664, 97 at 4096 (dtwj_ctx_set_tuning).  The survivor bits, 451 KB for every
+// tile of a chunk, are what larger chunks cost.
 constexpr int kLbChunkRounds = 4;
 // Largest piece an overflowing chunk is swept again in.  Every piece that
 // overflows again wastes a full DTW queue of work.  On the 262,144-sample

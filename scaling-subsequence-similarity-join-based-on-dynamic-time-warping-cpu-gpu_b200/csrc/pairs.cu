@@ -710,8 +710,11 @@ bool choose_band_join(int m, int w, BandShape* out) {
   // holds, so a narrow band takes few lanes with several cells each.  DTW
   // stage of ECG-like joins, (cells, lanes): w = 20 (6, 8) 9.2 ms, (3, 16)
   // 16.1; w = 13 (4, 8) 13.3, (2, 16) 29.0, (7, 4) 18.7; w = 7 (4, 4) 10.8,
-  // (2, 8) 13.5; w = 52 (7, 16) 150, one pair per warp (4, 32) 224.  A warp's
-  // windows must leave room for about 11 warps per SM.
+  // (2, 8) 13.5; w = 52 (7, 16) 150, one pair per warp (4, 32) 224.  Pairs that
+  // abandon early gain less from slots, whose preparation stalls their warp: random
+  // walks at m = 1024, w = 52 take 13 to 17 % less with (4, 32) at 1M (21.5 against
+  // 17.9 to 18.6 ms) and 300k, ECG-like ones 33 % more.  A warp's windows must leave
+  // room for about 11 warps per SM.
   const int first = w <= 7 ? 4 : (w <= 27 ? 8 : 16);
   for (int G = first; G <= 16; G *= 2) {
     const int C = slot_cells(w, G);

@@ -91,7 +91,6 @@ __device__ __forceinline__ double warp_iscan(double v, int lane) {
   return v;
 }
 
-// max(a, b, c) in one instruction (three-input max.f32, sm_100).
 // Adds one LB_Keogh term: query sample a (block-centered, scale sq, offset o
 // = query block offset - envelope block offset, both already scaled) against
 // the block-centered envelope ul = (U, L) (scale se).  With q = a sq + o,
