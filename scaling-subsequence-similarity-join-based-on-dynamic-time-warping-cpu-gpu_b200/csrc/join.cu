@@ -56,9 +56,10 @@ constexpr int kResweepTiles = 32;
 // against 1.04, of 131,071 (m = 512) 1.02 against 1.74; at 65,536 (590 tiles)
 // 0.62 against 0.56.
 constexpr int kSeedGroupTiles = 1024;
-// Tiles from which a sample decides whether the sweep uses the group bound at all
-// (9 us; such a join of a random walk takes 1 ms and more).
-constexpr int kProbeTiles = 256;
+// Tiles from which a sample decides whether the sweep uses the group bound at all:
+// 3 us, where a join of a random walk takes 0.7 ms and more; noise of 30,000
+// samples (151 tiles, m = 64, w = 0) takes 1.3 ms with it and 3.8 without.
+constexpr int kProbeTiles = 128;
 // Their lists of group pairs, and with the samples and five words the bytes
 // they take.
 constexpr unsigned int kSeedSupCap = 1u << 24, kSeedListCap = 1u << 22;

@@ -50,7 +50,7 @@ def test_group_seeds_are_those_of_a_walk(gpu_dtwj, synth, kind, n, m, w):
 
 
 def test_join_of_noise_without_the_group_bound(gpu_dtwj, oracle):
-    # 256 tiles and more: the sweep samples the bound too, and leaves every tile dense
+    # 128 tiles and more: the sweep samples the bound too, and leaves every tile dense
     x = np.random.default_rng(9).standard_normal(45000)
     ref = oracle.join(x, 128, 0)
     with gpu_dtwj.Context() as ctx:
