@@ -58,7 +58,7 @@ constexpr int kResweepTiles = 32;
 constexpr int kSeedGroupTiles = 1024;
 // Tiles from which a sample decides whether the sweep uses the group bound at all:
 // 3 us, where a join of a random walk takes 0.7 ms and more; noise of 30,000
-// samples (151 tiles, m = 64, w = 0) takes 1.3 ms with it and 3.8 without.
+// samples (144 tiles, m = 64, w = 0) takes 1.3 ms with it and 3.8 without.
 constexpr int kProbeTiles = 128;
 // Their lists of group pairs, and with the samples and five words the bytes
 // they take.
