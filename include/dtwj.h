@@ -104,7 +104,8 @@ typedef struct {
   double dist;             /* its DTW distance, recomputed in FP64           */
   double dist_fp32;        /* the FP32 distance the device search found      */
   double seed_bsf;         /* best-so-far after the ED-profile seeds         */
-  uint64_t pairs;          /* candidate pairs (non-flat, j - i >= m)         */
+  uint64_t pairs;          /* candidate pairs (j - i >= m; those with a flat
+                              window count as pruned by the sweep)           */
   uint64_t pruned_fast;    /* pruned by the sweep: the block-mean bound of window
                               groups, or the O(1) diagonal bound in the tiles
                               where that settles nothing                     */

@@ -142,7 +142,7 @@ __global__ void k_init_search(unsigned int* bsf2, int nslots, unsigned long long
       nseeds[nseries] = (unsigned int)seed_slots;
       nseeds[nseries + 1] = 0u;
       zready[0] = zready[1] = 0u;  // the window table: not filled
-      low[0] = 64u;  // 43 pruned before all are tried
+      low[0] = 64u;  // at least 129 are pruned before all are tried
       low[1] = 0u;
       probe[0] = probe[1] = 0u;
     }
