@@ -5,8 +5,8 @@ that covers the band computes the same distances, so the choice is only about
 speed.  `tune` times each candidate and keeps the fastest.  The default timer
 is band cells per second on exact FP32 DTW of random-walk window pairs
 (dtwj_time_band); `join_timer(sample)` times joins of a sample series instead,
-which includes early abandoning (groups that share a warp then fall out of
-step, which favours one pair per warp).  Results are cached in a JSON file:
+which includes early abandoning and the slots that joins run narrow bands in.
+Results are cached in a JSON file:
 
     {"m=1024,w=52": {"C": 7, "G": 16, "cells_per_s": ..., "tried": [[C, G, cells_per_s], ...]}}
 
